@@ -5,6 +5,8 @@
 // M2L blocks (:1338-1361), the skeleton blocks of get_L2P_P2M_box (:1105-1128),
 // and the dense product of the find_error fixture generator
 // (FMM2DTree_gen_rhs_x.hpp:2864-2871).
+#include <algorithm>
+
 #include "kernels.h"
 #include "entry.cuh"
 
@@ -35,28 +37,220 @@ __global__ void list_entries_kernel(const int* __restrict__ I, const int* __rest
     out[t] = lsa_entry(I[t], J[t], ctx);
 }
 
-// y(:, s) = A x(:, s) for nrhs columns (x, y: N x nrhs column-major).
-// Each CTA owns 128 target rows and a slice of source points; partial sums are
-// combined with atomics.
+// ---- y(:, s) = A x(:, s) for nrhs <= 8 columns (x, y: N x nrhs column-major)
+//
+// A far entry is a 121-term series in the source point's coefficients M(:, j)
+// whose Hankel values and angles depend on the target point and the source LEAF
+// only.  So the sources of a leaf are summed first: m(n, s) = sum_j M(n, j) x(j, s)
+// (moments_kernel), and one series per (target, leaf) replaces one per entry --
+// rank times fewer Bessel recurrences.
+//   sum_n H_n(R) e^{in th} m_n = sum_{n >= 0} (J_n + i Y_n) (p_n cos n th + q_n sin n th)
+//   p_n = m_n + (-1)^n m_{-n},  q_n = i (m_n - (-1)^n m_{-n}),  p_0 = m_0,  q_0 = 0
+// What bounds it: latency and issue of the FP64 recurrences (about 1,900 double
+// instructions per target, leaf and one right-hand side; the moments are warp-
+// uniform reads of shared memory).  36,864 unknowns, one right-hand side, through
+// dense_matvec with host buffers: 958 ms with a series per entry, 10.3 ms with a
+// series per leaf; 2,304 unknowns: 4.4 ms and 0.14 ms; 256 unknowns: 99 us and 66 us.
 constexpr int kMvRows = 128;
 constexpr int kMvMaxRhs = 8;
-template <bool PHI>
-__global__ void __launch_bounds__(kMvRows) dense_matvec_kernel(const double2* __restrict__ x, double2* y, int N,
-                                                                int nrhs, int cols_per_slice, EntryCtx ctx) {
-  const int i = blockIdx.x * kMvRows + threadIdx.x;
-  const int j0 = blockIdx.y * cols_per_slice;
-  const int j1 = min(N, j0 + cols_per_slice);
-  if (i >= N) return;
-  double2 acc[kMvMaxRhs];
-  for (int s = 0; s < kMvMaxRhs; ++s) acc[s] = make_double2(0.0, 0.0);
-  for (int j = j0; j < j1; ++j) {
-    double2 a = lsa_entry<PHI>(i, j, ctx);
-    if (a.x == 0.0 && a.y == 0.0) continue;
-    for (int s = 0; s < nrhs; ++s) acc[s] = cfma(a, __ldg(&x[j + (size_t)s * N]), acc[s]);
+constexpr size_t kMvMomentBytes = size_t(64) << 20;  // moments of one chunk of leaves
+struct Moment { double2 p, q; };
+
+__global__ void __launch_bounds__(128) moments_kernel(const double2* __restrict__ x, Moment* __restrict__ mom, int N,
+                                                      int nrhs, int leaf0, int rank, const double2* __restrict__ M) {
+  const int leaf = leaf0 + blockIdx.x;
+  for (int t = threadIdx.x; t < (AIFMM_SERIES + 1) * nrhs; t += blockDim.x) {
+    const int n = t / nrhs, s = t - n * nrhs;
+    const double2* xs = x + (size_t)leaf * rank + (size_t)s * N;
+    double2 a = make_double2(0.0, 0.0), b = a;
+    for (int j = 0; j < rank; ++j) {
+      const double2* Mc = M + (size_t)j * (2 * AIFMM_SERIES + 1) + AIFMM_SERIES;
+      const double2 xv = __ldg(&xs[j]);
+      a = cfma(__ldg(&Mc[n]), xv, a);
+      b = cfma(__ldg(&Mc[-n]), xv, b);
+    }
+    Moment o;
+    if (n == 0) {
+      o.p = a;
+      o.q = make_double2(0.0, 0.0);
+    } else {
+      if (n & 1) b = cneg(b);
+      const double2 d = csub(a, b);
+      o.p = cadd(a, b);
+      o.q = make_double2(-d.y, d.x);
+    }
+    mom[((size_t)blockIdx.x * (AIFMM_SERIES + 1) + n) * nrhs + s] = o;
   }
-  for (int s = 0; s < nrhs; ++s) {
-    atomicAdd(&y[i + (size_t)s * N].x, acc[s].x);
-    atomicAdd(&y[i + (size_t)s * N].y, acc[s].y);
+}
+
+// Coefficients of the Neumann sums that give Y_0 and Y_1 from the J values of
+// Miller's recurrence: even m contribute (-1)^(m/2) / (m/2) J_m to the first, odd
+// m contribute (-1)^((m+1)/2) (2/(m+1) + 2/(m-1)) J_m to the second (entry.cuh).
+constexpr int kNeumann = 512;
+struct NeumannTable {
+  double c[kNeumann];
+  constexpr NeumannTable() : c() {
+    for (int m = 1; m < kNeumann; ++m) c[m] = coef(m);
+  }
+  __host__ __device__ static constexpr double coef(int m) {
+    if (m % 2 == 0) return (m / 2 % 2 ? -1.0 : 1.0) / (m / 2);
+    const int a = (m + 1) / 2;
+    return (a % 2 ? -1.0 : 1.0) * (1.0 / a + (m > 1 ? 1.0 / (a - 1) : 0.0));
+  }
+};
+__constant__ NeumannTable c_neumann = NeumannTable();
+
+// acc[s] += sum_n H_n(R) (p_n cos n th + q_n sin n th), (dx, dy) = target - leaf centre.
+// All lanes of `mask` call it together: the downward recurrence starts at the
+// largest order any of them needs, so that the loop and its tables are uniform.
+template <int NR>
+__device__ __forceinline__ void moment_series(double dx, double dy, double kappa, const Moment* mom,
+                                              unsigned mask, double2 (&acc)[NR]) {
+  const double rho = sqrt(dx * dx + dy * dy);
+  const double R = kappa * rho;
+  const double2 e1 = make_double2(dx / rho, dy / rho);
+  // e^{i 16 th}, e^{i 32 th}, e^{i 48 th} restart the rotation every 16 orders
+  double2 t2 = cmul(e1, e1), t4 = cmul(t2, t2), t8 = cmul(t4, t4);
+  const double2 e16 = cmul(t8, t8), e32 = cmul(e16, e16), e48 = cmul(e32, e16);
+  const double big = fmax((double)AIFMM_SERIES, R);
+  int N = (int)(big + 24.0 + 10.0 * cbrt(big));
+  N += (N & 1);
+  N = __reduce_max_sync(mask, N);
+  const double inv2 = 2.0 / R;
+  double jp1 = 0.0, jcur = 1.0e-250, norm = 0.0;
+  double S0 = 0.0, S1 = 0.0;
+  double2 a[NR];
+#pragma unroll
+  for (int s = 0; s < NR; ++s) a[s] = make_double2(0.0, 0.0);
+  double2 e = cmul(e48, cmul(t8, t4));  // e^{i 60 th}
+  // ---- downward: J_m, m = N - 1 .. 0, unnormalised
+  double dk = N;  // m + 1 as a double: conversions run at a fraction of the FP64 rate
+  for (int m = N - 1; m >= 0; --m, dk -= 1.0) {
+    const double jnew = fma(dk * inv2, jcur, -jp1);
+    jp1 = jcur;
+    jcur = jnew;
+    const double c = m < kNeumann ? c_neumann.c[m] : NeumannTable::coef(m);
+    if (m & 1) {
+      S1 = fma(c, jnew, S1);
+    } else {
+      norm += jnew;  // doubled at the end, where J_0 counts once
+      S0 = fma(c, jnew, S0);
+    }
+    if (m <= AIFMM_SERIES) {
+      if (m < AIFMM_SERIES) e = (m & 15) == 15 ? (m == 47 ? cmul(e48, cconj(e1)) : m == 31 ? cmul(e32, cconj(e1)) : cmul(e16, cconj(e1)))
+                                               : cmul(e, cconj(e1));
+#pragma unroll
+      for (int s = 0; s < NR; ++s) {
+        const Moment& w = mom[m * NR + s];
+        const double2 p = w.p, q = w.q;
+        const double jc = jnew * e.x, js = jnew * e.y;
+        a[s].x = fma(p.x, jc, a[s].x); a[s].x = fma(q.x, js, a[s].x);
+        a[s].y = fma(p.y, jc, a[s].y); a[s].y = fma(q.y, js, a[s].y);
+      }
+    }
+    if ((__double2hiint(jcur) & 0x7fffffff) > 0x69800000) {  // |J| above about 1e200: rescale
+      const double f = 1.0e-200;
+      jcur *= f; jp1 *= f; norm *= f; S0 *= f; S1 *= f;
+#pragma unroll
+      for (int s = 0; s < NR; ++s) a[s] = cscale(a[s], f);
+    }
+  }
+  const double inorm = 1.0 / (2.0 * norm - jcur);
+  const double J0 = jcur * inorm, J1 = jp1 * inorm;
+  S0 *= inorm; S1 *= inorm;
+#pragma unroll
+  for (int s = 0; s < NR; ++s) {
+    acc[s].x = fma(a[s].x, inorm, acc[s].x);
+    acc[s].y = fma(a[s].y, inorm, acc[s].y);
+    a[s] = make_double2(0.0, 0.0);
+  }
+  // ---- upward: Y_n, n = 0 .. 60
+  const double kTwoOverPi = 0.63661977236758134307553505349;
+  const double kEuler = 0.57721566490153286060651209008;
+  const double lg = log(0.5 * R) + kEuler;
+  double yc = kTwoOverPi * (lg * J0 - 2.0 * S0);
+  double yn = -kTwoOverPi / R * J0 + kTwoOverPi * (lg * J1 + S1);
+  e = make_double2(1.0, 0.0);
+  dk = 1.0;
+  for (int n = 0; n <= AIFMM_SERIES; ++n, dk += 1.0) {
+    const double jc = yc * e.x, js = yc * e.y;
+#pragma unroll
+    for (int s = 0; s < NR; ++s) {
+      const Moment& w = mom[n * NR + s];
+      const double2 p = w.p, q = w.q;
+      a[s].x = fma(p.x, jc, a[s].x); a[s].x = fma(q.x, js, a[s].x);
+      a[s].y = fma(p.y, jc, a[s].y); a[s].y = fma(q.y, js, a[s].y);
+    }
+    const double y2 = fma(dk * inv2, yn, -yc);
+    yc = yn;
+    yn = y2;
+    e = (n & 15) == 15 ? (n == 15 ? e16 : n == 31 ? e32 : e48) : cmul(e, e1);
+  }
+#pragma unroll
+  for (int s = 0; s < NR; ++s) {  // + i SY
+    acc[s].x -= a[s].y;
+    acc[s].y += a[s].x;
+  }
+}
+
+// Each thread owns one target row and a slice of the chunk's source leaves; the
+// slices are combined with atomics.  NR = nrhs, so that the accumulators stay in
+// registers.
+template <bool PHI, int NR>
+__global__ void __launch_bounds__(kMvRows) leaf_matvec_kernel(const double2* __restrict__ x, double2* y, int N,
+                                                               int leaf0, int nleaf, int leaves_per_slice,
+                                                               const Moment* __restrict__ mom, EntryCtx ctx) {
+  __shared__ Moment sm[(AIFMM_SERIES + 1) * NR];
+  const bool live = blockIdx.x * kMvRows + threadIdx.x < N;
+  const int i = min((int)(blockIdx.x * kMvRows + threadIdx.x), N - 1);
+  const int l0 = blockIdx.y * leaves_per_slice;
+  const int l1 = min(nleaf, l0 + leaves_per_slice);
+  const int rank = ctx.rank, li = i / rank, ii = i - li * rank;
+  const int2 me = __ldg(&ctx.leafxy[li]);
+  const double2 ri = __ldg(&ctx.pts[i]);
+  const double qi = __ldg(&ctx.q[i]);
+  const double kq = ctx.kappa * ctx.kappa * qi;
+  // Entries below 1e-16 are zero (entry.cuh).  The operator's own entries are at
+  // most a few units, so a row with kappa^2 |q| < 1e-30 holds the identity alone.
+  const bool only_identity = PHI && !(fabs(kq) >= 1e-30);
+  double2 far[NR], near[NR];
+#pragma unroll
+  for (int s = 0; s < NR; ++s) far[s] = near[s] = make_double2(0.0, 0.0);
+  for (int l = l0; l < l1; ++l) {
+    // the leaf's moments, read by every thread order by order: one load latency
+    // for all of them instead of one per order
+    const double2* src = reinterpret_cast<const double2*>(mom + (size_t)l * (AIFMM_SERIES + 1) * NR);
+    for (int t = threadIdx.x; t < 2 * (AIFMM_SERIES + 1) * NR; t += kMvRows)
+      reinterpret_cast<double2*>(sm)[t] = __ldg(&src[t]);
+    __syncthreads();
+    const int lj = leaf0 + l;
+    const int2 b = __ldg(&ctx.leafxy[lj]);
+    const int dx = b.x - me.x, dy = b.y - me.y;
+    const bool close = dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1;
+    const bool series = !close && !only_identity;
+    const unsigned mask = __ballot_sync(0xffffffffu, series);
+    if (series) {
+      const double2 c = __ldg(&ctx.leafc[lj]);
+      moment_series<NR>(ri.x - c.x, ri.y - c.y, ctx.kappa, sm, mask, far);
+    } else if (close && (!only_identity || lj == li)) {
+      const int j0 = only_identity ? ii : 0, j1 = only_identity ? ii + 1 : rank;
+      for (int j = j0; j < j1; ++j) {
+        const double2 a = lsa_entry<PHI>(i, lj * rank + j, ctx);
+        if (a.x == 0.0 && a.y == 0.0) continue;
+#pragma unroll
+        for (int s = 0; s < NR; ++s) near[s] = cfma(a, __ldg(&x[(size_t)lj * rank + j + (size_t)s * N]), near[s]);
+      }
+    }
+    __syncthreads();
+  }
+  if (!live) return;
+#pragma unroll
+  for (int s = 0; s < NR; ++s) {
+    double2 v = make_double2(-0.25 * far[s].y, 0.25 * far[s].x);  // times i/4
+    if (PHI) v = cscale(v, kq);
+    v = cadd(v, near[s]);
+    atomicAdd(&y[i + (size_t)s * N].x, v.x);
+    atomicAdd(&y[i + (size_t)s * N].y, v.y);
   }
 }
 
@@ -80,29 +274,58 @@ int aifmm_launch_list_entries(const int* I, const int* J, long n, double2* out, 
   return (int)cudaGetLastError();
 }
 
+// bytes of moment scratch a dense product needs: one chunk of leaves
+size_t aifmm_matvec_scratch_bytes(int N, int rank, int nrhs) {
+  const size_t per_leaf = sizeof(Moment) * (AIFMM_SERIES + 1) * (size_t)nrhs;
+  const size_t nleaf = (size_t)N / rank;
+  return per_leaf * std::min(nleaf, std::max<size_t>(1, kMvMomentBytes / per_leaf));
+}
+
 namespace {
+template <bool PHI, int NR>
+void launch_leaf_matvec(dim3 grid, const double2* x, double2* y, int N, int leaf0, int nl, int lps, const Moment* mom,
+                        const EntryCtx& ctx, cudaStream_t stream) {
+  leaf_matvec_kernel<PHI, NR><<<grid, kMvRows, 0, stream>>>(x, y, N, leaf0, nl, lps, mom, ctx);
+}
 template <bool PHI>
-int launch_matvec(const double2* x, double2* y, int N, int nrhs, const EntryCtx& ctx, cudaStream_t stream) {
-  if (nrhs > kMvMaxRhs) return (int)cudaErrorInvalidValue;
+int launch_matvec(const double2* x, double2* y, int N, int nrhs, void* scratch, const EntryCtx& ctx,
+                  cudaStream_t stream) {
+  if (nrhs < 1 || nrhs > kMvMaxRhs) return (int)cudaErrorInvalidValue;
+  Moment* mom = static_cast<Moment*>(scratch);
+  const int nleaf = N / ctx.rank;
+  const int chunk = (int)(aifmm_matvec_scratch_bytes(N, ctx.rank, nrhs) / (sizeof(Moment) * (AIFMM_SERIES + 1) * nrhs));
   const int row_blocks = (N + kMvRows - 1) / kMvRows;
-  // enough slices to give every SM several CTAs
-  int slices = (148 * 8 + row_blocks - 1) / row_blocks;
-  if (slices < 1) slices = 1;
-  int cps = (N + slices - 1) / slices;
-  slices = (N + cps - 1) / cps;
-  dim3 grid(row_blocks, slices);
-  dense_matvec_kernel<PHI><<<grid, kMvRows, 0, stream>>>(x, y, N, nrhs, cps, ctx);
-  return (int)cudaGetLastError();
+  for (int leaf0 = 0; leaf0 < nleaf; leaf0 += chunk) {
+    const int nl = std::min(chunk, nleaf - leaf0);
+    moments_kernel<<<nl, 128, 0, stream>>>(x, mom, N, nrhs, leaf0, ctx.rank, ctx.M);
+    // Rows far outside the contrast finish at once, so the slices are many more than
+    // fill the chip: up to 64 CTAs for every SM, but at least 4 leaves a slice once
+    // there are 8 CTAs for every SM.
+    const int few = (148 * 8 + row_blocks - 1) / row_blocks, many = (148 * 64 + row_blocks - 1) / row_blocks;
+    const int slices0 = std::max(1, std::min(nl, std::max(few, std::min(many, nl / 4))));
+    const int lps = (nl + slices0 - 1) / slices0;
+    const dim3 grid(row_blocks, (nl + lps - 1) / lps);
+    switch (nrhs) {
+#define AIFMM_MV_CASE(R) \
+      case R: launch_leaf_matvec<PHI, R>(grid, x, y, N, leaf0, nl, lps, mom, ctx, stream); break;
+      AIFMM_MV_CASE(1) AIFMM_MV_CASE(2) AIFMM_MV_CASE(3) AIFMM_MV_CASE(4)
+      AIFMM_MV_CASE(5) AIFMM_MV_CASE(6) AIFMM_MV_CASE(7) AIFMM_MV_CASE(8)
+#undef AIFMM_MV_CASE
+    }
+    const int e = (int)cudaGetLastError();
+    if (e) return e;
+  }
+  return 0;
 }
 }  // namespace
 
-int aifmm_launch_dense_matvec(const double2* x, double2* y, int N, int nrhs, const EntryCtx& ctx,
+int aifmm_launch_dense_matvec(const double2* x, double2* y, int N, int nrhs, void* scratch, const EntryCtx& ctx,
                               cudaStream_t stream) {
   if (nrhs > kMvMaxRhs) return (int)cudaErrorInvalidValue;
   cudaMemsetAsync(y, 0, sizeof(double2) * (size_t)N * nrhs, stream);
-  return launch_matvec<true>(x, y, N, nrhs, ctx, stream);
+  return launch_matvec<true>(x, y, N, nrhs, scratch, ctx, stream);
 }
-int aifmm_launch_green_matvec_add(const double2* x, double2* y, int N, int nrhs, const EntryCtx& ctx,
+int aifmm_launch_green_matvec_add(const double2* x, double2* y, int N, int nrhs, void* scratch, const EntryCtx& ctx,
                                   cudaStream_t stream) {
-  return launch_matvec<false>(x, y, N, nrhs, ctx, stream);
+  return launch_matvec<false>(x, y, N, nrhs, scratch, ctx, stream);
 }

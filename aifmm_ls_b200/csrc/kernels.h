@@ -138,10 +138,12 @@ int aifmm_launch_block_entries(const BlockDesc* d_desc, const long long* d_off, 
                                const EntryCtx& ctx, cudaStream_t stream);
 int aifmm_launch_list_entries(const int* I, const int* J, long n, double2* out, const EntryCtx& ctx,
                               cudaStream_t stream);
-int aifmm_launch_dense_matvec(const double2* x, double2* y, int N, int nrhs, const EntryCtx& ctx,
+// scratch: aifmm_matvec_scratch_bytes on the device
+size_t aifmm_matvec_scratch_bytes(int N, int rank, int nrhs);
+int aifmm_launch_dense_matvec(const double2* x, double2* y, int N, int nrhs, void* scratch, const EntryCtx& ctx,
                               cudaStream_t stream);
 // y += G x with G the entries without kappa^2 q and identity (findPhi = false)
-int aifmm_launch_green_matvec_add(const double2* x, double2* y, int N, int nrhs, const EntryCtx& ctx,
+int aifmm_launch_green_matvec_add(const double2* x, double2* y, int N, int nrhs, void* scratch, const EntryCtx& ctx,
                                   cudaStream_t stream);
 int aifmm_launch_aca(const AcaJob* d_jobs, int njobs, double tol, const EntryCtx& ctx, cudaStream_t stream);
 int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int es, cudaStream_t s);

@@ -3537,6 +3537,7 @@ aifmm_status aifmm_dense_matvec(aifmm_problem* p, int nrhs, const double* x, dou
   if (!p || !x || !y || nrhs < 1 || nrhs > 8) return AIFMM_ERR_ARG;
   if (!p->tables_ready) { p->err = "tables not ready"; return AIFMM_ERR_STATE; }
   return guard(p, [&] {
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
     const size_t bytes = sizeof(double2) * (size_t)p->N * nrhs;
     const bool dev = flags & AIFMM_PTR_DEVICE;
     const double2* dx = reinterpret_cast<const double2*>(x);
@@ -3546,7 +3547,8 @@ aifmm_status aifmm_dense_matvec(aifmm_problem* p, int nrhs, const double* x, dou
       CK(cudaMemcpyAsync(tx.ptr, x, bytes, cudaMemcpyHostToDevice, p->st));
       dx = tx.as<double2>(); dy = ty.as<double2>();
     }
-    int e = aifmm_launch_dense_matvec(dx, dy, p->N, nrhs, p->ctx(), p->st);
+    aifmm_problem::Tmp ts(p, aifmm_matvec_scratch_bytes(p->N, p->rank, nrhs));
+    int e = aifmm_launch_dense_matvec(dx, dy, p->N, nrhs, ts.ptr, p->ctx(), p->st);
     if (e) throw Fail(AIFMM_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
     if (!dev) CK(cudaMemcpyAsync(y, dy, bytes, cudaMemcpyDeviceToHost, p->st));
     p->sync();
@@ -3558,6 +3560,7 @@ aifmm_status aifmm_total_field(aifmm_problem* p, int nrhs, const double* theta, 
   if (!p || !theta || !phi || !u || nrhs < 1 || nrhs > 8) return AIFMM_ERR_ARG;
   if (!p->tables_ready) { p->err = "tables not ready"; return AIFMM_ERR_STATE; }
   return guard(p, [&] {
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
     const size_t bytes = sizeof(double2) * (size_t)p->N * nrhs;
     const bool dev = flags & AIFMM_PTR_DEVICE;
     const double2* dphi = reinterpret_cast<const double2*>(phi);
@@ -3569,7 +3572,8 @@ aifmm_status aifmm_total_field(aifmm_problem* p, int nrhs, const double* theta, 
     }
     const double* dth = static_cast<const double*>(p->stage.put_raw(theta, sizeof(double) * nrhs, p->st));
     int e = aifmm_launch_incident_field(p->d_pts, p->d.kappa, p->N, nrhs, dth, du, p->st);
-    if (!e) e = aifmm_launch_green_matvec_add(dphi, du, p->N, nrhs, p->ctx(), p->st);
+    aifmm_problem::Tmp ts(p, aifmm_matvec_scratch_bytes(p->N, p->rank, nrhs));
+    if (!e) e = aifmm_launch_green_matvec_add(dphi, du, p->N, nrhs, ts.ptr, p->ctx(), p->st);
     if (e) throw Fail(AIFMM_ERR_CUDA, cudaGetErrorString((cudaError_t)e));
     if (!dev) CK(cudaMemcpyAsync(u, du, bytes, cudaMemcpyDeviceToHost, p->st));
     p->sync();
