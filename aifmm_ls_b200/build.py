@@ -15,7 +15,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libaifmm_b200.so")
-SOURCES = ["k_geom.cu", "k_tables.cu", "k_entries.cu", "k_aca.cu", "k_dense.cu", "solver.cu", "server.cpp"]
+SOURCES = ["k_geom.cu", "k_tables.cu", "k_entries.cu", "k_aca.cu", "k_dense.cu", "k_qr.cu", "k_compress.cu", "solver.cu", "server.cpp"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

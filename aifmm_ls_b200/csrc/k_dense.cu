@@ -14,34 +14,10 @@
 //  * Batched GEMM / GEAM / Frobenius norms.
 // One CTA per factorisation; everything else is batched over descriptor lists.
 #include <algorithm>
-#include <cfloat>
-#include "kernels.h"
+#include "dense.cuh"
 #include "entry.cuh"
 
 namespace {
-
-constexpr int kT = 256;
-constexpr int kW = kT / 32;
-constexpr double kPivotTie = 1e-11;  // same pivot tie tolerance as the ACA
-
-// Real-type constants of the two forms: machine epsilon, the smallest normal
-// number, and the range inside which a product may be inverted directly.
-template <typename R> struct rl;
-template <> struct rl<double> {
-  static constexpr double eps = DBL_EPSILON, tiny = DBL_MIN, lo = 1e-290, hi = 1e290;
-};
-template <> struct rl<float> {
-  static constexpr float eps = FLT_EPSILON, tiny = FLT_MIN, lo = 1e-35f, hi = 1e35f;
-};
-
-// Norms, reflector scalars and pivot reciprocals are computed in double for both
-// forms: complex64 blocks of the contrast's far corners hold values near 1e-25,
-// whose squares underflow FP32 and whose reciprocals overflow it.  The O(m n)
-// column updates stay in the blocks' own precision.
-__device__ __forceinline__ double cabs2d(double2 a) { return cabs2(a); }
-__device__ __forceinline__ double cabs2d(float2 a) { const double x = a.x, y = a.y; return x * x + y * y; }
-__device__ __forceinline__ double2 c2d(double2 a) { return a; }
-__device__ __forceinline__ double2 c2d(float2 a) { return make_double2(a.x, a.y); }
 
 template <typename R>
 __device__ __forceinline__ R warp_sum(R x) {
@@ -210,355 +186,6 @@ template <typename C>
 __global__ void __launch_bounds__(kT) qr_factor_kernel(const QRJob* __restrict__ jobs) {
   const QRJob J = jobs[blockIdx.x];
   qr_factor_body<C>(J, static_cast<C*>(J.a), J.lda, J.norms, J.norms + J.n, J.perm);
-}
-
-// Jobs whose matrix fits in shared memory, one barrier per pivot step.
-// The matrix sits in shared memory by original column ("slot"); a column swap
-// only exchanges the positions that two slots carry.  Each pivot step:
-//   1. every warp selects the pivot from the shared norms/positions and builds
-//      the reflector from the pivot column into its own buffer (all warps get the
-//      same bits: same data, same reduction order), so no warp waits for another;
-//   2. warp (k mod warps) writes the finished pivot column -- R above, beta on,
-//      the reflector below the diagonal -- straight to global memory;
-//   3. the four lanes of a group apply the reflector to each column the group
-//      owns (slots g, g + 64, ...; rows interleaved over the lanes) and downdate
-//      its norm;
-//   4. one barrier.
-// Norms and positions are double-buffered by step parity, so a warp running
-// ahead never changes what a slower warp is still scanning.  Columns left at
-// positions >= min(m, n) are written out at the end.
-// Arithmetic: pivot ties as in qr_factor_body; the reflector scalars tau and
-// 1/(a_kk - beta) come from one division; the norm downdate of LAPACK Working
-// Note 176 is evaluated without divisions -- with T = (nu - |r|)(nu + |r|) (the
-// LAWN quantity (1 - (|r|/nu)^2) times nu^2), the column is recomputed when
-// T <= sqrt(eps) nd^2 and otherwise nu becomes sqrt(T).
-constexpr int kQrGroups = kT / 4;
-__host__ __device__ __forceinline__ int qr_smem_ld(int m) { return m + ((12 - (m & 7)) & 7); }  // ld = 4 (mod 8)
-
-template <typename C>
-__device__ void qr_smem_body(const QRJob& J, C* qsm) {
-  const int m = J.m, n = J.n, size = min(m, n);
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, p = tid & 3, g = tid >> 2;
-  const int ld = qr_smem_ld(m);
-  const unsigned full = 0xffffffffu, gm = 0xfu << (lane & ~3);
-  C* A = qsm;                                                    // ld x n, by slot
-  C* V = A + (size_t)ld * n;                                     // kW x m: each warp's reflector
-  double* snu2 = reinterpret_cast<double*>(V + (size_t)kW * m);  // 2 x n: norms, by step parity
-  double* snd = snu2 + 2 * n;                                    // n: norms at the last recompute
-  double* srd = snd + n;                                         // size: |R_kk|
-  int* spos2 = reinterpret_cast<int*>(srd + size);               // 2 x n: positions, by step parity
-  const C* Ja = static_cast<const C*>(J.a);
-  C* Jout = static_cast<C*>(J.a);
-  C* Jtau = static_cast<C*>(J.tau);
-  for (int e = tid; e < m * n; e += kT) {
-    const int i = e % m, j = e / m;
-    A[i + (size_t)j * ld] = Ja[i + (size_t)j * J.lda];
-  }
-  __syncthreads();
-  for (int s = g; s < n; s += kQrGroups) {
-    const C* col = A + (size_t)s * ld;
-    double q = 0.0;
-    for (int i = p; i < m; i += 4) q += cabs2d(col[i]);
-    q += __shfl_xor_sync(gm, q, 1);
-    q += __shfl_xor_sync(gm, q, 2);
-    if (p == 0) { snu2[s] = snd[s] = sqrt(q); spos2[s] = s; }
-  }
-  __syncthreads();
-  const int nscan = (n + 31) >> 5;
-  double maxnorm = 0.0;
-  for (int q = 0; q < nscan; ++q) { const int s = lane + 32 * q; if (s < n) maxnorm = fmax(maxnorm, snu2[s]); }
-  for (int o = 16; o > 0; o >>= 1) maxnorm = fmax(maxnorm, __shfl_xor_sync(full, maxnorm, o));
-  const double eps = rl<typename cplx<C>::R>::eps;  // the precision of the data
-  const double thr_helper = m > 0 ? (maxnorm * eps) * (maxnorm * eps) / m : 0.0;
-  const double downdate_thr = sqrt(eps);
-  C* vw = V + (size_t)w * m;
-  int nzp = size;
-  double maxpivot = 0.0;
-  for (int k = 0; k < size; ++k) {
-    const double* snu = snu2 + (k & 1) * n;
-    const int* spos = spos2 + (k & 1) * n;
-    double* snu_n = snu2 + ((k + 1) & 1) * n;
-    int* spos_n = spos2 + ((k + 1) & 1) * n;
-    // 1. pivot: largest norm at positions >= k, the first position within the
-    //    tie tolerance.  Norms are non-negative: their bit patterns order like
-    //    their values, so the maximum is two unsigned warp reductions.
-    unsigned hi = 0, lo = 0;
-    for (int q = 0; q < nscan; ++q) {
-      const int s = lane + 32 * q;
-      if (s < n && spos[s] >= k) {
-        const double v = snu[s];
-        const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
-        if (h > hi || (h == hi && l > lo)) { hi = h; lo = l; }
-      }
-    }
-    const unsigned mh = __reduce_max_sync(full, hi);
-    const unsigned ml = __reduce_max_sync(full, hi == mh ? lo : 0u);
-    const double cut = __hiloint2double((int)mh, (int)ml) * (1.0 - kPivotTie);
-    unsigned key = 0xffffffffu;
-    for (int q = 0; q < nscan; ++q) {
-      const int s = lane + 32 * q;
-      if (s < n) {
-        const int ps = spos[s];
-        if (ps >= k && snu[s] >= cut) key = min(key, (unsigned)ps * 1024u + (unsigned)s);
-      }
-    }
-    key = __reduce_min_sync(full, key);
-    const int big = (int)(key >> 10), bslot = (int)(key & 1023u);
-    const double nub = snu[bslot];
-    if (nzp == size && nub * nub < thr_helper * (double)(m - k)) nzp = k;
-    //    reflector for the pivot column, rows k..m-1
-    const C* pc = A + (size_t)bslot * ld;
-    double tail = 0.0;
-    for (int i = k + 1 + lane; i < m; i += 32) tail += cabs2d(pc[i]);
-    for (int o = 16; o > 0; o >>= 1) tail += __shfl_xor_sync(full, tail, o);
-    const double2 c0 = c2d(pc[k]);
-    double beta;
-    C t;
-    if (tail <= DBL_MIN && c0.y * c0.y <= DBL_MIN) {
-      beta = c0.x;
-      t = cplx<C>::mk(0.0, 0.0);
-      for (int i = k + 1 + lane; i < m; i += 32) vw[i] = cplx<C>::mk(0.0, 0.0);
-    } else {
-      beta = sqrt(cabs2(c0) + tail);
-      if (c0.x >= 0.0) beta = -beta;
-      const double2 den = make_double2(c0.x - beta, c0.y);
-      const double dd = cabs2(den);
-      const double prod = beta * dd;
-      double ib, idd;  // 1/beta, 1/|den|^2
-      if (fabs(prod) > 1e-290 && fabs(prod) < 1e290) {
-        const double q = 1.0 / prod;
-        ib = dd * q;
-        idd = beta * q;
-      } else {
-        ib = 1.0 / beta;
-        idd = 1.0 / dd;
-      }
-      t = cplx<C>::from(make_double2((beta - c0.x) * ib, c0.y * ib));  // conj((beta - a_kk) / beta)
-      const double2 rden = make_double2(den.x * idd, -den.y * idd);    // 1 / (a_kk - beta)
-      for (int i = k + 1 + lane; i < m; i += 32) vw[i] = cplx<C>::from(cmul(c2d(pc[i]), rden));
-    }
-    maxpivot = fmax(maxpivot, fabs(beta));
-    __syncwarp();
-    // 2. the finished pivot column goes to position k
-    if (w == (k & (kW - 1))) {
-      C* out = Jout + (size_t)k * J.lda;
-      for (int i = lane; i < m; i += 32) out[i] = i < k ? pc[i] : (i == k ? cplx<C>::mk(beta, 0.0) : vw[i]);
-      if (lane == 0) { Jtau[k] = t; J.perm[k] = bslot; srd[k] = fabs(beta); }
-    }
-    // 3. G = I - t v v^H on the columns at positions > k; norm downdates
-    for (int s = g; s < n; s += kQrGroups) {
-      int ps = spos[s];
-      if (ps == big) ps = k;
-      else if (ps == k) ps = big;
-      if (ps > k) {
-        C* col = A + (size_t)s * ld;
-        const int i0 = k + 1 + ((p - (k + 1)) & 3);  // this lane's first row below k
-        C d0 = cplx<C>::mk(0.0, 0.0), d1 = cplx<C>::mk(0.0, 0.0);
-        int i = i0;
-        for (; i + 4 < m; i += 8) { d0 = cfmac(vw[i], col[i], d0); d1 = cfmac(vw[i + 4], col[i + 4], d1); }
-        if (i < m) d0 = cfmac(vw[i], col[i], d0);
-        C d = cadd(d0, d1);
-        d.x += __shfl_xor_sync(gm, d.x, 1); d.y += __shfl_xor_sync(gm, d.y, 1);
-        d.x += __shfl_xor_sync(gm, d.x, 2); d.y += __shfl_xor_sync(gm, d.y, 2);
-        const C akj = col[k];
-        const C tw = cmul(t, cadd(akj, d));
-        for (int r = i0; r < m; r += 4) col[r] = csub(col[r], cmul(vw[r], tw));
-        const C rkj = csub(akj, tw);
-        __syncwarp(gm);
-        if (p == 0) col[k] = rkj;
-        double nu = snu[s], nd = snd[s];
-        if (nu != 0.0) {
-          const double ar = sqrt(cabs2d(rkj));
-          double tt = (nu - ar) * (nu + ar);
-          if (tt < 0.0) tt = 0.0;
-          if (tt <= downdate_thr * (nd * nd)) {
-            double q = 0.0;
-            for (int r = i0; r < m; r += 4) q += cabs2d(col[r]);
-            q += __shfl_xor_sync(gm, q, 1);
-            q += __shfl_xor_sync(gm, q, 2);
-            nd = sqrt(q);
-            nu = nd;
-          } else {
-            nu = sqrt(tt);
-          }
-        }
-        if (p == 0) { snu_n[s] = nu; snd[s] = nd; }
-      }
-      if (p == 0) spos_n[s] = ps;
-    }
-    __syncthreads();
-  }
-  // 4. columns that were never pivots (positions >= size)
-  const int* spos = spos2 + (size & 1) * n;
-  for (int s = g; s < n; s += kQrGroups) {
-    const int ps = spos[s];
-    if (ps >= size) {
-      const C* col = A + (size_t)s * ld;
-      C* out = Jout + (size_t)ps * J.lda;
-      for (int i = p; i < m; i += 4) out[i] = col[i];
-      if (p == 0) J.perm[ps] = s;
-    }
-  }
-  if (tid == 0) {
-    const double thr = J.thr > 0.0 ? J.thr : (double)size * eps;
-    const double pre = fabs(maxpivot) * thr;
-    int rk = 0;
-    for (int i = 0; i < nzp; ++i) rk += (srd[i] > pre);
-    J.info[0] = nzp;
-    J.info[1] = rk;
-    if (J.maxpiv) J.maxpiv[0] = maxpivot;
-  }
-}
-
-template <typename C>
-__global__ void __launch_bounds__(kT) qr_factor_smem_kernel(const QRJob* __restrict__ jobs) {
-  extern __shared__ double2 qsm[];
-  const QRJob J = jobs[blockIdx.x];
-  qr_smem_body<C>(J, reinterpret_cast<C*>(qsm));
-}
-
-// ---------------------------------------------------------------- fused compression
-// CTA-wide building blocks on global-memory operands (written earlier by the
-// same CTA; a __syncthreads separates producer and consumer).
-
-// C (m x n, ldc) = alpha op(A) op(B) + beta C; op 1 = conjugate transpose.
-// Accumulation over k in increasing order, as gemm_kernel.
-template <typename C>
-__device__ void cta_gemm(C* Cm, int ldc, int m, int n, int k, const C* A, int lda, int opA,
-                         const C* B, int ldb, int opB, double2 alpha_, double2 beta_) {
-  const bool zero_beta = beta_.x == 0.0 && beta_.y == 0.0;
-  const C alpha = cplx<C>::from(alpha_), beta = cplx<C>::from(beta_);
-  for (int o = threadIdx.x; o < m * n; o += kT) {
-    const int i = o % m, jj = o / m;
-    C acc = cplx<C>::mk(0.0, 0.0);
-#pragma unroll 4
-    for (int kk = 0; kk < k; ++kk) {
-      const C a = opA ? cconj(A[kk + (size_t)i * lda]) : A[i + (size_t)kk * lda];
-      const C b = opB ? cconj(B[jj + (size_t)kk * ldb]) : B[kk + (size_t)jj * ldb];
-      acc = cfma(a, b, acc);
-    }
-    C v = cmul(alpha, acc);
-    if (!zero_beta) v = cadd(v, cmul(beta, Cm[i + (size_t)jj * ldc]));
-    Cm[i + (size_t)jj * ldc] = v;
-  }
-}
-
-size_t aifmm_formq_smem_bytes(int m, int size, int ncols, int es) {
-  return (size_t)es * ((size_t)(m | 1) * size + size + (size_t)m * ncols);
-}
-
-// Q(:, 0:ncols) = householderQ() of an m x n factor (reflectors below the
-// diagonal of qr, coefficients tau): column c is G_0^H ... G_min(c, size-1)^H e_c.
-// The factor is staged in shared memory; the four lanes of a group build one
-// column (rows interleaved), reducing the reflector dot products by shuffles.
-template <typename C>
-__device__ void cta_formq(const C* qr, int ldq, int m, int n, const C* tau, C* Q, int ldQ, int ncols, C* sm) {
-  const int size = min(m, n), ldf = m | 1;
-  const int tid = threadIdx.x, lane = tid & 31, p = tid & 3, g = tid >> 2;
-  const unsigned gm = 0xfu << (lane & ~3);
-  C* F = sm;
-  C* ts = F + (size_t)ldf * size;
-  C* Qs = ts + size;
-  for (int e = tid; e < m * size; e += kT) {
-    const int i = e % m, j = e / m;
-    F[i + (size_t)j * ldf] = qr[i + (size_t)j * ldq];
-  }
-  for (int k = tid; k < size; k += kT) ts[k] = cconj(tau[k]);
-  for (int e = tid; e < m * ncols; e += kT) {
-    const int i = e % m, j = e / m;
-    Qs[e] = cplx<C>::mk(i == j ? 1.0 : 0.0, 0.0);
-  }
-  __syncthreads();
-  for (int cc = g; cc < ncols; cc += kQrGroups) {
-    C* q = Qs + (size_t)cc * m;
-    for (int k = min(size - 1, cc); k >= 0; --k) {
-      const C* v = F + (size_t)k * ldf;
-      const int i0 = k + 1 + ((p - (k + 1)) & 3);
-      C d = cplx<C>::mk(0.0, 0.0);
-      for (int i = i0; i < m; i += 4) d = cfmac(v[i], q[i], d);
-      d.x += __shfl_xor_sync(gm, d.x, 1); d.y += __shfl_xor_sync(gm, d.y, 1);
-      d.x += __shfl_xor_sync(gm, d.x, 2); d.y += __shfl_xor_sync(gm, d.y, 2);
-      const C qk = q[k];
-      const C tw = cmul(ts[k], cadd(qk, d));
-      for (int i = i0; i < m; i += 4) q[i] = csub(q[i], cmul(v[i], tw));
-      __syncwarp(gm);
-      if (p == 0) q[k] = csub(qk, tw);
-      __syncwarp(gm);
-    }
-  }
-  __syncthreads();
-  for (int e = tid; e < m * ncols; e += kT) {
-    const int i = e % m, j = e / m;
-    Q[i + (size_t)j * ldQ] = Qs[e];
-  }
-}
-
-template <typename C>
-__global__ void __launch_bounds__(kT) compress_p2p_kernel(const CompressJob* __restrict__ jobs) {
-  extern __shared__ double2 csm_raw[];
-  C* csm = reinterpret_cast<C*>(csm_raw);
-  const CompressJob J = jobs[blockIdx.x];
-  const int m = J.m, rK = J.rK, c = J.c, rb = J.rb, n1 = rK + c;
-  const int tid = threadIdx.x;
-  const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
-  const C* L2P = static_cast<const C*>(J.L2P);
-  const C* Pkb = static_cast<const C*>(J.Pkb);
-  const C* P2M = static_cast<const C*>(J.P2M);
-  const C* M2L = static_cast<const C*>(J.M2L);
-  C* Acol = static_cast<C*>(J.Acol);
-  C* Arow = static_cast<C*>(J.Arow);
-  C* tau = static_cast<C*>(J.tau);
-  C* nL = static_cast<C*>(J.nL);
-  C* nPt = static_cast<C*>(J.nPt);
-  C* Rkp = static_cast<C*>(J.Rkp);
-  C* Rk = static_cast<C*>(J.Rk);
-  C* Rn = static_cast<C*>(J.Rn);
-  C* Rnp = static_cast<C*>(J.Rnp);
-  C* Tm = static_cast<C*>(J.Tm);
-  C* M2Lo = static_cast<C*>(J.M2Lo);
-  // [L2P_k | P2P_kb]
-  for (int e = tid; e < m * n1; e += kT) {
-    const int i = e % m, col = e / m;
-    Acol[e] = col < rK ? L2P[i + (size_t)col * J.ldL] : Pkb[i + (size_t)(col - rK) * J.ldP];
-  }
-  __syncthreads();
-  QRJob q{};
-  q.a = Acol; q.lda = m; q.m = m; q.n = n1; q.tau = tau; q.perm = J.perm; q.info = J.info; q.thr = J.tol;
-  qr_smem_body<C>(q, csm);
-  __syncthreads();
-  const int rc = J.info[1];
-  const int ldc_ = max(rc, 1);
-  cta_formq<C>(Acol, m, m, n1, tau, nL, m, rc, csm);
-  __syncthreads();
-  cta_gemm<C>(Rkp, ldc_, rc, c, m, nL, m, 1, Pkb, J.ldP, 0, one, zero);   // R' = nL^H P2P_kb
-  cta_gemm<C>(Rk, ldc_, rc, rK, m, nL, m, 1, L2P, J.ldL, 0, one, zero);   // R = nL^H L2P_k
-  __syncthreads();
-  // [P2M_b^H | R'^H]
-  const int n2 = rb + rc;
-  for (int e = tid; e < c * n2; e += kT) {
-    const int i = e % c, col = e / c;
-    Arow[e] = col < rb ? cconj(P2M[col + (size_t)i * J.ldM]) : cconj(Rkp[(col - rb) + (size_t)i * ldc_]);
-  }
-  __syncthreads();
-  q.a = Arow; q.lda = c; q.m = c; q.n = n2; q.info = J.info + 2;
-  qr_smem_body<C>(q, csm);
-  __syncthreads();
-  const int rr = J.info[3];
-  const int ldr_ = max(rr, 1);
-  cta_formq<C>(Arow, c, c, n2, tau, nPt, c, rr, csm);
-  __syncthreads();
-  cta_gemm<C>(Rn, ldr_, rr, rb, c, nPt, c, 1, P2M, J.ldM, 1, one, zero);    // nPt^H P2M_b^H
-  cta_gemm<C>(Rnp, ldr_, rr, rc, c, nPt, c, 1, Rkp, ldc_, 1, one, zero);    // nPt^H R'^H
-  cta_gemm<C>(Tm, ldc_, rc, rb, rK, Rk, ldc_, 0, M2L, J.ldT, 0, one, zero);  // R M2L_kb
-  __syncthreads();
-  cta_gemm<C>(M2Lo, J.ldO, rc, rr, rb, Tm, ldc_, 0, Rn, ldr_, 1, one, zero);
-  __syncthreads();
-  for (int e = tid; e < rc * rr; e += kT) {
-    const int i = e % rc, jj = e / rc;
-    C* o = M2Lo + i + (size_t)jj * J.ldO;
-    *o = cadd(cconj(Rnp[jj + (size_t)i * ldr_]), *o);
-  }
-  if (tid == 0) { J.ranks[0] = rc; J.ranks[1] = rr; }
 }
 
 // ---------------------------------------------------------------- QR solve (warp per column, registers)
@@ -1060,19 +687,6 @@ __global__ void __launch_bounds__(kT) skel_lu_kernel(const SkelLUJob* __restrict
 
 }  // namespace
 
-namespace {
-// the element size of a batch: 16 (complex128) or 8 (complex64)
-bool valid_es(int es) { return es == 16 || es == 8; }
-// opt a kernel into the large dynamic shared memory once per process
-template <typename K>
-void smem_attr_once(K kernel, bool& done) {
-  if (!done) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    done = true;
-  }
-}
-}  // namespace
-
 int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int es, cudaStream_t s) {
   if (njobs <= 0) return 0;
   if (!valid_es(es)) return (int)cudaErrorInvalidValue;
@@ -1111,24 +725,6 @@ int aifmm_launch_qr_solve_warp(const SolveJob* d_jobs, const int* d_cta_off, int
                   : launch_solve_warp<float2>(d_jobs, d_cta_off, njobs, total_ctas, rpl, smem, s);
 }
 
-size_t aifmm_qr_smem_bytes(int m, int n, int es) {
-  if (n > 1024) return ~size_t(0);  // pivot keys hold a column index below 1024
-  return (size_t)es * ((size_t)qr_smem_ld(m) * n + (size_t)kW * m) +
-         sizeof(double) * (3 * (size_t)n + (size_t)std::min(m, n)) + sizeof(int) * 2 * (size_t)n;
-}
-int aifmm_launch_qr_factor_smem(const QRJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s) {
-  if (njobs <= 0) return 0;
-  if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  static bool attr[2] = {false, false};
-  if (es == 16) {
-    smem_attr_once(qr_factor_smem_kernel<double2>, attr[0]);
-    qr_factor_smem_kernel<double2><<<njobs, kT, smem, s>>>(d_jobs);
-  } else {
-    smem_attr_once(qr_factor_smem_kernel<float2>, attr[1]);
-    qr_factor_smem_kernel<float2><<<njobs, kT, smem, s>>>(d_jobs);
-  }
-  return (int)cudaGetLastError();
-}
 int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,
                           cudaStream_t s) {
   if (njobs <= 0 || total_cols <= 0) return 0;
@@ -1136,27 +732,6 @@ int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njob
   const int grid = (total_cols + kW - 1) / kW;
   if (es == 16) qr_solve_kernel<double2><<<grid, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
   else qr_solve_kernel<float2><<<grid, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
-  return (int)cudaGetLastError();
-}
-size_t aifmm_compress_smem_bytes(int m, int rK, int c, int rb, int es) {
-  const int n1 = rK + c, s1 = std::min(m, n1), n2 = rb + s1, s2 = std::min(c, n2);
-  if (m > 1024 || c > 1024) return 0;
-  size_t b = std::max(aifmm_qr_smem_bytes(m, n1, es), aifmm_qr_smem_bytes(c, n2, es));
-  b = std::max(b, aifmm_formq_smem_bytes(m, s1, s1, es));
-  b = std::max(b, aifmm_formq_smem_bytes(c, s2, s2, es));
-  return b <= (size_t(200) << 10) ? b : 0;
-}
-int aifmm_launch_compress_p2p(const CompressJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s) {
-  if (njobs <= 0) return 0;
-  if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  static bool attr[2] = {false, false};
-  if (es == 16) {
-    smem_attr_once(compress_p2p_kernel<double2>, attr[0]);
-    compress_p2p_kernel<double2><<<njobs, kT, smem, s>>>(d_jobs);
-  } else {
-    smem_attr_once(compress_p2p_kernel<float2>, attr[1]);
-    compress_p2p_kernel<float2><<<njobs, kT, smem, s>>>(d_jobs);
-  }
   return (int)cudaGetLastError();
 }
 int aifmm_launch_formq(const FormQJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,

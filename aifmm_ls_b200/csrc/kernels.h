@@ -123,7 +123,7 @@ struct CompressJob {
   void* nPt;                       // out: c x rr (ld c), room for min(c, rb + min(m, rK + c)) columns
   void* M2Lo; int ldO;             // out: rc x rr
   int* ranks;                      // out: rc, rr
-  // scratch
+  // scratch (down to info: the shared-memory QR only)
   void* Acol;                      // m x (rK + c)
   void* Arow;                      // c x (rb + rc)
   void* tau; int* perm; int* info;
@@ -156,6 +156,16 @@ int aifmm_launch_qr_solve_warp(const SolveJob* d_jobs, const int* d_cta_off, int
                                int nzpmax, int es, cudaStream_t s);
 // one CTA per factorisation, the matrix in shared memory (aifmm_qr_smem_bytes)
 int aifmm_launch_qr_factor_smem(const QRJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s);
+// the columns in registers: the kernel class of an m x n block, -1 if no class holds it
+int aifmm_qr_class(int m, int n);
+int aifmm_launch_qr_factor_reg(const QRJob* d_jobs, int njobs, int cls, int n, int es, cudaStream_t s);
+// the fused compression on the register QR, and on the shared-memory QR where the
+// class is -1
+int aifmm_compress_class(int m, int rK, int c, int rb, int es);
+bool aifmm_compress_class_holds(int cls, int ncol);
+size_t aifmm_compress_reg_smem_bytes(int cls, int m, int rK, int c, int rb, int es);
+int aifmm_launch_compress_reg(const CompressJob* d_jobs, int njobs, int cls, int n, size_t smem, int es,
+                              cudaStream_t s);
 // shared memory the fused compression needs for these sizes (0: does not fit)
 size_t aifmm_compress_smem_bytes(int m, int rK, int c, int rb, int es);
 int aifmm_launch_compress_p2p(const CompressJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s);

@@ -684,21 +684,31 @@ struct aifmm_problem {
   int qr_es = 16, solve_es = 16, formq_es = 16;  // element size of each pending batch
   void flush_qr() {
     if (qj.empty()) return;
-    std::vector<QRJob> small, large;
-    size_t smem = 0;
-    double fl_small = 0, fl_large = 0;
+    // by kernel: the register kernels' classes, the shared-memory kernel (key -1),
+    // and the global-memory kernel for what neither holds
+    struct Group { std::vector<QRJob> jobs; int n = 0; size_t smem = 0; double fl = 0; };
+    std::map<int, Group> groups;
+    std::vector<QRJob> large;
+    double fl_large = 0;
     const int es = qr_es;
     for (auto& j : qj) {
+      const int cls = aifmm_qr_class(j.m, j.n);
       const size_t b = aifmm_qr_smem_bytes(j.m, j.n, es);
-      if (b <= size_t(200) << 10) { small.push_back(j); smem = std::max(smem, b); fl_small += qr_flops(j.m, j.n); }
-      else { large.push_back(j); fl_large += qr_flops(j.m, j.n); }
+      if (cls < 0 && b > size_t(200) << 10) { large.push_back(j); fl_large += qr_flops(j.m, j.n); continue; }
+      Group& g = groups[cls];
+      g.jobs.push_back(j);
+      g.n = std::max(g.n, j.n);
+      g.smem = std::max(g.smem, b);
+      g.fl += qr_flops(j.m, j.n);
     }
-    if (!small.empty()) {
-      const QRJob* dq = stage.put(small, cur);
+    for (auto& kv : groups) {
+      Group& g = kv.second;
+      const QRJob* dq = stage.put(g.jobs, cur);
       cudaEvent_t a;
       const bool pr = prof_begin(0, a);
-      KL(aifmm_launch_qr_factor_smem(dq, (int)small.size(), smem, es, cur));
-      if (pr) prof_end(0, a, fl_small);
+      if (kv.first >= 0) KL(aifmm_launch_qr_factor_reg(dq, (int)g.jobs.size(), kv.first, g.n, es, cur));
+      else KL(aifmm_launch_qr_factor_smem(dq, (int)g.jobs.size(), g.smem, es, cur));
+      if (pr) prof_end(0, a, g.fl);
     }
     if (!large.empty()) {
       const QRJob* dq = stage.put(large, cur);
@@ -1635,6 +1645,9 @@ struct aifmm_problem {
     const int kk[2] = {k, b}, bb[2] = {b, k};
     CompressOut* out[2] = {&kb, &bk};
     size_t smem = 0;
+    // both directions on the register QR when its class holds them, else both on the
+    // shared-memory QR
+    int cls[2], ncol = 0;
     for (int s = 0; s < 2; ++s) {
       Box& K = T[j][kk[s]];
       Box& Bb = T[j][bb[s]];
@@ -1646,6 +1659,21 @@ struct aifmm_problem {
       const size_t need = aifmm_compress_smem_bytes(K.L2P.r, K.L2P.c, Pkb.c, Bb.P2M.r, es_);
       if (need == 0) return false;
       smem = std::max(smem, need);
+      cls[s] = aifmm_compress_class(K.L2P.r, K.L2P.c, Pkb.c, Bb.P2M.r, es_);
+      const int n1 = K.L2P.c + Pkb.c;
+      ncol = std::max(ncol, std::max(n1, Bb.P2M.r + std::min(K.L2P.r, n1)));
+    }
+    int cl = std::max(cls[0], cls[1]);
+    if (std::min(cls[0], cls[1]) < 0 || !aifmm_compress_class_holds(cl, ncol)) cl = -1;
+    if (cl >= 0) {
+      size_t need = 0;
+      for (int s = 0; s < 2; ++s) {
+        Box& K = T[j][kk[s]];
+        const Blk& Pkb = K.P2P[bb[s]];
+        need = std::max(need, aifmm_compress_reg_smem_bytes(cl, K.L2P.r, K.L2P.c, Pkb.c, T[j][bb[s]].P2M.r, es_));
+      }
+      if (need <= (size_t(200) << 10)) smem = need;
+      else cl = -1;
     }
     std::vector<CompressJob> jobs(2);
     int* ranks = static_cast<int*>(scratch.get(sizeof(int) * 4));
@@ -1674,11 +1702,16 @@ struct aifmm_problem {
       J.M2Lo = out[s]->M2L.p.v(); J.ldO = out[s]->M2L.ld;
       J.ranks = ranks + 2 * s;
       auto cg = [&](long elems) { return scratch.get((size_t)es_ * std::max(1L, elems)); };
-      J.Acol = cg((long)m * n1);
-      J.Arow = cg((long)c * n2max);
-      J.tau = cg(std::max(rcmax[s], rrmax[s]));
-      J.perm = static_cast<int*>(scratch.get(sizeof(int) * std::max(1, std::max(n1, n2max))));
-      J.info = static_cast<int*>(scratch.get(sizeof(int) * 4));
+      if (cl < 0) {
+        J.Acol = cg((long)m * n1);
+        J.Arow = cg((long)c * n2max);
+        J.tau = cg(std::max(rcmax[s], rrmax[s]));
+        J.perm = static_cast<int*>(scratch.get(sizeof(int) * std::max(1, std::max(n1, n2max))));
+        J.info = static_cast<int*>(scratch.get(sizeof(int) * 4));
+      } else {
+        J.Acol = J.Arow = J.tau = nullptr;
+        J.perm = J.info = nullptr;
+      }
       J.Rkp = cg((long)rcmax[s] * c);
       J.Rk = cg((long)rcmax[s] * rK);
       J.Rn = cg((long)rrmax[s] * rb);
@@ -1687,7 +1720,8 @@ struct aifmm_problem {
     }
     flush_all();
     const CompressJob* dj = stage.put(jobs, st);
-    KL(aifmm_launch_compress_p2p(dj, 2, smem, es_, st));
+    if (cl >= 0) KL(aifmm_launch_compress_reg(dj, 2, cl, ncol, smem, es_, st));
+    else KL(aifmm_launch_compress_p2p(dj, 2, smem, es_, st));
     sync();
     int rk[4];
     d2h(rk, ranks, sizeof rk);
