@@ -370,33 +370,59 @@ __global__ void __launch_bounds__(kT) formq_kernel(const FormQJob* __restrict__ 
 }
 
 // ---------------------------------------------------------------- GEMM
-// C = alpha sum_t op(A_t) op(B_t) + beta C over a list of GEMMs, one 32 x 32
-// tile of C per CTA (16 x 16 threads, 2 x 2 outputs each).  The k dimension of
-// all terms is walked in chunks of 32; the next chunk's global loads are issued
-// into registers before the current chunk is multiplied out of shared memory,
-// so one load latency hides behind each chunk's arithmetic.  Accumulation runs
-// over k in increasing order, term after term.
-// Output tile TM x TN(SJ) with TN = 16 SJ: SJ = 2 gives 32 x 32 tiles, SJ = 1
-// gives 32 x 16 tiles for thin products (a block times a few right-hand sides).
-constexpr int TM = 32, TK = 32;
-template <int SJ>
-__device__ __forceinline__ void gemm_fetch(const GemmTerm& T, int k0, int row0, int col0, int m, int n,
-                                           double2 (&ra)[4], double2 (&rb)[2 * SJ]) {
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int e = threadIdx.x + 256 * u;
-    const int kk = e / TM, ii = e % TM, gi = row0 + ii, gk = k0 + kk;
-    ra[u] = make_double2(0.0, 0.0);
-    const double2* A = static_cast<const double2*>(T.A);
-    if (gi < m && gk < T.k) ra[u] = T.opA ? cconj(A[gk + (size_t)gi * T.lda]) : A[gi + (size_t)gk * T.lda];
-  }
-#pragma unroll
-  for (int u = 0; u < 2 * SJ; ++u) {
-    const int e = threadIdx.x + 256 * u;
-    const int jj = e / TK, kb = e % TK, gj = col0 + jj, gkb = k0 + kb;
-    rb[u] = make_double2(0.0, 0.0);
-    const double2* B = static_cast<const double2*>(T.B);
-    if (gj < n && gkb < T.k) rb[u] = T.opB ? cconj(B[gj + (size_t)gkb * T.ldb]) : B[gkb + (size_t)gj * T.ldb];
+// C = alpha sum_t op(A_t) op(B_t) + beta C over a list of products.  A warp owns one
+// 8 x 8 sub-tile of C, a CTA WM x WN of them.  The k dimension of all terms is
+// walked in chunks of up to tk, which cp.async brings into a ring of NS buffers (tk <=
+// 48; NS = 1: products of a single chunk, tk <= 96).  With NS > 1 a second set of as many warps
+// fetches, so that its address arithmetic runs beside the products.  Accumulation
+// runs over k in increasing order, term after term.
+// What bounds it: latency -- the descriptor, the operands' way from L2, the
+// instructions that fetch a chunk, and the DMMAs of a sub-tile one after the other
+// (four for every 4 of k at 16 cycles each) -- so tiles are small and many: 16 x 16
+// for blocks, 32 x 8 for up to 8 right-hand sides; 32 x 32 reads its operands half as
+// often, for batches that fill the chip (flush_gemm).
+// An operand lies in shared memory as it lies in global memory, contiguous along the
+// rows of op = 0's A and op = 1's B, else along k; leading dimensions = 2 (mod 8)
+// and = 4 (mod 8) keep the fragment loads free of bank conflicts either way.  Rows and
+// columns outside C are not loaded: what they hold reaches only outputs that are not
+// written.
+constexpr int kGemmTK = 48, kGemmTK1 = 96, kGemmTerms = 64;  // chunk of a ring, of a single buffer
+__host__ __device__ constexpr int gemm_ld_row(int t) { return t + 2; }                       // t = 8, 16, 32
+__host__ __device__ constexpr int gemm_ld_k(int tk) { return (tk & 7) == 4 ? tk : tk + 4; }  // tk = 0 (mod 4)
+__host__ __device__ constexpr int gemm_area(int t, int tk) {
+  return tk * gemm_ld_row(t) > t * gemm_ld_k(tk) ? tk * gemm_ld_row(t) : t * gemm_ld_k(tk);
+}
+
+__device__ __forceinline__ void cp_async(double2* dst, const double2* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async(float2* dst, const float2* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+// A chunk of one operand, T threads: element (r, k), r < rows (of a tile of TR), k < kc, from
+// src[r + k ld] (along_r) or src[k + r ld].
+template <typename C, int TR, int T>
+__device__ __forceinline__ void gemm_fetch(C* dst, const C* src, int ld, bool along_r, int rows, int kc, int ldk) {
+  const int tid = threadIdx.x % T;
+  if (along_r) {
+    const int r = tid % TR, k0 = tid / TR;
+    if (r < rows) {
+      const C* s = src + r + (size_t)k0 * ld;
+      C* d = dst + k0 * gemm_ld_row(TR) + r;
+      const size_t step = (size_t)(T / TR) * ld;
+#pragma unroll 3
+      for (int k = k0; k < kc; k += T / TR, s += step, d += (T / TR) * gemm_ld_row(TR)) cp_async(d, s);
+    }
+  } else {
+    const int k0 = tid & 15;
+    for (int r = tid >> 4; r < rows; r += T / 16) {
+      const C* s = src + (size_t)r * ld;
+      C* d = dst + r * ldk;
+#pragma unroll 3
+      for (int k = k0; k < kc; k += 16) cp_async(d + k, s + k);
+    }
   }
 }
 // d += a b for one m8n8k4 FP64 tensor-core product (each lane: one A element,
@@ -406,148 +432,148 @@ __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
       : "+d"(d[0]), "+d"(d[1])
       : "d"(a), "d"(b));
 }
-template <int SJ>
-__global__ void __launch_bounds__(256) gemm_kernel(const GemmDesc* __restrict__ ds, const GemmTerm* __restrict__ terms,
-                                                   const int* __restrict__ tile_off, int nd) {
-  constexpr int TN = 16 * SJ;
-  const int bid = blockIdx.x;
-  int lo = 0, hi = nd - 1;
-  while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (tile_off[mid] <= bid) lo = mid; else hi = mid - 1; }
-  const GemmDesc D = ds[lo];
-  const int t = bid - tile_off[lo];
-  const int tiles_m = (D.m + TM - 1) / TM;
-  const int tm = t % tiles_m, tn = t / tiles_m;
-  __shared__ double2 As[TK][TM + 1];
-  __shared__ double2 Bs[TK][TN + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int si = warp & 3, sj0 = SJ * (warp >> 2);
-  double cr[SJ][2], ci[SJ][2];
-#pragma unroll
-  for (int q = 0; q < SJ; ++q) cr[q][0] = cr[q][1] = ci[q][0] = ci[q][1] = 0.0;
-  const int row0 = tm * TM, col0 = tn * TN;
-  int tt = 0, k0 = 0;
-  GemmTerm T{};
-  bool have = false;
-  for (; tt < D.nterms; ++tt) { T = terms[D.term0 + tt]; if (T.k > 0) { have = true; break; } }
-  double2 ra[4], rb[2 * SJ];
-  if (have) gemm_fetch<SJ>(T, k0, row0, col0, D.m, D.n, ra, rb);
-  while (have) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e = threadIdx.x + 256 * u;
-      As[e / TM][e % TM] = ra[u];
-    }
-#pragma unroll
-    for (int u = 0; u < 2 * SJ; ++u) {
-      const int e = threadIdx.x + 256 * u;
-      Bs[e % TK][e / TK] = rb[u];
-    }
-    __syncthreads();
-    // issue the next chunk's loads (possibly the next term's) before the arithmetic
-    k0 += TK;
-    bool next = true;
-    if (k0 >= T.k) {
-      next = false;
-      k0 = 0;
-      for (++tt; tt < D.nterms; ++tt) { T = terms[D.term0 + tt]; if (T.k > 0) { next = true; break; } }
-    }
-    if (next) gemm_fetch<SJ>(T, k0, row0, col0, D.m, D.n, ra, rb);
-    // FP64 tensor cores: mma.sync m8n8k4 (DMMA).  Warp w owns the 8x8 output
-    // sub-tiles (si, sj0 .. sj0 + SJ - 1) of the tile; a complex product is four
-    // real products, Cr += Ar Br + (-Ai) Bi and Ci += Ar Bi + Ai Br.
-    // Fragments (PTX ISA, mma.m8n8k4 .f64): A row = lane/4, col = lane%4;
-    // B row = lane%4, col = lane/4; C row = lane/4, cols 2(lane%4) + {0, 1}.
-#pragma unroll
-    for (int k4 = 0; k4 < TK; k4 += 4) {
-      const double2 a = As[k4 + (lane & 3)][si * 8 + (lane >> 2)];
-      const double ar = a.x, ai = a.y, nai = -a.y;
-#pragma unroll
-      for (int q = 0; q < SJ; ++q) {
-        const double2 b = Bs[k4 + (lane & 3)][(sj0 + q) * 8 + (lane >> 2)];
-        dmma884(cr[q], ar, b.x);
-        dmma884(cr[q], nai, b.y);
-        dmma884(ci[q], ar, b.y);
-        dmma884(ci[q], ai, b.x);
-      }
-    }
-    __syncthreads();
-    have = next;
+
+// One 8 x 8 sub-tile of a chunk of kc; element (i, k) of A at i ai + k ak, (k, j) of B
+// at k bk + j bj.  complex128: FP64 tensor cores, a complex product as four real
+// ones, Cr += Ar Br + (-Ai) Bi and Ci += Ar Bi + Ai Br, k zero-padded to a multiple of
+// 4.  Fragments (PTX ISA, mma.m8n8k4 .f64): A row = lane/4, col = lane%4; B row =
+// lane%4, col = lane/4; C row = lane/4, cols 2(lane%4) + {0, 1}.
+__device__ __forceinline__ void gemm_chunk(const double2* A, const double2* B, int kc, int ai, int ak, int bk, int bj,
+                                           int ca, int cb, int lane, double (&cr)[2], double (&ci)[2]) {
+  const int kl = lane & 3;
+  const double2* a_ = A + (lane >> 2) * ai + kl * ak;
+  const double2* b_ = B + kl * bk + (lane >> 2) * bj;
+  const double sa = ca ? -1.0 : 1.0, sb = cb ? -1.0 : 1.0;
+#pragma unroll 3
+  for (int k4 = 0; k4 < kc; k4 += 4, a_ += 4 * ak, b_ += 4 * bk) {
+    double2 a = make_double2(0.0, 0.0), b = a;
+    if (k4 + kl < kc) { a = *a_; b = *b_; }
+    a.y *= sa;
+    b.y *= sb;
+    dmma884(cr, a.x, b.x);
+    dmma884(cr, -a.y, b.y);
+    dmma884(ci, a.x, b.y);
+    dmma884(ci, a.y, b.x);
   }
-  const bool zero_beta = D.beta.x == 0.0 && D.beta.y == 0.0;
-#pragma unroll
-  for (int q = 0; q < SJ; ++q)
+}
+// The complex64 products of the mixed form: FP32 fused multiply-adds on the CUDA
+// cores, the outputs of a lane where the DMMA's accumulators are.
+__device__ __forceinline__ void gemm_chunk(const float2* A, const float2* B, int kc, int ai, int ak, int bk, int bj,
+                                           int ca, int cb, int lane, float (&cr)[2], float (&ci)[2]) {
+  const float2* a_ = A + (lane >> 2) * ai;
+  const float2* b_ = B + 2 * (lane & 3) * bj;
+#pragma unroll 4
+  for (int kk = 0; kk < kc; ++kk) {
+    float2 a = a_[kk * ak];
+    if (ca) a.y = -a.y;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int gi = row0 + si * 8 + (lane >> 2), gj = col0 + (sj0 + q) * 8 + 2 * (lane & 3) + h;
-      if (gi < D.m && gj < D.n) {
-        double2* c = static_cast<double2*>(D.C) + gi + (size_t)gj * D.ldc;
-        double2 v = cmul(D.alpha, make_double2(cr[q][h], ci[q][h]));
-        if (!zero_beta) v = cadd(v, cmul(D.beta, *c));
-        *c = v;
-      }
+      float2 b = b_[kk * bk + h * bj];
+      if (cb) b.y = -b.y;
+      const float2 c = cfma(a, b, make_float2(cr[h], ci[h]));
+      cr[h] = c.x;
+      ci[h] = c.y;
     }
+  }
 }
 
-// The complex64 products of the mixed form: the same tiles and descriptor
-// lists, FP32 fused multiply-adds with FP32 accumulation on the CUDA cores
-// (these products are a few tens of rows deep: their time is the launch and
-// the load latency, not the arithmetic).  Thread t computes rows t % 32 of
-// the tile in columns t / 32 + 8 q.
-template <int SJ>
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const GemmDesc* __restrict__ ds,
-                                                       const GemmTerm* __restrict__ terms,
-                                                       const int* __restrict__ tile_off, int nd) {
-  constexpr int TN = 16 * SJ, NQ = TN / 8;
-  const int bid = blockIdx.x;
-  int lo = 0, hi = nd - 1;
-  while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (tile_off[mid] <= bid) lo = mid; else hi = mid - 1; }
-  const GemmDesc D = ds[lo];
-  const int t = bid - tile_off[lo];
+template <typename C, int WM, int WN, int NS>
+__global__ void __launch_bounds__(32 * WM * WN * (NS == 1 ? 1 : 2)) gemm_kernel(const GemmDesc* __restrict__ ds,
+                                                            const GemmTerm* __restrict__ terms,
+                                                            const int2* __restrict__ tiles, int tk) {
+  constexpr int T = 32 * WM * WN, TM = 8 * WM, TN = 8 * WN, LDA = gemm_ld_row(TM), LDB = gemm_ld_row(TN);
+  using R = typename cplx<C>::R;
+  extern __shared__ double2 gsm_raw[];
+  C* ring = reinterpret_cast<C*>(gsm_raw);
+  __shared__ GemmTerm st[NS == 1 ? 1 : kGemmTerms];
+  const int2 tile = __ldg(&tiles[blockIdx.x]);
+  const GemmDesc D = ds[tile.x];
+  const int ldk = gemm_ld_k(tk), offb = gemm_area(TM, tk), stage = offb + gemm_area(TN, tk);
   const int tiles_m = (D.m + TM - 1) / TM;
-  const int tm = t % tiles_m, tn = t / tiles_m;
-  __shared__ float2 As[TK][TM + 1];
-  __shared__ float2 Bs[TK][TN + 1];
-  const int ti = threadIdx.x & 31, tj = threadIdx.x >> 5;
-  float2 acc[NQ];
+  const int row0 = (tile.y % tiles_m) * TM, col0 = (tile.y / tiles_m) * TN;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int si = 8 * (warp % WM), sj = 8 * (warp / WM);
+  const int rows = min(TM, D.m - row0), cols = min(TN, D.n - col0);
+  const bool mine = si < rows && sj < cols;  // else the sub-tile lies outside C
+  R cr[2] = {0, 0}, ci[2] = {0, 0};
+  auto fetch = [&](const GemmTerm& F, int k0, C* As) {
+    const int kc = min(tk, F.k - k0);
+    const C* A = static_cast<const C*>(F.A);
+    const C* B = static_cast<const C*>(F.B);
+    gemm_fetch<C, TM, T>(As, F.opA ? A + k0 + (size_t)row0 * F.lda : A + row0 + (size_t)k0 * F.lda, F.lda, !F.opA, rows,
+                         kc, ldk);
+    gemm_fetch<C, TN, T>(As + offb, F.opB ? B + col0 + (size_t)k0 * F.ldb : B + k0 + (size_t)col0 * F.ldb, F.ldb,
+                         F.opB, cols, kc, ldk);
+  };
+  auto multiply = [&](const GemmTerm& G, int k0, const C* As) {
+    const int ai = G.opA ? ldk : 1, ak = G.opA ? 1 : LDA, bk = G.opB ? LDB : 1, bj = G.opB ? 1 : ldk;
+    gemm_chunk(As + si * ai, As + offb + sj * bj, min(tk, G.k - k0), ai, ak, bk, bj, G.opA, G.opB, lane, cr, ci);
+  };
+  if (NS == 1) {  // at most one term of at most tk
+    if (D.nterms > 0) {
+      const GemmTerm G = terms[D.term0];
+      if (G.k > 0) {
+        fetch(G, 0, ring);
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        if (mine) multiply(G, 0, ring);
+      }
+    }
+  } else {
+    {
+      const int words = min(D.nterms, kGemmTerms) * (int)(sizeof(GemmTerm) / 8);
+      const unsigned long long* src = reinterpret_cast<const unsigned long long*>(terms + D.term0);
+      for (int e = tid; e < words; e += 2 * T) reinterpret_cast<unsigned long long*>(st)[e] = __ldg(&src[e]);
+    }
+    __syncthreads();
+    auto term = [&](int t) { return t < kGemmTerms ? st[t] : terms[D.term0 + t]; };
+    if (tid >= T) {  // the fetching warps: one barrier per chunk, after the chunk has arrived
+      int ft = 0, fk = 0, slot = 0, chunks = 0;
+      GemmTerm F{};
+      if (D.nterms > 0) F = term(0);
+      auto next = [&]() {  // one chunk into the next buffer of the ring (none left: an empty group)
+        while (ft < D.nterms && fk >= F.k) {
+          fk = 0;
+          if (++ft < D.nterms) F = term(ft);
+        }
+        if (ft < D.nterms) {
+          fetch(F, fk, ring + slot * stage);
+          fk += tk;
+          ++chunks;
+        }
+        if (++slot == NS) slot = 0;
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+      };
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) acc[q] = make_float2(0.f, 0.f);
-  const int row0 = tm * TM, col0 = tn * TN;
-  for (int tt = 0; tt < D.nterms; ++tt) {
-    const GemmTerm T = terms[D.term0 + tt];
-    const float2* A = static_cast<const float2*>(T.A);
-    const float2* B = static_cast<const float2*>(T.B);
-    for (int k0 = 0; k0 < T.k; k0 += TK) {
-      for (int e = threadIdx.x; e < TK * TM; e += 256) {
-        const int kk = e / TM, ii = e % TM, gi = row0 + ii, gk = k0 + kk;
-        float2 v = make_float2(0.f, 0.f);
-        if (gi < D.m && gk < T.k) v = T.opA ? cconj(A[gk + (size_t)gi * T.lda]) : A[gi + (size_t)gk * T.lda];
-        As[kk][ii] = v;
+      for (int q = 0; q < NS - 1; ++q) next();
+      for (int c = 0; c < chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(NS >= 2 ? NS - 2 : 0) : "memory");
+        __syncthreads();  // chunk c has arrived, and the buffer of chunk c - 1 is free
+        next();
       }
-      for (int e = threadIdx.x; e < TK * TN; e += 256) {
-        const int jj = e / TK, kb = e % TK, gj = col0 + jj, gk = k0 + kb;
-        float2 v = make_float2(0.f, 0.f);
-        if (gj < D.n && gk < T.k) v = T.opB ? cconj(B[gj + (size_t)gk * T.ldb]) : B[gk + (size_t)gj * T.ldb];
-        Bs[kb][jj] = v;
+      return;
+    }
+    int slot = 0;
+    for (int t = 0; t < D.nterms; ++t) {
+      const GemmTerm G = term(t);
+      for (int k0 = 0; k0 < G.k; k0 += tk) {
+        __syncthreads();
+        if (mine) multiply(G, k0, ring + slot * stage);
+        if (++slot == NS) slot = 0;
       }
-      __syncthreads();
-      const int kmax = min(TK, T.k - k0);
-      for (int kk = 0; kk < kmax; ++kk) {
-        const float2 a = As[kk][ti];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q] = cfma(a, Bs[kk][tj + 8 * q], acc[q]);
-      }
-      __syncthreads();
     }
   }
   const bool zero_beta = D.beta.x == 0.0 && D.beta.y == 0.0;
-  const float2 alpha = cplx<float2>::from(D.alpha), beta = cplx<float2>::from(D.beta);
-  const int gi = row0 + ti;
+  const C alpha = cplx<C>::from(D.alpha), beta = cplx<C>::from(D.beta);
 #pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    const int gj = col0 + tj + 8 * q;
-    if (gi < D.m && gj < D.n) {
-      float2* c = static_cast<float2*>(D.C) + gi + (size_t)gj * D.ldc;
-      float2 v = cmul(alpha, acc[q]);
+  for (int h = 0; h < 2; ++h) {
+    const int i = si + (lane >> 2), j = sj + 2 * (lane & 3) + h;
+    if (i < rows && j < cols) {
+      C* c = static_cast<C*>(D.C) + row0 + i + (size_t)(col0 + j) * D.ldc;
+      C s;
+      s.x = cr[h];
+      s.y = ci[h];
+      C v = cmul(alpha, s);
       if (!zero_beta) v = cadd(v, cmul(beta, *c));
       *c = v;
     }
@@ -743,18 +769,44 @@ int aifmm_launch_formq(const FormQJob* d_jobs, const int* d_col_off, int njobs, 
   else formq_kernel<float2><<<grid, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
   return (int)cudaGetLastError();
 }
-int aifmm_launch_gemm(const GemmDesc* d, const GemmTerm* d_terms, const int* d_tile_off, int nd, int total_tiles,
-                      cudaStream_t s, int tile_cols, int es) {
-  if (nd <= 0 || total_tiles <= 0) return 0;
-  if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  if (es == 16) {
-    if (tile_cols == 16) gemm_kernel<1><<<total_tiles, 256, 0, s>>>(d, d_terms, d_tile_off, nd);
-    else gemm_kernel<2><<<total_tiles, 256, 0, s>>>(d, d_terms, d_tile_off, nd);
-  } else {
-    if (tile_cols == 16) gemm_f32_kernel<1><<<total_tiles, 256, 0, s>>>(d, d_terms, d_tile_off, nd);
-    else gemm_f32_kernel<2><<<total_tiles, 256, 0, s>>>(d, d_terms, d_tile_off, nd);
-  }
+namespace {
+template <typename C, int WM, int WN, int NS>
+int launch_gemm_ns(const GemmDesc* d, const GemmTerm* t, const int2* tiles, int ntiles, int tk, cudaStream_t s) {
+  static bool attr = false;
+  smem_attr_once(gemm_kernel<C, WM, WN, NS>, attr);
+  const size_t smem = sizeof(C) * NS * (size_t)(gemm_area(8 * WM, tk) + gemm_area(8 * WN, tk));
+  gemm_kernel<C, WM, WN, NS><<<ntiles, 32 * WM * WN * (NS == 1 ? 1 : 2), smem, s>>>(d, t, tiles, tk);
   return (int)cudaGetLastError();
+}
+template <typename C, int WM, int WN>
+int launch_gemm(const GemmDesc* d, const GemmTerm* t, const int2* tiles, int ntiles, int kmax, int tmax,
+                cudaStream_t s) {
+  // every product one chunk: one buffer, so that many CTAs share an SM
+  if (tmax <= 1 && kmax <= kGemmTK1)
+    return launch_gemm_ns<C, WM, WN, 1>(d, t, tiles, ntiles, std::max(4, (kmax + 3) & ~3), s);
+  const int tk = std::max(4, std::min(kGemmTK, (kmax + 3) & ~3));
+  // few CTAs: four buffers hide more of the load latency; many: three, for more CTAs an SM
+  if (ntiles <= 2 * 148 && 8 * WM < 32) return launch_gemm_ns<C, WM, WN, 4>(d, t, tiles, ntiles, tk, s);
+  return launch_gemm_ns<C, WM, WN, 3>(d, t, tiles, ntiles, tk, s);
+}
+}  // namespace
+void aifmm_gemm_tile(int shape, int* tm, int* tn) {
+  *tm = shape == 16 ? 16 : 32;
+  *tn = shape;
+}
+int aifmm_launch_gemm(const GemmDesc* d, const GemmTerm* d_terms, const int2* d_tiles, int ntiles, int shape, int kmax,
+                      int tmax, cudaStream_t s, int es) {
+  if (ntiles <= 0) return 0;
+  if (!valid_es(es)) return (int)cudaErrorInvalidValue;
+  switch (shape) {
+#define AIFMM_GEMM_CASE(S, WM, WN)                                                                  \
+    case S:                                                                                        \
+      return es == 16 ? launch_gemm<double2, WM, WN>(d, d_terms, d_tiles, ntiles, kmax, tmax, s)   \
+                      : launch_gemm<float2, WM, WN>(d, d_terms, d_tiles, ntiles, kmax, tmax, s);
+    AIFMM_GEMM_CASE(8, 4, 1) AIFMM_GEMM_CASE(16, 2, 2) AIFMM_GEMM_CASE(32, 4, 4)
+#undef AIFMM_GEMM_CASE
+  }
+  return (int)cudaErrorInvalidValue;
 }
 int aifmm_launch_geam(const GeamDesc* d, const long long* d_off, int nd, long long total, cudaStream_t s) {
   if (nd <= 0 || total <= 0) return 0;

@@ -170,9 +170,12 @@ int aifmm_launch_compress_reg(const CompressJob* d_jobs, int njobs, int cls, int
 size_t aifmm_compress_smem_bytes(int m, int rK, int c, int rb, int es);
 int aifmm_launch_compress_p2p(const CompressJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s);
 int aifmm_launch_formq(const FormQJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es, cudaStream_t s);
-// tile_cols: output tile width, 32 (32 x 32 tiles) or 16 (32 x 16 tiles for thin products)
-int aifmm_launch_gemm(const GemmDesc* d, const GemmTerm* d_terms, const int* d_tile_off, int nd, int total_tiles,
-                      cudaStream_t s, int tile_cols, int es = 16);
+// d_tiles: one entry per output tile, (product, tile index down the rows first); shape
+// 8, 16 or 32 columns (aifmm_gemm_tile: 32 x 8, 16 x 16 or 32 x 32 tiles); kmax, tmax:
+// the batch's largest k and number of terms
+void aifmm_gemm_tile(int shape, int* tm, int* tn);
+int aifmm_launch_gemm(const GemmDesc* d, const GemmTerm* d_terms, const int2* d_tiles, int ntiles, int shape, int kmax,
+                      int tmax, cudaStream_t s, int es = 16);
 int aifmm_launch_geam(const GeamDesc* d, const long long* d_off, int nd, long long total, cudaStream_t s);
 int aifmm_launch_norms(const NormDesc* d, int nd, cudaStream_t s);
 int aifmm_launch_equilibrate(const EquilDesc* d, int nd, cudaStream_t s);

@@ -580,8 +580,11 @@ struct aifmm_problem {
   }
   // GEMM output-tile width per product shape, set by autotune(): [0] for batches
   // whose products are all thin (n <= 16 columns, e.g. a block times the
-  // right-hand sides), [1] otherwise
-  int gemm_cols[2] = {32, 32};
+  // right-hand sides), [1] otherwise.  Untuned: 16, the faster one up to 64-row blocks
+  // (72 products of 36 x 36 x 36: 8.4 us against 9.5 us; 2,048: 83 against 148 us; 1,024
+  // of 144 x 144 x 144: 1,991 against 1,793 us).  Products of at most 8 columns take
+  // 32 x 8 tiles (4,096 of 36 x 8 x 36: 53 us; 16 terms of 36: 19 us).
+  int gemm_cols[2] = {16, 16};
   // one element size per batch: a product of the other size flushes the batch first
   int gemm_es = 16;
   void gemm_batch_es(int es) {
@@ -592,24 +595,33 @@ struct aifmm_problem {
     if (gd.empty()) { gt.clear(); return; }
     int nmax = 0;
     for (auto& g : gd) nmax = std::max(nmax, g.n);
-    const int tc = gemm_cols[nmax <= 16 ? 0 : 1];
-    std::vector<int> off(gd.size());
-    int tot = 0;
-    for (size_t i = 0; i < gd.size(); ++i) { off[i] = tot; tot += ((gd[i].m + 31) / 32) * ((gd[i].n + tc - 1) / tc); }
+    const int shape = nmax <= 8 ? 8 : gemm_cols[nmax <= 16 ? 0 : 1];
+    int tm, tn, kmax = 0, tmax = 0;
+    aifmm_gemm_tile(shape, &tm, &tn);
+    std::vector<int2> tiles;
     double fl = 0;
-    for (auto& g : gd)
-      for (int t = 0; t < g.nterms; ++t) fl += 8.0 * g.m * g.n * gt[g.term0 + t].k;
+    for (size_t i = 0; i < gd.size(); ++i) {
+      const GemmDesc& g = gd[i];
+      const long nt = (long)((g.m + tm - 1) / tm) * ((g.n + tn - 1) / tn);
+      if (nt + (long)tiles.size() > INT_MAX) throw Fail(AIFMM_ERR_ARG, "gemm batch too large");
+      for (int t = 0; t < (int)nt; ++t) tiles.push_back(make_int2((int)i, t));
+      for (int t = 0; t < g.nterms; ++t) {
+        kmax = std::max(kmax, gt[g.term0 + t].k);
+        fl += 8.0 * g.m * g.n * gt[g.term0 + t].k;
+      }
+      tmax = std::max(tmax, g.nterms);
+    }
     if (gt.empty()) gt.push_back(GemmTerm{});
     auto ptrs = put_many_({{gt.data(), gt.size() * sizeof(GemmTerm)}, {gd.data(), gd.size() * sizeof(GemmDesc)},
-                           {off.data(), off.size() * sizeof(int)}});
+                           {tiles.data(), tiles.size() * sizeof(int2)}});
     cudaEvent_t a;
     const bool pr = prof_begin(2, a);
     {
       const GemmDesc* d1 = static_cast<const GemmDesc*>(ptrs[1]);
       const GemmTerm* d0 = static_cast<const GemmTerm*>(ptrs[0]);
-      const int* d2 = static_cast<const int*>(ptrs[2]);
-      const int nd = (int)gd.size(), es = gemm_es;
-      KL(run_op([=](cudaStream_t s_) { return aifmm_launch_gemm(d1, d0, d2, nd, tot, s_, tc, es); }));
+      const int2* d2 = static_cast<const int2*>(ptrs[2]);
+      const int nt = (int)tiles.size(), es = gemm_es;
+      KL(run_op([=](cudaStream_t s_) { return aifmm_launch_gemm(d1, d0, d2, nt, shape, kmax, tmax, s_, es); }));
     }
     if (pr) prof_end(2, a, fl);
     gd.clear(); gt.clear();
@@ -2577,14 +2589,14 @@ struct aifmm_problem {
 
   // ---- autotuner: the GEMM tile width per product shape, from timings of both
   // widths on batches shaped like this problem's products (leaf blocks rank x rank,
-  // their products with 8 right-hand sides, and the 4-rank blocks of the level
+  // their products with 16 right-hand sides, and the 4-rank blocks of the level
   // above), CUDA events on the handle's stream; the faster width is kept per shape.
   double tune_ms[2][2] = {{0, 0}, {0, 0}};  // [thin, wide][16, 32]
   void autotune() {
     const int r = rank, R = std::min(4 * rank, 160);
     const int nb = std::max(256, std::min(4096, nleaf / 2));  // the tree need not be built yet
     struct Shape { int m, n, k; };
-    const Shape thin[2] = {{r, 8, r}, {R, 8, R}}, wide[2] = {{r, r, r}, {R, R, R}};
+    const Shape thin[2] = {{r, 16, r}, {R, 16, R}}, wide[2] = {{r, r, r}, {R, R, R}};
     size_t elems = 0;
     for (const Shape* sh : {thin, wide})
       for (int q = 0; q < 2; ++q) elems = std::max(elems, (size_t)sh[q].m * sh[q].k + (size_t)sh[q].k * sh[q].n +

@@ -152,10 +152,10 @@ aifmm_status aifmm_factorize(aifmm_problem* p, int precision, int flags);
  * the work already queued on it, and work queued on it afterwards sees x. */
 aifmm_status aifmm_solve(aifmm_problem* p, int nrhs, const double* b, long ldb, double* x, long ldx, void* stream,
                          int flags);
-/* No counterpart in the reference: pick the batched GEMM's output-tile width (32 x 16 or
+/* No counterpart in the reference: pick the batched GEMM's output-tile width (16 x 16 or
  * 32 x 32) for this handle by timing both on batches shaped like the problem's products
- * (thin: blocks times 8 right-hand sides; wide: block times block), at the leaf rank
- * and at four times it.  ms (may be NULL): 4 timings in ms, [thin 16, thin 32, wide 16,
+ * (thin: blocks times 16 right-hand sides; wide: block times block), at the leaf rank
+ * and at four times it.  Products of at most 8 columns take 32 x 8 tiles either way.  ms (may be NULL): 4 timings in ms, [thin 16, thin 32, wide 16,
  * wide 32]; tile_cols (may be NULL): the chosen widths [thin, wide].  Results do not
  * depend on the choice beyond rounding: both widths sum every product in the same order. */
 aifmm_status aifmm_autotune(aifmm_problem* p, double* ms, int* tile_cols);
