@@ -188,101 +188,6 @@ __global__ void __launch_bounds__(kT) qr_factor_kernel(const QRJob* __restrict__
   qr_factor_body<C>(J, static_cast<C*>(J.a), J.lda, J.norms, J.norms + J.n, J.perm);
 }
 
-// ---------------------------------------------------------------- QR solve (warp per column, registers)
-// One warp per right-hand side; lane l holds rows l, l+32, ... of its column in
-// registers (RPL rows per lane, m <= 32*RPL).  The first nzp columns of the
-// factor and tau are staged once per CTA in shared memory.  Only warp shuffles
-// synchronise: Q^H b reflector by reflector, then column-oriented back
-// substitution with R, then the column permutation.
-template <typename C, int RPL>
-__global__ void __launch_bounds__(kT) qr_solve_warp_kernel(const SolveJob* __restrict__ jobs,
-                                                           const int* __restrict__ cta_off, int njobs) {
-  extern __shared__ double2 fsm_raw[];
-  int lo = 0, hi = njobs - 1;
-  while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (cta_off[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1; }
-  const SolveJob J = jobs[lo];
-  const C* Jqr = static_cast<const C*>(J.qr);
-  const C* Jtau = static_cast<const C*>(J.tau);
-  const C* JB = static_cast<const C*>(J.B);
-  const int m = J.m, n = J.n, nzp = J.info[0];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int c = (blockIdx.x - cta_off[lo]) * kW + w;
-  const int ldf = m | 1;
-  // 1 / R_kk in double (a complex64 pivot near 1e-40 has no FP32 reciprocal), so
-  // that back substitution only multiplies; then the factor and tau
-  double2* rinv = fsm_raw;
-  C* F = reinterpret_cast<C*>(rinv + nzp);  // m x nzp, ld = m|1
-  C* tau = F + (size_t)ldf * nzp;
-  for (int e = threadIdx.x; e < m * nzp; e += kT) {
-    const int i = e % m, j = e / m;
-    F[i + (size_t)j * ldf] = Jqr[i + (size_t)j * J.ldq];
-  }
-  for (int k = threadIdx.x; k < nzp; k += kT) {
-    tau[k] = Jtau[k];
-    rinv[k] = cdiv(make_double2(1.0, 0.0), c2d(Jqr[k + (size_t)k * J.ldq]));
-  }
-  __syncthreads();
-  if (c >= J.nrhs) return;
-  C* x = static_cast<C*>(J.X) + (size_t)c * J.ldx;
-  if (nzp == 0) {
-    for (int i = lane; i < n; i += 32) x[i] = cplx<C>::mk(0.0, 0.0);
-    return;
-  }
-  C b[RPL];
-#pragma unroll
-  for (int r = 0; r < RPL; ++r) {
-    const int i = lane + 32 * r;
-    b[r] = i < m ? (JB ? JB[i + (size_t)c * J.ldb] : cplx<C>::mk(i == c ? 1.0 : 0.0, 0.0)) : cplx<C>::mk(0.0, 0.0);
-  }
-  for (int k = 0; k < nzp; ++k) {
-    const C* v = F + (size_t)k * ldf;
-    C s = cplx<C>::mk(0.0, 0.0);
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int i = lane + 32 * r;
-      if (i > k && i < m) s = cfmac(v[i], b[r], s);
-    }
-    s = warp_sum2(s);
-    const int ok = k & 31, rk = k >> 5;
-    C bk = cplx<C>::mk(0.0, 0.0);
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) if (r == rk) bk = b[r];
-    bk.x = __shfl_sync(0xffffffffu, bk.x, ok);
-    bk.y = __shfl_sync(0xffffffffu, bk.y, ok);
-    const C tw = cmul(tau[k], cadd(bk, s));
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int i = lane + 32 * r;
-      if (i > k && i < m) b[r] = csub(b[r], cmul(v[i], tw));
-      else if (i == k) b[r] = csub(b[r], tw);
-    }
-  }
-  for (int i = nzp - 1; i >= 0; --i) {
-    const int oi = i & 31, ri = i >> 5;
-    C bi = cplx<C>::mk(0.0, 0.0);
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) if (r == ri) bi = b[r];
-    bi.x = __shfl_sync(0xffffffffu, bi.x, oi);
-    bi.y = __shfl_sync(0xffffffffu, bi.y, oi);
-    const C xi = cplx<C>::from(cmul(c2d(bi), rinv[i]));
-    const C* Rc = F + (size_t)i * ldf;
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int l = lane + 32 * r;
-      if (l < i) b[r] = csub(b[r], cmul(Rc[l], xi));
-      else if (l == i) b[r] = xi;
-    }
-  }
-  for (int i = lane; i < n; i += 32) x[i] = cplx<C>::mk(0.0, 0.0);
-  __syncwarp();
-  const C alpha = cplx<C>::from(J.alpha);
-#pragma unroll
-  for (int r = 0; r < RPL; ++r) {
-    const int i = lane + 32 * r;
-    if (i < nzp) x[J.perm[i]] = cmul(alpha, b[r]);
-  }
-}
-
 // ---------------------------------------------------------------- QR solve
 // one warp per right-hand side column
 template <typename C>
@@ -580,6 +485,155 @@ __global__ void __launch_bounds__(32 * WM * WN * (NS == 1 ? 1 : 2)) gemm_kernel(
   }
 }
 
+// ---------------------------------------------------------------- QR solve (registers)
+// Eight lanes own one right-hand side: lane q holds rows q, q + 8, ... in registers,
+// a CTA of 128 threads takes 16 columns (kSolveCols).  The first nzp columns of the
+// factor and tau are staged once per CTA in shared memory; then only shuffles
+// synchronise: Q^H b reflector by reflector, column-oriented back substitution with
+// R, the column permutation.
+// What bounds it: the chain of 2 nzp dependent steps; a reflector's is its dot
+// product over eight lanes (three shuffles: the two upper levels of the sum over 32
+// rows stay in a lane), tau and the update, about 430 cycles of it instruction issue
+// and latency in equal parts.  36 x 36, 12 boxes, 8 columns: 18.6 us (a warp per
+// column: 20.8 us); 300 boxes: 21 us (36 us).
+// Sums run in the order of 32 lanes over the rows (row mod 32), levels 16 to 1.
+constexpr int kSolveCols = 16, kSolveT = 8 * kSolveCols;
+// rows of a phase (x 8): the rows of earlier phases cost nothing in a forward step
+__host__ __device__ constexpr int solve_phase(int rpl) { return (rpl + 5) / 6; }
+
+template <typename C, int RPL, int I0>
+__device__ __forceinline__ void solve_forward(const C* F, int ldf, const C* tau, int m, int nzp, int q, unsigned gm,
+                                              C (&b)[RPL]) {
+  constexpr int I1 = I0 + solve_phase(RPL) < RPL ? I0 + solve_phase(RPL) : RPL;
+  const int kend = min(8 * I1, nzp);
+  constexpr bool ahead = RPL <= 12;  // more rows: the registers do not hold two reflectors
+  C vn[ahead ? RPL : 1];
+  if (ahead) {
+#pragma unroll
+    for (int t = I0; t < RPL; ++t) vn[t] = 8 * I0 < kend && q + 8 * t < m ? F[(size_t)(8 * I0) * ldf + q + 8 * t] : b[t];
+  }
+  for (int k = 8 * I0; k < kend; ++k) {
+    C v[RPL];
+    C s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = cplx<C>::mk(0.0, 0.0);
+#pragma unroll
+    for (int t = I0; t < RPL; ++t) {
+      if (ahead) v[t] = vn[t];
+      else if (q + 8 * t < m) v[t] = F[(size_t)k * ldf + q + 8 * t];
+      if ((unsigned)(q + 8 * t - k - 1) < (unsigned)(m - k - 1)) s[t & 3] = cfmac(v[t], b[t], s[t & 3]);
+    }
+    const C tk = tau[k];
+    if (ahead && k + 1 < kend) {
+#pragma unroll
+      for (int t = I0; t < RPL; ++t)
+        if (q + 8 * t < m) vn[t] = F[(size_t)(k + 1) * ldf + q + 8 * t];
+    }
+    C bk = b[I0];
+#pragma unroll
+    for (int t = I0; t < I1; ++t)
+      if (q + 8 * t == k) bk = b[t];
+    bk.x = __shfl_sync(gm, bk.x, k & 7, 8);
+    bk.y = __shfl_sync(gm, bk.y, k & 7, 8);
+    C z = cadd(cadd(s[0], s[2]), cadd(s[1], s[3]));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      z.x += __shfl_xor_sync(gm, z.x, o);
+      z.y += __shfl_xor_sync(gm, z.y, o);
+    }
+    // (the complex64 form has always fused the other product here)
+    const C tw = sizeof(C) == 16 ? cmul_p(tk, cadd(bk, z)) : cmul_t(tk, cadd(bk, z));
+    const C bn = csub(bk, tw);
+#pragma unroll
+    for (int t = I0; t < RPL; ++t) {
+      if ((unsigned)(q + 8 * t - k - 1) < (unsigned)(m - k - 1)) b[t] = csub(b[t], cmul_p(v[t], tw));
+      if (t < I1 && q + 8 * t == k) b[t] = bn;
+    }
+  }
+  if constexpr (I1 < RPL) {
+    if (nzp > 8 * I1) solve_forward<C, RPL, I1>(F, ldf, tau, m, nzp, q, gm, b);
+  }
+}
+template <typename C, int RPL, int I0>
+__device__ __forceinline__ void solve_backward(const C* F, int ldf, const double2* rinv, int nzp, int q, unsigned gm,
+                                               C (&b)[RPL]) {
+  constexpr int I1 = I0 + solve_phase(RPL) < RPL ? I0 + solve_phase(RPL) : RPL;
+  if constexpr (I1 < RPL) {
+    if (nzp > 8 * I1) solve_backward<C, RPL, I1>(F, ldf, rinv, nzp, q, gm, b);
+  }
+  for (int i = min(nzp, 8 * I1) - 1; i >= 8 * I0; --i) {
+    C r[RPL];
+#pragma unroll
+    for (int t = 0; t < I1; ++t)
+      if (q + 8 * t < i) r[t] = F[(size_t)i * ldf + q + 8 * t];
+    const double2 ri = rinv[i];
+    C bi = b[I0];
+#pragma unroll
+    for (int t = I0; t < I1; ++t)
+      if (q + 8 * t == i) bi = b[t];
+    bi.x = __shfl_sync(gm, bi.x, i & 7, 8);
+    bi.y = __shfl_sync(gm, bi.y, i & 7, 8);
+    const C xi = cplx<C>::from(cmul_p(c2d(bi), ri));
+#pragma unroll
+    for (int t = 0; t < I1; ++t) {
+      if (q + 8 * t < i) b[t] = csub(b[t], cmul_p(r[t], xi));
+      else if (t >= I0 && q + 8 * t == i) b[t] = xi;
+    }
+  }
+}
+
+template <typename C, int RPL>
+__global__ void __launch_bounds__(kSolveT) qr_solve_reg_kernel(const SolveJob* __restrict__ jobs,
+                                                               const int2* __restrict__ ctas) {
+  extern __shared__ double2 fsm_raw[];
+  const int2 at = __ldg(&ctas[blockIdx.x]);  // job, first column
+  const SolveJob J = jobs[at.x];
+  const C* Jqr = static_cast<const C*>(J.qr);
+  const C* Jtau = static_cast<const C*>(J.tau);
+  const C* JB = static_cast<const C*>(J.B);
+  const int m = J.m, n = J.n, nzp = J.info[0];
+  const int tid = threadIdx.x, lane = tid & 31, q = tid & 7, c = at.y + (tid >> 3);
+  const int ldf = m | 1;
+  // 1 / R_kk in double (a complex64 pivot near 1e-40 has no FP32 reciprocal), so
+  // that back substitution only multiplies; then the factor and tau
+  double2* rinv = fsm_raw;
+  C* F = reinterpret_cast<C*>(rinv + nzp);  // m x nzp, ld = m|1
+  C* tau = F + (size_t)ldf * nzp;
+  for (int j = tid >> 5; j < nzp; j += kSolveT / 32)
+    for (int i = lane; i < m; i += 32) cp_async(&F[i + j * ldf], &Jqr[i + (size_t)j * J.ldq]);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  C b[RPL];
+  const bool mine = c < J.nrhs;
+#pragma unroll
+  for (int t = 0; t < RPL; ++t) {
+    const int i = q + 8 * t;
+    b[t] = mine && i < m ? (JB ? JB[i + (size_t)c * J.ldb] : cplx<C>::mk(i == c ? 1.0 : 0.0, 0.0)) : cplx<C>::mk(0.0, 0.0);
+  }
+  for (int k = tid; k < nzp; k += kSolveT) {
+    tau[k] = Jtau[k];
+    rinv[k] = cdiv(make_double2(1.0, 0.0), c2d(Jqr[k + (size_t)k * J.ldq]));
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  if (!mine) return;
+  C* x = static_cast<C*>(J.X) + (size_t)c * J.ldx;
+  const unsigned gm = 0xffu << (lane & ~7);
+  if (nzp > 0) {
+    solve_forward<C, RPL, 0>(F, ldf, tau, m, nzp, q, gm, b);
+    solve_backward<C, RPL, 0>(F, ldf, rinv, nzp, q, gm, b);
+  }
+  if (nzp < n) {
+    for (int i = q; i < n; i += 8) x[i] = cplx<C>::mk(0.0, 0.0);
+    __syncwarp(gm);
+  }
+  const C alpha = cplx<C>::from(J.alpha);
+#pragma unroll
+  for (int t = 0; t < RPL; ++t) {
+    const int i = q + 8 * t;
+    if (i < nzp) x[J.perm[i]] = cmul(alpha, b[t]);
+  }
+}
+
 // ---------------------------------------------------------------- GEAM
 // Element sizes per descriptor: the arithmetic is complex128, a complex64
 // operand is widened on load and a complex64 result rounded on store.
@@ -723,32 +777,29 @@ int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int es, cudaStream_t 
 
 namespace {
 template <typename C>
-int launch_solve_warp(const SolveJob* d_jobs, const int* d_cta_off, int njobs, int total_ctas, int rpl, size_t smem,
-                      cudaStream_t s) {
-  static bool attr[8] = {false, false, false, false, false, false, false, false};
-  switch (rpl) {
-#define AIFMM_SOLVE_CASE(R)                                                               \
-    case R:                                                                               \
-      smem_attr_once(qr_solve_warp_kernel<C, R>, attr[R]);                                \
-      qr_solve_warp_kernel<C, R><<<total_ctas, kT, smem, s>>>(d_jobs, d_cta_off, njobs);  \
-      break;
-    AIFMM_SOLVE_CASE(1) AIFMM_SOLVE_CASE(2) AIFMM_SOLVE_CASE(3) AIFMM_SOLVE_CASE(4)
-    AIFMM_SOLVE_CASE(5) AIFMM_SOLVE_CASE(6) AIFMM_SOLVE_CASE(7)
-#undef AIFMM_SOLVE_CASE
-    default: return (int)cudaErrorInvalidValue;
+int launch_solve_reg(const SolveJob* d_jobs, const int2* d_ctas, int nctas, int mmax, size_t smem, cudaStream_t s) {
+  static bool attr[6] = {false, false, false, false, false, false};
+#define AIFMM_SOLVE_CASE(I, R)                                                      \
+  if (mmax <= 8 * R) {                                                              \
+    smem_attr_once(qr_solve_reg_kernel<C, R>, attr[I]);                             \
+    qr_solve_reg_kernel<C, R><<<nctas, kSolveT, smem, s>>>(d_jobs, d_ctas);         \
+    return (int)cudaGetLastError();                                                 \
   }
-  return (int)cudaGetLastError();
+  AIFMM_SOLVE_CASE(0, 3) AIFMM_SOLVE_CASE(1, 5) AIFMM_SOLVE_CASE(2, 8) AIFMM_SOLVE_CASE(3, 12)
+  AIFMM_SOLVE_CASE(4, 18) AIFMM_SOLVE_CASE(5, 28)
+#undef AIFMM_SOLVE_CASE
+  return (int)cudaErrorInvalidValue;
 }
 }  // namespace
 
-int aifmm_launch_qr_solve_warp(const SolveJob* d_jobs, const int* d_cta_off, int njobs, int total_ctas, int mmax,
-                               int nzpmax, int es, cudaStream_t s) {
-  if (njobs <= 0 || total_ctas <= 0) return 0;
+int aifmm_solve_cols() { return kSolveCols; }
+int aifmm_launch_qr_solve_reg(const SolveJob* d_jobs, const int2* d_ctas, int nctas, int mmax, int nzpmax, int es,
+                              cudaStream_t s) {
+  if (nctas <= 0) return 0;
   if (!valid_es(es)) return (int)cudaErrorInvalidValue;
   const size_t smem = (size_t)es * ((size_t)(mmax | 1) * nzpmax + (size_t)nzpmax) + sizeof(double2) * nzpmax + 64;
-  const int rpl = (mmax + 31) / 32;
-  return es == 16 ? launch_solve_warp<double2>(d_jobs, d_cta_off, njobs, total_ctas, rpl, smem, s)
-                  : launch_solve_warp<float2>(d_jobs, d_cta_off, njobs, total_ctas, rpl, smem, s);
+  return es == 16 ? launch_solve_reg<double2>(d_jobs, d_ctas, nctas, mmax, smem, s)
+                  : launch_solve_reg<float2>(d_jobs, d_ctas, nctas, mmax, smem, s);
 }
 
 int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,

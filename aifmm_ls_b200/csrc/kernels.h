@@ -150,10 +150,12 @@ int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int es, cudaStream_t 
 int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,
                           cudaStream_t s);
 size_t aifmm_qr_smem_bytes(int m, int n, int es);
-// one warp per right-hand side (8 per CTA), the column in registers; m <= 224 and
-// the factor's first nzp columns must fit in shared memory
-int aifmm_launch_qr_solve_warp(const SolveJob* d_jobs, const int* d_cta_off, int njobs, int total_ctas, int mmax,
-                               int nzpmax, int es, cudaStream_t s);
+// eight lanes per right-hand side, the column in registers; m <= 224 and the factor's
+// first nzp columns must fit in shared memory.  d_ctas: (job, first column) of each
+// CTA of aifmm_solve_cols() columns
+int aifmm_solve_cols();
+int aifmm_launch_qr_solve_reg(const SolveJob* d_jobs, const int2* d_ctas, int nctas, int mmax, int nzpmax, int es,
+                              cudaStream_t s);
 // one CTA per factorisation, the matrix in shared memory (aifmm_qr_smem_bytes)
 int aifmm_launch_qr_factor_smem(const QRJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s);
 // the columns in registers: the kernel class of an m x n block, -1 if no class holds it

@@ -749,8 +749,8 @@ struct aifmm_problem {
   }
   void flush_solve() {
     if (sj.empty()) return;
-    // m <= 224 whose factor fits in shared memory: one warp per column with the
-    // column in registers; larger systems (the base level): the global-memory kernel
+    // m <= 224 whose factor fits in shared memory: the columns in registers; larger
+    // systems (the base level): the global-memory kernel
     std::vector<SolveJob> small, large;
     int mmax = 1, nmax = 1;
     const int es = solve_es;
@@ -771,19 +771,19 @@ struct aifmm_problem {
       small.clear();
     }
     if (!small.empty()) {
-      std::vector<int> off(small.size());
-      int tot = 0;
-      for (size_t i = 0; i < small.size(); ++i) { off[i] = tot; tot += (small[i].nrhs + 7) / 8; }
-      auto ptrs = put_many_({{small.data(), small.size() * sizeof(SolveJob)}, {off.data(), off.size() * sizeof(int)}});
+      std::vector<int2> ctas;
+      for (size_t i = 0; i < small.size(); ++i)
+        for (int c = 0; c < small[i].nrhs; c += aifmm_solve_cols()) ctas.push_back(make_int2((int)i, c));
+      auto ptrs = put_many_({{small.data(), small.size() * sizeof(SolveJob)}, {ctas.data(), ctas.size() * sizeof(int2)}});
       double fl = 0;
       for (auto& j : small) { const double mz = std::min(j.m, j.n); fl += (16.0 * j.m * mz - 4.0 * mz * mz) * j.nrhs; }
       cudaEvent_t a;
       const bool pr = prof_begin(1, a);
       {
         const SolveJob* d0 = static_cast<const SolveJob*>(ptrs[0]);
-        const int* d1 = static_cast<const int*>(ptrs[1]);
-        const int nj = (int)small.size();
-        KL(run_op([=](cudaStream_t s_) { return aifmm_launch_qr_solve_warp(d0, d1, nj, tot, mmax, nmax, es, s_); }));
+        const int2* d1 = static_cast<const int2*>(ptrs[1]);
+        const int nc = (int)ctas.size();
+        KL(run_op([=](cudaStream_t s_) { return aifmm_launch_qr_solve_reg(d0, d1, nc, mmax, nmax, es, s_); }));
       }
       if (pr) prof_end(1, a, fl);
     }
