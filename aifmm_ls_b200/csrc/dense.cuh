@@ -54,6 +54,37 @@ __device__ __forceinline__ C cmul_t(C a, C b) {
 __device__ __forceinline__ double cabs2_p(double2 a) { return __fma_rn(a.x, a.x, __dmul_rn(a.y, a.y)); }
 __device__ __forceinline__ double cabs2_p(float2 a) { return cabs2_p(make_double2(a.x, a.y)); }
 
+// Programmatic dependent launch.  The kernels of an elimination step or a solve wave
+// are a chain of launches of a few microseconds each; a kernel launched this way is
+// set up (and reads its descriptors) while the one before it still runs, and waits in
+// pdl_wait until that one has finished and its writes are visible.  Every kernel
+// launched with launch_chain calls both, pdl_wait before its first access to memory that
+// another kernel writes: then a kernel that has finished implies that all before it
+// have.
+__device__ __forceinline__ void pdl_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+int launch_chain(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// Descriptors of a small batch travel in the kernel's parameters: no copy between the
+// launches of a chain.
+template <int BYTES>
+struct Inline {
+  alignas(16) unsigned char b[BYTES];
+};
+
 // the element size of a batch: 16 (complex128) or 8 (complex64)
 inline bool valid_es(int es) { return es == 16 || es == 8; }
 // opt a kernel into the large dynamic shared memory once per process

@@ -1,6 +1,8 @@
 // k_compress.cu -- one direction of compress_P2P (FMM2DTree_find_error.hpp:1532-1559)
 // per CTA, on the register QR or, for blocks that it does not hold, on the
 // shared-memory QR (qr.cuh).
+#include <cstring>
+
 #include "qr.cuh"
 
 namespace {
@@ -146,7 +148,11 @@ __global__ void __launch_bounds__(kT) compress_p2p_kernel(const CompressJob* __r
     C* o = M2Lo + i + (size_t)jj * J.ldO;
     *o = cadd(cconj(Rnp[jj + (size_t)i * ldr_]), *o);
   }
-  if (tid == 0) { J.ranks[0] = rc; J.ranks[1] = rr; }
+  if (tid == 0) {  // may be mapped host memory
+    J.ranks[0] = rc;
+    J.ranks[1] = rr;
+    __threadfence_system();
+  }
 }
 
 // ---- the same with the register QR
@@ -256,6 +262,9 @@ __device__ __forceinline__ void cta_formq_reg(C* F, int ldf, const C* tau, int m
   __syncthreads();
 }
 
+constexpr int kCompressInline = 8;
+using CompressInline = Inline<kCompressInline * sizeof(CompressJob)>;
+
 // Where the operands of the compression live: the factor, the QR's own arrays, then
 // the inputs and the intermediate products as far as shared memory goes; what does
 // not fit stays in global memory (the kernel's code is the same: generic pointers).
@@ -300,11 +309,14 @@ __device__ __forceinline__ C* place(char* smem, size_t off, void* g) {
 }
 
 template <typename C, int RPL>
-__global__ void __launch_bounds__(qr_threads(RPL)) compress_reg_kernel(const CompressJob* __restrict__ jobs) {
+__global__ void __launch_bounds__(qr_threads(RPL)) compress_reg_kernel(const CompressJob* __restrict__ jobs,
+                                                                       const __grid_constant__ CompressInline inl) {
   extern __shared__ double2 csm_raw[];
   __shared__ int info[4];
   char* sm = reinterpret_cast<char*>(csm_raw);
-  const CompressJob J = jobs[blockIdx.x];
+  pdl_begin();
+  const CompressJob J = jobs ? jobs[blockIdx.x] : reinterpret_cast<const CompressJob*>(inl.b)[blockIdx.x];
+  pdl_wait();
   const int m = J.m, rK = J.rK, c = J.c, rb = J.rb, n1 = rK + c, s1 = min(m, n1);
   const CompressLayout L = compress_layout(RPL, m, rK, c, rb, (int)sizeof(C));
   int ldP, ldL, ldM, ldT;
@@ -344,15 +356,21 @@ __global__ void __launch_bounds__(qr_threads(RPL)) compress_reg_kernel(const Com
   cta_gemm_s<C, 0, 0>(Tm, ldc_, rc, rb, rK, Rk, ldc_, M2L, ldT);    // R M2L_kb
   __syncthreads();
   cta_gemm_s<C, 0, 1, true>(static_cast<C*>(J.M2Lo), J.ldO, rc, rr, rb, Tm, ldc_, Rn, ldr_, Rnp, ldr_);
-  if (threadIdx.x == 0) { J.ranks[0] = rc; J.ranks[1] = rr; }
+  if (threadIdx.x == 0) {  // may be mapped host memory
+    J.ranks[0] = rc;
+    J.ranks[1] = rr;
+    __threadfence_system();
+  }
 }
 
 template <typename C, int RPL>
-int launch_compress_reg(const CompressJob* d_jobs, int njobs, int n, size_t smem, cudaStream_t s) {
+int launch_compress_reg(const CompressJob* d_jobs, const CompressJob* h_jobs, int njobs, int n, size_t smem,
+                        cudaStream_t s) {
   static bool attr = false;
   smem_attr_once(compress_reg_kernel<C, RPL>, attr);
-  compress_reg_kernel<C, RPL><<<njobs, threads_for(n), smem, s>>>(d_jobs);
-  return (int)cudaGetLastError();
+  CompressInline inl;
+  if (!d_jobs) memcpy(inl.b, h_jobs, sizeof(CompressJob) * njobs);
+  return launch_chain(compress_reg_kernel<C, RPL>, dim3(njobs), threads_for(n), smem, s, d_jobs, inl);
 }
 }  // namespace
 
@@ -392,15 +410,17 @@ size_t aifmm_compress_reg_smem_bytes(int cls, int m, int rK, int c, int rb, int 
   return compress_layout(kRpl[cls], m, rK, c, rb, es).total;
 }
 // all jobs of one class; n: the largest column count rK + c or rb + min(m, rK + c)
-int aifmm_launch_compress_reg(const CompressJob* d_jobs, int njobs, int cls, int n, size_t smem, int es,
-                              cudaStream_t s) {
+int aifmm_compress_inline_max() { return kCompressInline; }
+int aifmm_launch_compress_reg(const CompressJob* d_jobs, const CompressJob* h_jobs, int njobs, int cls, int n,
+                              size_t smem, int es, cudaStream_t s) {
   if (njobs <= 0) return 0;
+  if (!d_jobs && njobs > kCompressInline) return (int)cudaErrorInvalidValue;
   if (!valid_es(es) || cls < 0 || cls >= kClasses || 4 * n > qr_threads(kRpl[cls])) return (int)cudaErrorInvalidValue;
   switch (kRpl[cls]) {
 #define AIFMM_CASE(R)                                                           \
     case R:                                                                     \
-      return es == 16 ? launch_compress_reg<double2, R>(d_jobs, njobs, n, smem, s) \
-                      : launch_compress_reg<float2, R>(d_jobs, njobs, n, smem, s);
+      return es == 16 ? launch_compress_reg<double2, R>(d_jobs, h_jobs, njobs, n, smem, s) \
+                      : launch_compress_reg<float2, R>(d_jobs, h_jobs, njobs, n, smem, s);
     AIFMM_CASE(5) AIFMM_CASE(9) AIFMM_CASE(16) AIFMM_CASE(24) AIFMM_CASE(36)
 #undef AIFMM_CASE
   }

@@ -14,6 +14,8 @@
 //  * Batched GEMM / GEAM / Frobenius norms.
 // One CTA per factorisation; everything else is batched over descriptor lists.
 #include <algorithm>
+#include <cstring>
+
 #include "dense.cuh"
 #include "entry.cuh"
 
@@ -382,17 +384,38 @@ __device__ __forceinline__ void gemm_chunk(const float2* A, const float2* B, int
   }
 }
 
+// products that travel in the kernel's parameters (kernels.h, GemmOne)
+template <int NS>
+using GemmInline = Inline<NS == 1 ? kGemmInline * (int)sizeof(GemmOne) : 16>;
+
 template <typename C, int WM, int WN, int NS>
 __global__ void __launch_bounds__(32 * WM * WN * (NS == 1 ? 1 : 2)) gemm_kernel(const GemmDesc* __restrict__ ds,
                                                             const GemmTerm* __restrict__ terms,
-                                                            const int2* __restrict__ tiles, int tk) {
+                                                            const int2* __restrict__ tiles, int tk,
+                                                            const __grid_constant__ GemmInline<NS> inl) {
   constexpr int T = 32 * WM * WN, TM = 8 * WM, TN = 8 * WN, LDA = gemm_ld_row(TM), LDB = gemm_ld_row(TN);
   using R = typename cplx<C>::R;
   extern __shared__ double2 gsm_raw[];
   C* ring = reinterpret_cast<C*>(gsm_raw);
   __shared__ GemmTerm st[NS == 1 ? 1 : kGemmTerms];
-  const int2 tile = __ldg(&tiles[blockIdx.x]);
-  const GemmDesc D = ds[tile.x];
+  pdl_begin();
+  int2 tile;
+  GemmDesc D;
+  GemmTerm one{};
+  if (NS == 1 && !ds) {  // products in the parameters: one grid row each
+    const GemmOne& P = reinterpret_cast<const GemmOne*>(inl.b)[blockIdx.y];
+    if ((int)blockIdx.x >= ((P.m + TM - 1) / TM) * ((P.n + TN - 1) / TN)) return;
+    tile = make_int2((int)blockIdx.y, (int)blockIdx.x);
+    D.C = P.C; D.ldc = P.ldc; D.m = P.m; D.n = P.n;
+    D.alpha = make_double2((double)P.alpha, 0.0);
+    D.beta = make_double2((double)P.beta, 0.0);
+    D.term0 = 0; D.nterms = P.k > 0 ? 1 : 0;
+    one.A = P.A; one.B = P.B; one.lda = P.lda; one.ldb = P.ldb; one.opA = P.op & 1; one.opB = P.op >> 1; one.k = P.k;
+  } else {
+    tile = __ldg(&tiles[blockIdx.x]);
+    D = ds[tile.x];
+    if (NS == 1 && D.nterms > 0) one = terms[D.term0];
+  }
   const int ldk = gemm_ld_k(tk), offb = gemm_area(TM, tk), stage = offb + gemm_area(TN, tk);
   const int tiles_m = (D.m + TM - 1) / TM;
   const int row0 = (tile.y % tiles_m) * TM, col0 = (tile.y / tiles_m) * TN;
@@ -415,8 +438,9 @@ __global__ void __launch_bounds__(32 * WM * WN * (NS == 1 ? 1 : 2)) gemm_kernel(
     gemm_chunk(As + si * ai, As + offb + sj * bj, min(tk, G.k - k0), ai, ak, bk, bj, G.opA, G.opB, lane, cr, ci);
   };
   if (NS == 1) {  // at most one term of at most tk
+    pdl_wait();
     if (D.nterms > 0) {
-      const GemmTerm G = terms[D.term0];
+      const GemmTerm G = one;
       if (G.k > 0) {
         fetch(G, 0, ring);
         asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
@@ -431,6 +455,7 @@ __global__ void __launch_bounds__(32 * WM * WN * (NS == 1 ? 1 : 2)) gemm_kernel(
       for (int e = tid; e < words; e += 2 * T) reinterpret_cast<unsigned long long*>(st)[e] = __ldg(&src[e]);
     }
     __syncthreads();
+    pdl_wait();
     auto term = [&](int t) { return t < kGemmTerms ? st[t] : terms[D.term0 + t]; };
     if (tid >= T) {  // the fetching warps: one barrier per chunk, after the chunk has arrived
       int ft = 0, fk = 0, slot = 0, chunks = 0;
@@ -582,12 +607,27 @@ __device__ __forceinline__ void solve_backward(const C* F, int ldf, const double
   }
 }
 
+constexpr int kSolveInline = 30;
+using SolveInline = Inline<kSolveInline * sizeof(SolveJob)>;
+
 template <typename C, int RPL>
 __global__ void __launch_bounds__(kSolveT) qr_solve_reg_kernel(const SolveJob* __restrict__ jobs,
-                                                               const int2* __restrict__ ctas) {
+                                                               const int2* __restrict__ ctas, int early,
+                                                               const __grid_constant__ SolveInline inl) {
   extern __shared__ double2 fsm_raw[];
-  const int2 at = __ldg(&ctas[blockIdx.x]);  // job, first column
-  const SolveJob J = jobs[at.x];
+  pdl_begin();
+  int2 at;  // job, first column
+  SolveJob J;
+  if (jobs) {
+    at = __ldg(&ctas[blockIdx.x]);
+    J = jobs[at.x];
+  } else {  // jobs in the parameters: one grid row each
+    at = make_int2((int)blockIdx.y, (int)blockIdx.x * kSolveCols);
+    J = reinterpret_cast<const SolveJob*>(inl.b)[blockIdx.y];
+    if (at.y >= J.nrhs) return;
+  }
+  // a kept factor (early) is staged while the launch before this one still runs
+  if (!early) pdl_wait();
   const C* Jqr = static_cast<const C*>(J.qr);
   const C* Jtau = static_cast<const C*>(J.tau);
   const C* JB = static_cast<const C*>(J.B);
@@ -602,16 +642,17 @@ __global__ void __launch_bounds__(kSolveT) qr_solve_reg_kernel(const SolveJob* _
   for (int j = tid >> 5; j < nzp; j += kSolveT / 32)
     for (int i = lane; i < m; i += 32) cp_async(&F[i + j * ldf], &Jqr[i + (size_t)j * J.ldq]);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
+  for (int k = tid; k < nzp; k += kSolveT) {
+    tau[k] = Jtau[k];
+    rinv[k] = cdiv(make_double2(1.0, 0.0), c2d(Jqr[k + (size_t)k * J.ldq]));
+  }
+  if (early) pdl_wait();
   C b[RPL];
   const bool mine = c < J.nrhs;
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
     const int i = q + 8 * t;
     b[t] = mine && i < m ? (JB ? JB[i + (size_t)c * J.ldb] : cplx<C>::mk(i == c ? 1.0 : 0.0, 0.0)) : cplx<C>::mk(0.0, 0.0);
-  }
-  for (int k = tid; k < nzp; k += kSolveT) {
-    tau[k] = Jtau[k];
-    rinv[k] = cdiv(make_double2(1.0, 0.0), c2d(Jqr[k + (size_t)k * J.ldq]));
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
@@ -644,28 +685,41 @@ __device__ __forceinline__ void st_any(void* p, size_t i, int es, double2 v) {
   if (es == 16) static_cast<double2*>(p)[i] = v;
   else static_cast<float2*>(p)[i] = cplx<float2>::from(v);
 }
-__global__ void geam_kernel(const GeamDesc* __restrict__ ds, const long long* __restrict__ off, int nd,
-                            long long total) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    int lo = 0, hi = nd - 1;
-    while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (off[mid] <= e) lo = mid; else hi = mid - 1; }
-    const GeamDesc D = ds[lo];
-    long long loc = e - off[lo];
-    int i = (int)(loc % D.m), j = (int)(loc / D.m);
-    double2 a = D.opA ? cconj(ld_any(D.A, j + (size_t)i * D.lda, D.esA)) : ld_any(D.A, i + (size_t)j * D.lda, D.esA);
-    if (D.rs) a = cscale(a, D.rs[i]);
-    if (D.cs) a = cscale(a, D.cs[j]);
-    double2 v = cmul(D.alpha, a);
-    const size_t ci = i + (size_t)j * D.ldc;
-    if (!(D.beta.x == 0.0 && D.beta.y == 0.0)) v = cadd(v, cmul(D.beta, ld_any(D.C, ci, D.esC)));
-    st_any(D.C, ci, D.esC, v);
+constexpr int kGeamInline = 36;
+using GeamInline = Inline<kGeamInline * sizeof(GeamDesc)>;
+// one grid row per block
+__global__ void __launch_bounds__(256) geam_kernel(const GeamDesc* __restrict__ ds, int nd,
+                                                   const __grid_constant__ GeamInline inl) {
+  pdl_begin();
+  bool waited = false;
+  for (int b = blockIdx.y; b < nd; b += gridDim.y) {
+    const GeamDesc D = ds ? ds[b] : reinterpret_cast<const GeamDesc*>(inl.b)[b];
+    if (!waited) {
+      pdl_wait();
+      waited = true;
+    }
+    const int tot = D.m * D.n;
+    for (int e = blockIdx.x * 256 + threadIdx.x; e < tot; e += gridDim.x * 256) {
+      const int j = e / D.m, i = e - j * D.m;
+      double2 a = D.opA ? cconj(ld_any(D.A, j + (size_t)i * D.lda, D.esA)) : ld_any(D.A, i + (size_t)j * D.lda, D.esA);
+      if (D.rs) a = cscale(a, D.rs[i]);
+      if (D.cs) a = cscale(a, D.cs[j]);
+      double2 v = cmul(D.alpha, a);
+      const size_t ci = i + (size_t)j * D.ldc;
+      if (!(D.beta.x == 0.0 && D.beta.y == 0.0)) v = cadd(v, cmul(D.beta, ld_any(D.C, ci, D.esC)));
+      st_any(D.C, ci, D.esC, v);
+    }
   }
 }
 
 // ---------------------------------------------------------------- norms
-__global__ void __launch_bounds__(kT) norm_kernel(const NormDesc* __restrict__ ds) {
-  const NormDesc D = ds[blockIdx.x];
+constexpr int kNormInline = 64;
+using NormInline = Inline<kNormInline * sizeof(NormDesc)>;
+__global__ void __launch_bounds__(kT) norm_kernel(const NormDesc* __restrict__ ds,
+                                                  const __grid_constant__ NormInline inl) {
+  pdl_begin();
+  const NormDesc D = ds ? ds[blockIdx.x] : reinterpret_cast<const NormDesc*>(inl.b)[blockIdx.x];
+  pdl_wait();
   __shared__ double sh[kW + 1];
   double s = 0.0;
   for (long long e = threadIdx.x; e < (long long)D.m * D.n; e += kT) {
@@ -777,13 +831,18 @@ int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int es, cudaStream_t 
 
 namespace {
 template <typename C>
-int launch_solve_reg(const SolveJob* d_jobs, const int2* d_ctas, int nctas, int mmax, size_t smem, cudaStream_t s) {
+int launch_solve_reg(const SolveBatch& g, size_t smem, cudaStream_t s) {
   static bool attr[6] = {false, false, false, false, false, false};
-#define AIFMM_SOLVE_CASE(I, R)                                                      \
-  if (mmax <= 8 * R) {                                                              \
-    smem_attr_once(qr_solve_reg_kernel<C, R>, attr[I]);                             \
-    qr_solve_reg_kernel<C, R><<<nctas, kSolveT, smem, s>>>(d_jobs, d_ctas);         \
-    return (int)cudaGetLastError();                                                 \
+  SolveInline inl;
+  dim3 grid(g.nctas);
+  if (!g.d) {
+    memcpy(inl.b, g.h, sizeof(SolveJob) * g.njobs);
+    grid = dim3(g.nctas, g.njobs);  // nctas: the most CTAs of one job
+  }
+#define AIFMM_SOLVE_CASE(I, R)                                                                                       \
+  if (g.mmax <= 8 * R) {                                                                                             \
+    smem_attr_once(qr_solve_reg_kernel<C, R>, attr[I]);                                                              \
+    return launch_chain(qr_solve_reg_kernel<C, R>, grid, kSolveT, smem, s, g.d, g.ctas, (int)g.early, inl);          \
   }
   AIFMM_SOLVE_CASE(0, 3) AIFMM_SOLVE_CASE(1, 5) AIFMM_SOLVE_CASE(2, 8) AIFMM_SOLVE_CASE(3, 12)
   AIFMM_SOLVE_CASE(4, 18) AIFMM_SOLVE_CASE(5, 28)
@@ -793,13 +852,12 @@ int launch_solve_reg(const SolveJob* d_jobs, const int2* d_ctas, int nctas, int 
 }  // namespace
 
 int aifmm_solve_cols() { return kSolveCols; }
-int aifmm_launch_qr_solve_reg(const SolveJob* d_jobs, const int2* d_ctas, int nctas, int mmax, int nzpmax, int es,
-                              cudaStream_t s) {
-  if (nctas <= 0) return 0;
-  if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  const size_t smem = (size_t)es * ((size_t)(mmax | 1) * nzpmax + (size_t)nzpmax) + sizeof(double2) * nzpmax + 64;
-  return es == 16 ? launch_solve_reg<double2>(d_jobs, d_ctas, nctas, mmax, smem, s)
-                  : launch_solve_reg<float2>(d_jobs, d_ctas, nctas, mmax, smem, s);
+int aifmm_solve_inline_max() { return kSolveInline; }
+int aifmm_launch_qr_solve_reg(const SolveBatch& g, int es, cudaStream_t s) {
+  if (g.nctas <= 0) return 0;
+  if (!valid_es(es) || (!g.d && g.njobs > kSolveInline)) return (int)cudaErrorInvalidValue;
+  const size_t smem = (size_t)es * ((size_t)(g.mmax | 1) * g.nzpmax + (size_t)g.nzpmax) + sizeof(double2) * g.nzpmax + 64;
+  return es == 16 ? launch_solve_reg<double2>(g, smem, s) : launch_solve_reg<float2>(g, smem, s);
 }
 
 int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,
@@ -822,59 +880,71 @@ int aifmm_launch_formq(const FormQJob* d_jobs, const int* d_col_off, int njobs, 
 }
 namespace {
 template <typename C, int WM, int WN, int NS>
-int launch_gemm_ns(const GemmDesc* d, const GemmTerm* t, const int2* tiles, int ntiles, int tk, cudaStream_t s) {
+int launch_gemm_ns(const GemmBatch& g, int tk, cudaStream_t s) {
   static bool attr = false;
   smem_attr_once(gemm_kernel<C, WM, WN, NS>, attr);
   const size_t smem = sizeof(C) * NS * (size_t)(gemm_area(8 * WM, tk) + gemm_area(8 * WN, tk));
-  gemm_kernel<C, WM, WN, NS><<<ntiles, 32 * WM * WN * (NS == 1 ? 1 : 2), smem, s>>>(d, t, tiles, tk);
-  return (int)cudaGetLastError();
+  GemmInline<NS> inl;
+  dim3 grid(g.ntiles);
+  if (!g.d) {
+    memcpy(inl.b, g.one, sizeof(GemmOne) * g.none);
+    grid = dim3(g.ntiles, g.none);  // ntiles: the most tiles of one product
+  }
+  return launch_chain(gemm_kernel<C, WM, WN, NS>, grid, 32 * WM * WN * (NS == 1 ? 1 : 2), smem, s, g.d, g.terms, g.tiles,
+                      tk, inl);
 }
 template <typename C, int WM, int WN>
-int launch_gemm(const GemmDesc* d, const GemmTerm* t, const int2* tiles, int ntiles, int kmax, int tmax,
-                cudaStream_t s) {
+int launch_gemm(const GemmBatch& g, cudaStream_t s) {
   // every product one chunk: one buffer, so that many CTAs share an SM
-  if (tmax <= 1 && kmax <= kGemmTK1)
-    return launch_gemm_ns<C, WM, WN, 1>(d, t, tiles, ntiles, std::max(4, (kmax + 3) & ~3), s);
-  const int tk = std::max(4, std::min(kGemmTK, (kmax + 3) & ~3));
+  if (!g.d || (g.tmax <= 1 && g.kmax <= kGemmTK1))
+    return launch_gemm_ns<C, WM, WN, 1>(g, std::max(4, (g.kmax + 3) & ~3), s);
+  const int tk = std::max(4, std::min(kGemmTK, (g.kmax + 3) & ~3));
   // few CTAs: four buffers hide more of the load latency; many: three, for more CTAs an SM
-  if (ntiles <= 2 * 148 && 8 * WM < 32) return launch_gemm_ns<C, WM, WN, 4>(d, t, tiles, ntiles, tk, s);
-  return launch_gemm_ns<C, WM, WN, 3>(d, t, tiles, ntiles, tk, s);
+  if (g.ntiles <= 2 * 148 && 8 * WM < 32) return launch_gemm_ns<C, WM, WN, 4>(g, tk, s);
+  return launch_gemm_ns<C, WM, WN, 3>(g, tk, s);
 }
 }  // namespace
 void aifmm_gemm_tile(int shape, int* tm, int* tn) {
   *tm = shape == 16 ? 16 : 32;
   *tn = shape;
 }
-int aifmm_launch_gemm(const GemmDesc* d, const GemmTerm* d_terms, const int2* d_tiles, int ntiles, int shape, int kmax,
-                      int tmax, cudaStream_t s, int es) {
-  if (ntiles <= 0) return 0;
-  if (!valid_es(es)) return (int)cudaErrorInvalidValue;
+bool aifmm_gemm_inline(int nproducts, int kmax, int tmax) {
+  return nproducts <= kGemmInline && kmax <= kGemmTK1 && tmax <= 1;
+}
+int aifmm_launch_gemm(const GemmBatch& g, int shape, cudaStream_t s, int es) {
+  if (g.ntiles <= 0) return 0;
+  if (!valid_es(es) || (!g.d && !aifmm_gemm_inline(g.none, g.kmax, g.tmax))) return (int)cudaErrorInvalidValue;
   switch (shape) {
-#define AIFMM_GEMM_CASE(S, WM, WN)                                                                  \
-    case S:                                                                                        \
-      return es == 16 ? launch_gemm<double2, WM, WN>(d, d_terms, d_tiles, ntiles, kmax, tmax, s)   \
-                      : launch_gemm<float2, WM, WN>(d, d_terms, d_tiles, ntiles, kmax, tmax, s);
+#define AIFMM_GEMM_CASE(S, WM, WN) \
+    case S: return es == 16 ? launch_gemm<double2, WM, WN>(g, s) : launch_gemm<float2, WM, WN>(g, s);
     AIFMM_GEMM_CASE(8, 4, 1) AIFMM_GEMM_CASE(16, 2, 2) AIFMM_GEMM_CASE(32, 4, 4)
 #undef AIFMM_GEMM_CASE
   }
   return (int)cudaErrorInvalidValue;
 }
-int aifmm_launch_geam(const GeamDesc* d, const long long* d_off, int nd, long long total, cudaStream_t s) {
-  if (nd <= 0 || total <= 0) return 0;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148LL * 32) blocks = 148LL * 32;
-  geam_kernel<<<(int)blocks, 256, 0, s>>>(d, d_off, nd, total);
-  return (int)cudaGetLastError();
+int aifmm_geam_inline_max() { return kGeamInline; }
+int aifmm_launch_geam(const GeamDesc* d, const GeamDesc* h, int nd, int max_elems, cudaStream_t s) {
+  if (nd <= 0 || max_elems <= 0) return 0;
+  if (!d && nd > kGeamInline) return (int)cudaErrorInvalidValue;
+  GeamInline inl;
+  if (!d) memcpy(inl.b, h, sizeof(GeamDesc) * nd);
+  // four elements a thread; few blocks: one each, so that a small copy is one round of loads
+  const int per = nd > 1024 ? 1024 : 256;
+  const int gx = std::min(std::max(1, (max_elems + per - 1) / per), 148 * 4);
+  return launch_chain(geam_kernel, dim3(gx, std::min(nd, 65535)), 256, 0, s, d, nd, inl);
 }
 int aifmm_launch_equilibrate(const EquilDesc* d, int nd, cudaStream_t s) {
   if (nd <= 0) return 0;
   equilibrate_kernel<<<nd, kT, 0, s>>>(d);
   return (int)cudaGetLastError();
 }
-int aifmm_launch_norms(const NormDesc* d, int nd, cudaStream_t s) {
+int aifmm_norm_inline_max() { return kNormInline; }
+int aifmm_launch_norms(const NormDesc* d, const NormDesc* h, int nd, cudaStream_t s) {
   if (nd <= 0) return 0;
-  norm_kernel<<<nd, kT, 0, s>>>(d);
-  return (int)cudaGetLastError();
+  if (!d && nd > kNormInline) return (int)cudaErrorInvalidValue;
+  NormInline inl;
+  if (!d) memcpy(inl.b, h, sizeof(NormDesc) * nd);
+  return launch_chain(norm_kernel, dim3(nd), kT, 0, s, d, inl);
 }
 int aifmm_launch_skel_lu(const SkelLUJob* d, int nd, const EntryCtx& ctx, cudaStream_t s) {
   if (nd <= 0) return 0;

@@ -151,34 +151,66 @@ int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njob
                           cudaStream_t s);
 size_t aifmm_qr_smem_bytes(int m, int n, int es);
 // eight lanes per right-hand side, the column in registers; m <= 224 and the factor's
-// first nzp columns must fit in shared memory.  d_ctas: (job, first column) of each
-// CTA of aifmm_solve_cols() columns
+// first nzp columns must fit in shared memory.  Jobs on the device with (job, first
+// column) of each CTA of aifmm_solve_cols() columns, or up to aifmm_solve_inline_max()
+// jobs in the parameters (d = nullptr; nctas: the most CTAs of one job).  early: the
+// factors were written before the launch that precedes this one started.
+struct SolveBatch {
+  const SolveJob* d; const int2* ctas; int nctas;
+  const SolveJob* h; int njobs;
+  int mmax, nzpmax;
+  bool early;
+};
 int aifmm_solve_cols();
-int aifmm_launch_qr_solve_reg(const SolveJob* d_jobs, const int2* d_ctas, int nctas, int mmax, int nzpmax, int es,
-                              cudaStream_t s);
+int aifmm_solve_inline_max();
+int aifmm_launch_qr_solve_reg(const SolveBatch& g, int es, cudaStream_t s);
 // one CTA per factorisation, the matrix in shared memory (aifmm_qr_smem_bytes)
 int aifmm_launch_qr_factor_smem(const QRJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s);
 // the columns in registers: the kernel class of an m x n block, -1 if no class holds it
 int aifmm_qr_class(int m, int n);
-int aifmm_launch_qr_factor_reg(const QRJob* d_jobs, int njobs, int cls, int n, int es, cudaStream_t s);
+// Small batches (up to ..._inline_max jobs) travel in the kernel's parameters: the
+// device pointer is nullptr then and the host array is read.
+int aifmm_qr_inline_max();
+int aifmm_launch_qr_factor_reg(const QRJob* d_jobs, const QRJob* h_jobs, int njobs, int cls, int n, int es,
+                               cudaStream_t s);
 // the fused compression on the register QR, and on the shared-memory QR where the
 // class is -1
 int aifmm_compress_class(int m, int rK, int c, int rb, int es);
 bool aifmm_compress_class_holds(int cls, int ncol);
 size_t aifmm_compress_reg_smem_bytes(int cls, int m, int rK, int c, int rb, int es);
-int aifmm_launch_compress_reg(const CompressJob* d_jobs, int njobs, int cls, int n, size_t smem, int es,
-                              cudaStream_t s);
+int aifmm_compress_inline_max();
+int aifmm_launch_compress_reg(const CompressJob* d_jobs, const CompressJob* h_jobs, int njobs, int cls, int n,
+                              size_t smem, int es, cudaStream_t s);
 // shared memory the fused compression needs for these sizes (0: does not fit)
 size_t aifmm_compress_smem_bytes(int m, int rK, int c, int rb, int es);
 int aifmm_launch_compress_p2p(const CompressJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s);
 int aifmm_launch_formq(const FormQJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es, cudaStream_t s);
-// d_tiles: one entry per output tile, (product, tile index down the rows first); shape
-// 8, 16 or 32 columns (aifmm_gemm_tile: 32 x 8, 16 x 16 or 32 x 32 tiles); kmax, tmax:
-// the batch's largest k and number of terms
+// A product of one term whose alpha and beta are small whole numbers, compact: these
+// travel in the kernel's parameters, up to kGemmInline of them.
+struct GemmOne {
+  void* C; const void* A; const void* B;
+  int ldc, lda, ldb;
+  unsigned short m, n, k;
+  signed char alpha, beta;
+  int op;                // opA + 2 opB
+};
+constexpr int kGemmInline = 74;  // 74 products of 48 bytes: a box's 64 fill-ins and its bases fit in 4 KB
+// Products on the device with one entry per output tile (product, tile index down the
+// rows first), or in the parameters (d = nullptr; ntiles: the most tiles of one
+// product).  shape 8, 16 or 32 columns (aifmm_gemm_tile: 32 x 8, 16 x 16 or 32 x 32
+// tiles); kmax, tmax: the batch's largest k and number of terms.
+struct GemmBatch {
+  const GemmDesc* d; const GemmTerm* terms; const int2* tiles; int ntiles;
+  const GemmOne* one; int none;
+  int kmax, tmax;
+};
 void aifmm_gemm_tile(int shape, int* tm, int* tn);
-int aifmm_launch_gemm(const GemmDesc* d, const GemmTerm* d_terms, const int2* d_tiles, int ntiles, int shape, int kmax,
-                      int tmax, cudaStream_t s, int es = 16);
-int aifmm_launch_geam(const GeamDesc* d, const long long* d_off, int nd, long long total, cudaStream_t s);
-int aifmm_launch_norms(const NormDesc* d, int nd, cudaStream_t s);
+bool aifmm_gemm_inline(int nproducts, int kmax, int tmax);
+int aifmm_launch_gemm(const GemmBatch& g, int shape, cudaStream_t s, int es = 16);
+// max_elems: the largest m n of the batch
+int aifmm_geam_inline_max();
+int aifmm_launch_geam(const GeamDesc* d, const GeamDesc* h, int nd, int max_elems, cudaStream_t s);
+int aifmm_norm_inline_max();
+int aifmm_launch_norms(const NormDesc* d, const NormDesc* h, int nd, cudaStream_t s);
 int aifmm_launch_equilibrate(const EquilDesc* d, int nd, cudaStream_t s);
 int aifmm_launch_skel_lu(const SkelLUJob* d, int nd, const EntryCtx& ctx, cudaStream_t s);

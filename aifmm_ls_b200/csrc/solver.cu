@@ -446,6 +446,8 @@ struct aifmm_problem {
   double* d_norms = nullptr;   // device view of h_norms
   double* h_norms = nullptr;
   int norm_cap = 0;
+  // the recompressions' ranks, in mapped pinned host memory too
+  int *h_ranks = nullptr, *d_ranks = nullptr;
   cudaEvent_t ev_norm[2] = {nullptr, nullptr};  // after the x- and z-phase norm launches
   int ncand[2] = {0, 0};                        // candidates recorded when each event was set
   bool norms_pending = false;
@@ -598,32 +600,60 @@ struct aifmm_problem {
     const int shape = nmax <= 8 ? 8 : gemm_cols[nmax <= 16 ? 0 : 1];
     int tm, tn, kmax = 0, tmax = 0;
     aifmm_gemm_tile(shape, &tm, &tn);
-    std::vector<int2> tiles;
     double fl = 0;
-    for (size_t i = 0; i < gd.size(); ++i) {
-      const GemmDesc& g = gd[i];
-      const long nt = (long)((g.m + tm - 1) / tm) * ((g.n + tn - 1) / tn);
-      if (nt + (long)tiles.size() > INT_MAX) throw Fail(AIFMM_ERR_ARG, "gemm batch too large");
-      for (int t = 0; t < (int)nt; ++t) tiles.push_back(make_int2((int)i, t));
+    bool simple = !recording;  // a recorded plan keeps its descriptors on the device
+    for (const GemmDesc& g : gd) {
       for (int t = 0; t < g.nterms; ++t) {
         kmax = std::max(kmax, gt[g.term0 + t].k);
         fl += 8.0 * g.m * g.n * gt[g.term0 + t].k;
       }
       tmax = std::max(tmax, g.nterms);
+      auto whole = [](double2 v) { return v.y == 0.0 && v.x >= -100.0 && v.x <= 100.0 && v.x == (double)(int)v.x; };
+      simple = simple && g.m < 65536 && g.n < 65536 && whole(g.alpha) && whole(g.beta);
     }
-    if (gt.empty()) gt.push_back(GemmTerm{});
-    auto ptrs = put_many_({{gt.data(), gt.size() * sizeof(GemmTerm)}, {gd.data(), gd.size() * sizeof(GemmDesc)},
-                           {tiles.data(), tiles.size() * sizeof(int2)}});
+    simple = simple && aifmm_gemm_inline((int)gd.size(), kmax, tmax);
+    auto tiles_of = [&](const GemmDesc& g) { return (long)((g.m + tm - 1) / tm) * ((g.n + tn - 1) / tn); };
+    GemmBatch gb{};
+    gb.kmax = kmax; gb.tmax = tmax;
+    const int es = gemm_es;
     cudaEvent_t a;
-    const bool pr = prof_begin(2, a);
-    {
-      const GemmDesc* d1 = static_cast<const GemmDesc*>(ptrs[1]);
-      const GemmTerm* d0 = static_cast<const GemmTerm*>(ptrs[0]);
-      const int2* d2 = static_cast<const int2*>(ptrs[2]);
-      const int nt = (int)tiles.size(), es = gemm_es;
-      KL(run_op([=](cudaStream_t s_) { return aifmm_launch_gemm(d1, d0, d2, nt, shape, kmax, tmax, s_, es); }));
+    if (simple) {
+      std::vector<GemmOne> one(gd.size());
+      long nt = 1;
+      for (size_t i = 0; i < gd.size(); ++i) {
+        const GemmDesc& g = gd[i];
+        GemmOne& o = one[i];
+        o.C = g.C; o.ldc = g.ldc; o.m = (unsigned short)g.m; o.n = (unsigned short)g.n;
+        o.alpha = (signed char)g.alpha.x; o.beta = (signed char)g.beta.x;
+        o.A = o.B = nullptr; o.lda = o.ldb = 1; o.k = 0; o.op = 0;
+        if (g.nterms) {
+          const GemmTerm& t = gt[g.term0];
+          o.A = t.A; o.B = t.B; o.lda = t.lda; o.ldb = t.ldb; o.k = (unsigned short)t.k; o.op = t.opA + 2 * t.opB;
+        }
+        nt = std::max(nt, tiles_of(g));
+      }
+      gb.ntiles = (int)nt; gb.one = one.data(); gb.none = (int)one.size();
+      const bool pr = prof_begin(2, a);
+      KL(aifmm_launch_gemm(gb, shape, cur, es));
+      if (pr) prof_end(2, a, fl);
+    } else {
+      std::vector<int2> tiles;
+      for (size_t i = 0; i < gd.size(); ++i) {
+        const long nt = tiles_of(gd[i]);
+        if (nt + (long)tiles.size() > INT_MAX) throw Fail(AIFMM_ERR_ARG, "gemm batch too large");
+        for (int t = 0; t < (int)nt; ++t) tiles.push_back(make_int2((int)i, t));
+      }
+      if (gt.empty()) gt.push_back(GemmTerm{});
+      auto ptrs = put_many_({{gt.data(), gt.size() * sizeof(GemmTerm)}, {gd.data(), gd.size() * sizeof(GemmDesc)},
+                             {tiles.data(), tiles.size() * sizeof(int2)}});
+      gb.terms = static_cast<const GemmTerm*>(ptrs[0]);
+      gb.d = static_cast<const GemmDesc*>(ptrs[1]);
+      gb.tiles = static_cast<const int2*>(ptrs[2]);
+      gb.ntiles = (int)tiles.size();
+      const bool pr = prof_begin(2, a);
+      KL(run_op([=](cudaStream_t s_) { return aifmm_launch_gemm(gb, shape, s_, es); }));
+      if (pr) prof_end(2, a, fl);
     }
-    if (pr) prof_end(2, a, fl);
     gd.clear(); gt.clear();
   }
   void geam(const Blk& C, const Blk& A, int opA, double2 alpha, double2 beta) {
@@ -639,15 +669,16 @@ struct aifmm_problem {
   void copy(const Blk& C, const Blk& A) { geam(C, A, 0, C1, C0); }
   void flush_geam() {
     if (ged.empty()) return;
-    std::vector<long long> off(ged.size());
-    long long tot = 0;
-    for (size_t i = 0; i < ged.size(); ++i) { off[i] = tot; tot += (long long)ged[i].m * ged[i].n; }
-    auto ptrs = put_many_({{ged.data(), ged.size() * sizeof(GeamDesc)}, {off.data(), off.size() * sizeof(long long)}});
-    {
+    long most = 0;
+    for (auto& g : ged) most = std::max(most, (long)g.m * g.n);
+    if (most > INT_MAX) throw Fail(AIFMM_ERR_ARG, "block too large");
+    const int nd = (int)ged.size(), me = (int)most;
+    if (!recording && nd <= aifmm_geam_inline_max()) {
+      KL(aifmm_launch_geam(nullptr, ged.data(), nd, me, cur));
+    } else {
+      auto ptrs = put_many_({{ged.data(), ged.size() * sizeof(GeamDesc)}});
       const GeamDesc* d0 = static_cast<const GeamDesc*>(ptrs[0]);
-      const long long* d1 = static_cast<const long long*>(ptrs[1]);
-      const int nd = (int)ged.size();
-      KL(run_op([=](cudaStream_t s_) { return aifmm_launch_geam(d0, d1, nd, tot, s_); }));
+      KL(run_op([=](cudaStream_t s_) { return aifmm_launch_geam(d0, nullptr, nd, me, s_); }));
     }
     ged.clear();
   }
@@ -666,7 +697,8 @@ struct aifmm_problem {
     }
   }
   // QR factorisation of A in place (threshold 0 -> Eigen default)
-  void qr_prepare(QRF& f, const Blk& A, double thr, bool persistent) {
+  // info: where the pivot count and the rank go (nullptr: with the factor)
+  void qr_prepare(QRF& f, const Blk& A, double thr, bool persistent, int* info = nullptr) {
     f.qr = A;
     const int n = A.c, s = std::min(A.r, A.c);
     if (persistent) {
@@ -683,7 +715,7 @@ struct aifmm_problem {
     } else {
       f.tau = scratch.get(sizeof(double2) * std::max(1, s));
       f.perm = static_cast<int*>(scratch.get(sizeof(int) * std::max(1, n)));
-      f.info = static_cast<int*>(scratch.get(sizeof(int) * 4));
+      f.info = info ? info : static_cast<int*>(scratch.get(sizeof(int) * 4));
       f.norms = static_cast<double*>(scratch.get(sizeof(double) * std::max(1, 2 * n)));
     }
     f.valid = true;
@@ -715,10 +747,11 @@ struct aifmm_problem {
     }
     for (auto& kv : groups) {
       Group& g = kv.second;
-      const QRJob* dq = stage.put(g.jobs, cur);
+      const bool inl = kv.first >= 0 && (int)g.jobs.size() <= aifmm_qr_inline_max();
+      const QRJob* dq = inl ? nullptr : stage.put(g.jobs, cur);
       cudaEvent_t a;
       const bool pr = prof_begin(0, a);
-      if (kv.first >= 0) KL(aifmm_launch_qr_factor_reg(dq, (int)g.jobs.size(), kv.first, g.n, es, cur));
+      if (kv.first >= 0) KL(aifmm_launch_qr_factor_reg(dq, g.jobs.data(), (int)g.jobs.size(), kv.first, g.n, es, cur));
       else KL(aifmm_launch_qr_factor_smem(dq, (int)g.jobs.size(), g.smem, es, cur));
       if (pr) prof_end(0, a, g.fl);
     }
@@ -731,6 +764,8 @@ struct aifmm_problem {
     }
     qj.clear();
   }
+  // Set while a solve runs against kept factors: nothing on the stream still writes them.
+  bool kept_factors = false;
   // X = alpha QR^{-1} B  (B.p == nullptr with B.c = r -> identity)
   void solve(const QRF& f, const Blk& B, const Blk& X, double2 alpha, bool identity = false) {
     const int nr = identity ? X.c : B.c;
@@ -771,21 +806,35 @@ struct aifmm_problem {
       small.clear();
     }
     if (!small.empty()) {
-      std::vector<int2> ctas;
-      for (size_t i = 0; i < small.size(); ++i)
-        for (int c = 0; c < small[i].nrhs; c += aifmm_solve_cols()) ctas.push_back(make_int2((int)i, c));
-      auto ptrs = put_many_({{small.data(), small.size() * sizeof(SolveJob)}, {ctas.data(), ctas.size() * sizeof(int2)}});
       double fl = 0;
-      for (auto& j : small) { const double mz = std::min(j.m, j.n); fl += (16.0 * j.m * mz - 4.0 * mz * mz) * j.nrhs; }
-      cudaEvent_t a;
-      const bool pr = prof_begin(1, a);
-      {
-        const SolveJob* d0 = static_cast<const SolveJob*>(ptrs[0]);
-        const int2* d1 = static_cast<const int2*>(ptrs[1]);
-        const int nc = (int)ctas.size();
-        KL(run_op([=](cudaStream_t s_) { return aifmm_launch_qr_solve_reg(d0, d1, nc, mmax, nmax, es, s_); }));
+      int most = 0;
+      const int sc = aifmm_solve_cols();
+      for (auto& j : small) {
+        const double mz = std::min(j.m, j.n);
+        fl += (16.0 * j.m * mz - 4.0 * mz * mz) * j.nrhs;
+        most = std::max(most, (j.nrhs + sc - 1) / sc);
       }
-      if (pr) prof_end(1, a, fl);
+      SolveBatch sb{};
+      sb.mmax = mmax; sb.nzpmax = nmax;
+      sb.early = kept_factors;
+      cudaEvent_t a;
+      if (!recording && (int)small.size() <= aifmm_solve_inline_max()) {
+        sb.h = small.data(); sb.njobs = (int)small.size(); sb.nctas = most;
+        const bool pr = prof_begin(1, a);
+        KL(aifmm_launch_qr_solve_reg(sb, es, cur));
+        if (pr) prof_end(1, a, fl);
+      } else {
+        std::vector<int2> ctas;
+        for (size_t i = 0; i < small.size(); ++i)
+          for (int c = 0; c < small[i].nrhs; c += sc) ctas.push_back(make_int2((int)i, c));
+        auto ptrs = put_many_({{small.data(), small.size() * sizeof(SolveJob)}, {ctas.data(), ctas.size() * sizeof(int2)}});
+        sb.d = static_cast<const SolveJob*>(ptrs[0]);
+        sb.ctas = static_cast<const int2*>(ptrs[1]);
+        sb.nctas = (int)ctas.size();
+        const bool pr = prof_begin(1, a);
+        KL(run_op([=](cudaStream_t s_) { return aifmm_launch_qr_solve_reg(sb, es, s_); }));
+        if (pr) prof_end(1, a, fl);
+      }
     }
     if (!large.empty()) {
       std::vector<int> off(large.size());
@@ -944,6 +993,8 @@ struct aifmm_problem {
     norm_cap = 4096;
     CK(cudaHostAlloc(&h_norms, sizeof(double) * norm_cap, cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer(&d_norms, h_norms, 0));
+    CK(cudaHostAlloc(&h_ranks, sizeof(int) * 16, cudaHostAllocMapped));
+    CK(cudaHostGetDevicePointer(&d_ranks, h_ranks, 0));
     for (auto& e : ev_norm) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     sync();
   }
@@ -955,6 +1006,7 @@ struct aifmm_problem {
     cudaFree(d_pts); cudaFree(d_q); cudaFree(d_leafc); cudaFree(d_leafxy); cudaFree(d_M); cudaFree(d_near);
     cudaFree(d_iota);
     if (h_norms) cudaFreeHost(h_norms);
+    if (h_ranks) cudaFreeHost(h_ranks);
     for (auto& e : ev_norm) if (e) cudaEventDestroy(e);
     if (st) cudaStreamDestroy(st);
     if (st2) cudaStreamDestroy(st2);
@@ -1409,8 +1461,8 @@ struct aifmm_problem {
   // phase 0: the norms recorded by eliminate_x; phase 1: by eliminate_z
   void flush_norms(int phase) {
     if (!ndv.empty()) {
-      const NormDesc* dn = stage.put(ndv, st);
-      KL(aifmm_launch_norms(dn, (int)ndv.size(), st));
+      const bool inl = (int)ndv.size() <= aifmm_norm_inline_max();
+      KL(aifmm_launch_norms(inl ? nullptr : stage.put(ndv, st), ndv.data(), (int)ndv.size(), st));
       ndv.clear();
     }
     CK(cudaEventRecord(ev_norm[phase], st));
@@ -1688,7 +1740,7 @@ struct aifmm_problem {
       else cl = -1;
     }
     std::vector<CompressJob> jobs(2);
-    int* ranks = static_cast<int*>(scratch.get(sizeof(int) * 4));
+    int* ranks = d_ranks;
     int rcmax[2], rrmax[2];
     for (int s = 0; s < 2; ++s) {
       Box& K = T[j][kk[s]];
@@ -1731,12 +1783,10 @@ struct aifmm_problem {
       J.Tm = cg((long)rcmax[s] * rb);
     }
     flush_all();
-    const CompressJob* dj = stage.put(jobs, st);
-    if (cl >= 0) KL(aifmm_launch_compress_reg(dj, 2, cl, ncol, smem, es_, st));
-    else KL(aifmm_launch_compress_p2p(dj, 2, smem, es_, st));
+    if (cl >= 0) KL(aifmm_launch_compress_reg(nullptr, jobs.data(), 2, cl, ncol, smem, es_, st));
+    else KL(aifmm_launch_compress_p2p(stage.put(jobs, st), 2, smem, es_, st));
     sync();
-    int rk[4];
-    d2h(rk, ranks, sizeof rk);
+    const int* rk = h_ranks;
     for (int s = 0; s < 2; ++s) {
       const int rc = rk[2 * s], rr = rk[2 * s + 1];
       if (rc < 0 || rc > rcmax[s] || rr < 0 || rr > rrmax[s]) throw Fail(AIFMM_ERR_NUMERIC, "compress_P2P: rank out of range");
@@ -1981,14 +2031,11 @@ struct aifmm_problem {
     geam(Blk{Arow.p + (size_t)rk * Arow.ld, mk, Lbk.r, Arow.ld}, Lbk, 1, C1, C0);
     flush_geam();
     QRF qc, qw;
-    qr_prepare(qc, Acol, tol_factor, false);
-    qr_prepare(qw, Arow, tol_factor, false);
+    qr_prepare(qc, Acol, tol_factor, false, d_ranks);
+    qr_prepare(qw, Arow, tol_factor, false, d_ranks + 4);
     flush_qr();
     sync();
-    int ic[2], iw[2];
-    d2h(ic, qc.info, sizeof ic);
-    d2h(iw, qw.info, sizeof iw);
-    const int rc = ic[1], rr = iw[1];
+    const int rc = h_ranks[1], rr = h_ranks[5];
     Blk nLk = newblk(Acol.r, rc), nPtk = newblk(Arow.r, rr);
     formq(qc, nLk);
     formq(qw, nPtk);
@@ -2540,6 +2587,11 @@ struct aifmm_problem {
     nrhs = nrhs_;
     cur = st;
     release_solve_state();
+    struct Kept {
+      bool& f;
+      explicit Kept(bool& f_) : f(f_) { f = true; }
+      ~Kept() { f = false; }
+    } kept(kept_factors);
     for (int j = 2; j <= depth; ++j)
       for (int k = 0; k < nBoxes[j]; ++k) {
         Box& B = T[j][k];
