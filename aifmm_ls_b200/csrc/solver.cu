@@ -438,19 +438,20 @@ struct aifmm_problem {
   double ms[4] = {0, 0, 0, 0};
   long launches_ = 0, launches_fs = 0, launches_asm = 0;
   int nrhs = 1;
-  // pending fill-in candidates of the last eliminated box (kind 0 = P2P, 1 = P2L)
-  struct Cand { int kind, nn, pp; };
-  std::vector<Cand> cands;
-  // Fill-in norm slots in mapped pinned host memory: the norm kernels write them
-  // and the host reads them once the event of their phase has completed.
+  // Fill-in candidates of an eliminated box that its successor's step may recompress
+  // (kind 0 = P2P, 1 = P2L).  A candidate's norm sits in a slot of mapped pinned host
+  // memory: the norm kernels write it and the host reads it once the event of its wave
+  // and phase has completed.
+  struct Cand { int kind, nn, pp, slot; double val; };
+  struct Pend { std::vector<Cand> c[2]; int wave = -1; };  // by phase: eliminate_x, eliminate_z
+  std::vector<Pend> pend;      // of the current level, by the box whose step takes them
   double* d_norms = nullptr;   // device view of h_norms
   double* h_norms = nullptr;
   int norm_cap = 0;
+  std::vector<int> norm_free;  // free slots
+  cudaEvent_t ev_norm[2] = {nullptr, nullptr};  // after the x- and z-phase norm launches of the last wave
   // the recompressions' ranks, in mapped pinned host memory too
   int *h_ranks = nullptr, *d_ranks = nullptr;
-  cudaEvent_t ev_norm[2] = {nullptr, nullptr};  // after the x- and z-phase norm launches
-  int ncand[2] = {0, 0};                        // candidates recorded when each event was set
-  bool norms_pending = false;
 
   EntryCtx ctx() const {
     EntryCtx c;
@@ -990,10 +991,10 @@ struct aifmm_problem {
     const double* d_cheb = static_cast<const double*>(stage.put_raw(cheb.data(), sizeof(double) * cheb.size(), st));
     KL(aifmm_launch_geometry(d.n_cheb, depth, d.L, d.q_kind, d.q_amp, d.q_width, d.q_radius, d_cheb, d_pts, d_q,
                              d_leafc, d_leafxy, st));
-    norm_cap = 4096;
+    norm_cap = 1 << 14;
     CK(cudaHostAlloc(&h_norms, sizeof(double) * norm_cap, cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer(&d_norms, h_norms, 0));
-    CK(cudaHostAlloc(&h_ranks, sizeof(int) * 16, cudaHostAllocMapped));
+    CK(cudaHostAlloc(&h_ranks, sizeof(int) * kRankSlots, cudaHostAllocMapped));
     CK(cudaHostGetDevicePointer(&d_ranks, h_ranks, 0));
     for (auto& e : ev_norm) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     sync();
@@ -1449,14 +1450,34 @@ struct aifmm_problem {
   // ------------------------------------------------------------------ elimination
   Blk& X_of(Box& Nn, bool nn_elim, int k) { return nn_elim ? Nn.P2L[k] : Nn.P2P[k]; }
 
-  void record_cand(int kind, int nn, int pp, const Blk& b) {
-    if ((int)cands.size() >= norm_cap) throw Fail(AIFMM_ERR_NUMERIC, "too many fill-in candidates");
+  // Only the next box's step looks at box k's candidates, and only at those that
+  // involve it (F:2411-2443).
+  void record_cand(int phase, int kind, int k, int nn, int pp, const Blk& b) {
+    if (nn != k + 1 && pp != k + 1) return;
+    if (norm_free.empty()) harvest_norms();
     // every slot is written by a norm kernel (an empty block gives 0), so all
     // writes to the slots are ordered by the stream
+    const int slot = norm_free.back();
+    norm_free.pop_back();
     NormDesc n; n.A = b.p.v(); n.es = b.p.es; n.lda = std::max(b.ld, 1); n.m = b.size() ? b.r : 0; n.n = b.size() ? b.c : 0;
-    n.out = d_norms + cands.size();
-    cands.push_back({kind, nn, pp});
+    n.out = d_norms + slot;
+    pend[k + 1].c[phase].push_back({kind, nn, pp, slot, 0.0});
+    pend[k + 1].wave = wave_now;
     ndv.push_back(n);
+  }
+  // All slots in use: take the values of the finished waves to the host.
+  void harvest_norms() {
+    sync();
+    for (auto& pd : pend)
+      if (pd.wave >= 0 && pd.wave < wave_now)
+        for (auto& ph : pd.c)
+          for (auto& c : ph)
+            if (c.slot >= 0) {
+              c.val = h_norms[c.slot];
+              norm_free.push_back(c.slot);
+              c.slot = -1;
+            }
+    if (norm_free.empty()) throw Fail(AIFMM_ERR_NUMERIC, "too many fill-in candidates");
   }
   // phase 0: the norms recorded by eliminate_x; phase 1: by eliminate_z
   void flush_norms(int phase) {
@@ -1466,7 +1487,6 @@ struct aifmm_problem {
       ndv.clear();
     }
     CK(cudaEventRecord(ev_norm[phase], st));
-    ncand[phase] = (int)cands.size();
   }
   void wait_norms(int phase) {
     auto t0 = std::chrono::steady_clock::now();
@@ -1474,7 +1494,72 @@ struct aifmm_problem {
     st_sync_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     ++st_syncs;
   }
-  void clear_cands() { cands.clear(); ncand[0] = ncand[1] = 0; }
+
+  // The boxes of a level in waves.  The reference eliminates them one after the other
+  // (F:2409-2450); here wave(k) = 1 + the last wave of an earlier box whose step
+  // touches a block that k's step touches, so every block sees the same operations in
+  // the same order, and the steps of a wave run as one batch.  What a step touches:
+  //  * the blocks between any two of k and its neighbours, and k's bases;
+  //  * if its predecessor k - 1 is a neighbour, the recompressions that may follow from
+  //    k - 1's fill-ins, with the boxes o opposite of k: the bases of k, the blocks of k
+  //    with its interaction list and with o, the bases of k's parent -- and the same of
+  //    o, if o comes after k (P2P) and is not eliminated yet.
+  // Depth 5: 1,024 boxes in 581 waves; depth 6: 4,096 in 1,548.
+  std::vector<std::vector<int>> elimination_waves(int j) const {
+    const int nbx = nBoxes[j];
+    std::vector<int> X(nbx), Y(nbx);
+    for (int k = 0; k < nbx; ++k) box_xy(k, j, X[k], Y[k]);
+    std::vector<int> pair((size_t)nbx * 49, -1), basis(nbx, -1), parent(std::max(1, nbx / 4), -1), wave(nbx, 0);
+    std::vector<int*> res;
+    int nw = 0;
+    for (int k = 0; k < nbx; ++k) {
+      res.clear();
+      auto touch = [&](int a, int b) {
+        res.push_back(&pair[(size_t)a * 49 + (Y[b] - Y[a] + 3) * 7 + (X[b] - X[a] + 3)]);
+      };
+      auto far = [&](int a, int b) { return std::max(std::abs(X[a] - X[b]), std::abs(Y[a] - Y[b])); };
+      auto changed = [&](int c) {  // c's bases change
+        res.push_back(&basis[c]);
+        res.push_back(&parent[c / 4]);
+        const Box& B = T[j][c];
+        for (int x : B.inner) if (x != -1) { touch(c, x); touch(x, c); }
+        for (int x : B.outer) if (x != -1) { touch(c, x); touch(x, c); }
+      };
+      int nbr[9], nn = 0;
+      nbr[nn++] = k;
+      for (int x : T[j][k].nb) if (x != -1) nbr[nn++] = x;
+      for (int a = 0; a < nn; ++a)
+        for (int b = 0; b < nn; ++b) touch(nbr[a], nbr[b]);
+      res.push_back(&basis[k]);
+      if (k > 0 && far(k, k - 1) == 1) {
+        bool any = false;
+        for (int o : T[j][k - 1].nb) {
+          if (o == -1 || far(o, k) != 2) continue;
+          any = true;
+          touch(k, o);
+          touch(o, k);
+          if (o > k) changed(o);
+        }
+        if (any) changed(k);
+      }
+      int w = 0;
+      for (int* r : res) w = std::max(w, *r + 1);
+      for (int* r : res) *r = w;
+      wave[k] = w;
+      nw = std::max(nw, w + 1);
+    }
+    std::vector<std::vector<int>> waves(nw);
+    for (int k = 0; k < nbx; ++k) waves[wave[k]].push_back(k);
+    return waves;
+  }
+  int wave_now = 0;
+  // one box's step, as it passes through the phases of its wave
+  struct Step {
+    int k;
+    bool on = false;   // box k carries unknowns
+    Blk XL, W[8];
+    std::vector<std::pair<int, int>> p2p, p2l;
+  };
 
   // The part of eliminate_x that the recompressions of the same step cannot
   // change: they touch the bases of k and of boxes well separated from k, the
@@ -1482,75 +1567,75 @@ struct aifmm_problem {
   // blocks towards its neighbours.  So the factorisation of P2P[k][k] and its
   // solves with those blocks run on the second stream, overlapping the
   // recompressions and their synchronisations on the main stream.
-  struct SideX { bool on = false; Blk W[8]; };
-  SideX sx;
-  void eliminate_x_side(int j, int k) {
-    sx = SideX();
-    Box& B = T[j][k];
-    Blk& Pkk = B.P2P[k];
-    if (Pkk.size() == 0) return;
+  void fork() {
     flush_all();
     CK(cudaEventRecord(ev_fork, st));
     CK(cudaStreamWaitEvent(st2, ev_fork, 0));
     cur = st2;
-    qr_prepare(B.qx, Pkk, 0.0, true);  // factored in place; P2P[k][k] is not read again
-    flush_qr();
-    const int m = Pkk.c;
-    for (int pI = 0; pI < 8; ++pI) {
-      const int pp = B.nb[pI];
-      if (pp == -1) continue;
-      const Blk& src = T[j][pp].elim ? B.M2P[pp] : B.P2P[pp];
-      sx.W[pI] = scr(m, src.c);
-      solve(B.qx, src, sx.W[pI], C1);
-    }
-    flush_solve();
+  }
+  void unfork() {
     CK(cudaEventRecord(ev_join, st2));
     cur = st;
-    sx.on = true;
   }
-  void eliminate_x(int j, int k) {  // F:1814-1840, 1961-2075 (and the no-QR branch :1843-1957)
-    Box& B = T[j][k];
-    Blk& Pkk = B.P2P[k];
-    if (Pkk.size() != 0) {
-      const int m = Pkk.c;
-      Blk XL = scr(m, B.L2P.c), W[8];
-      if (sx.on) {
-        CK(cudaStreamWaitEvent(st, ev_join, 0));
-        for (int q = 0; q < 8; ++q) W[q] = sx.W[q];
-        solve(B.qx, B.L2P, XL, C1);
-      } else {
-        qr_prepare(B.qx, Pkk, 0.0, true);
-        flush_qr();
-        solve(B.qx, B.L2P, XL, C1);
-        for (int pI = 0; pI < 8; ++pI) {
-          const int pp = B.nb[pI];
-          if (pp == -1) continue;
-          const Blk& src = T[j][pp].elim ? B.M2P[pp] : B.P2P[pp];
-          W[pI] = scr(m, src.c);
-          solve(B.qx, src, W[pI], C1);
-        }
+  void eliminate_x_side(int j, std::vector<Step>& ws) {
+    fork();
+    for (Step& S : ws) {
+      Box& B = T[j][S.k];
+      S.on = B.P2P[S.k].size() != 0;
+      if (S.on) qr_prepare(B.qx, B.P2P[S.k], 0.0, true);  // factored in place; P2P[k][k] is not read again
+    }
+    flush_qr();
+    for (Step& S : ws) {
+      if (!S.on) continue;
+      Box& B = T[j][S.k];
+      const int m = B.P2P[S.k].c;
+      for (int pI = 0; pI < 8; ++pI) {
+        const int pp = B.nb[pI];
+        if (pp == -1) continue;
+        const Blk& src = T[j][pp].elim ? B.M2P[pp] : B.P2P[pp];
+        S.W[pI] = scr(m, src.c);
+        solve(B.qx, src, S.W[pI], C1);
       }
-      sx.on = false;
-      flush_solve();
-      { Blk t = newblk(B.P2M.r, XL.c); gemm(t, B.P2M, 0, XL, 0, CM1, C0); assign(B.L2M_f, t); }
+    }
+    flush_solve();
+    unfork();
+  }
+  void eliminate_x(int j, std::vector<Step>& ws) {  // F:1814-1840, 1961-2075
+    CK(cudaStreamWaitEvent(st, ev_join, 0));
+    for (Step& S : ws) {
+      if (!S.on) { eliminate_x_empty(j, S.k); continue; }
+      Box& B = T[j][S.k];
+      S.XL = scr(B.P2P[S.k].c, B.L2P.c);
+      solve(B.qx, B.L2P, S.XL, C1);
+    }
+    flush_solve();
+    for (Step& S : ws) {
+      if (!S.on) continue;
+      Box& B = T[j][S.k];
+      { Blk t = newblk(B.P2M.r, S.XL.c); gemm(t, B.P2M, 0, S.XL, 0, CM1, C0); assign(B.L2M_f, t); }
       for (int n = 0; n < 8; ++n) {
         const int nn = B.nb[n];
         if (nn == -1) continue;
-        Blk t = newblk(B.P2M.r, W[n].c);
-        gemm(t, B.P2M, 0, W[n], 0, CM1, C0);
+        Blk t = newblk(B.P2M.r, S.W[n].c);
+        gemm(t, B.P2M, 0, S.W[n], 0, CM1, C0);
         if (!T[j][nn].elim) assign(B.P2M_f[nn], t); else assign(B.M2M_f[nn], t);
       }
-      // box k's own products first: the z-phase factorisation and solves need only
-      // them, and run on the second stream while the fill-ins of the neighbours'
-      // blocks below are computed
-      flush_gemm();
-      eliminate_z_side(j, k);
+    }
+    // box k's own products first: the z-phase factorisation and solves need only
+    // them, and run on the second stream while the fill-ins of the neighbours'
+    // blocks below are computed
+    flush_gemm();
+    eliminate_z_side(j, ws);
+    for (Step& S : ws) {
+      if (!S.on) continue;
+      const int k = S.k;
+      Box& B = T[j][k];
       for (int n = 0; n < 8; ++n) {
         const int nn = B.nb[n];
         if (nn == -1) continue;
         Box& Nn = T[j][nn];
         const Blk Xnk = X_of(Nn, Nn.elim, k);
-        { Blk t = newblk(Xnk.r, XL.c); gemm(t, Xnk, 0, XL, 0, CM1, C0); assign(B.Lf[n], t); }
+        { Blk t = newblk(Xnk.r, S.XL.c); gemm(t, Xnk, 0, S.XL, 0, CM1, C0); assign(B.Lf[n], t); }
         for (int pI = 0; pI < 8; ++pI) {
           const int pp = B.nb[pI];
           if (pp == -1) continue;
@@ -1561,93 +1646,89 @@ struct aifmm_problem {
           else { tgt = pe ? &Nn.M2L[pp] : &Nn.P2L[pp]; if (!pe && well_sep(j, nn, pp)) kind = 1; }
           const bool must_exist = Nn.elim && pe;  // M2L: the reference subtracts without a size check
           if (tgt->size() == 0 && !must_exist) {
-            Blk t = newblk(Xnk.r, W[pI].c);
-            gemm(t, Xnk, 0, W[pI], 0, CM1, C0);
+            Blk t = newblk(Xnk.r, S.W[pI].c);
+            gemm(t, Xnk, 0, S.W[pI], 0, CM1, C0);
             assign(*tgt, t);
           } else {
-            gemm(*tgt, Xnk, 0, W[pI], 0, CM1, C1);
+            gemm(*tgt, Xnk, 0, S.W[pI], 0, CM1, C1);
           }
-          if (kind >= 0) record_cand(kind, nn, pp, *tgt);
+          if (kind >= 0) record_cand(0, kind, k, nn, pp, *tgt);
         }
       }
-      flush_gemm();
-      flush_norms(0);
-    } else {
-      // box k carries no unknowns: the reference stores uninitialised blocks whose
-      // intended value (a product with an empty inner dimension) is zero
-      { Blk t = newblk(B.P2M.r, B.L2P.c); zero(t); assign(B.L2M_f, t); }
-      for (int n = 0; n < 8; ++n) {
-        const int nn = B.nb[n];
-        if (nn == -1) continue;
-        if (!T[j][nn].elim) { Blk t = newblk(B.P2M.r, B.P2P[nn].c); zero(t); assign(B.P2M_f[nn], t); }
-        else { Blk t = newblk(B.P2M.r, B.M2P[nn].c); zero(t); assign(B.M2M_f[nn], t); }
-      }
-      for (int n = 0; n < 8; ++n) {
-        const int nn = B.nb[n];
-        if (nn == -1) continue;
-        Box& Nn = T[j][nn];
-        { Blk t = newblk(X_of(Nn, Nn.elim, k).r, B.L2P.c); zero(t); assign(B.Lf[n], t); }
-        for (int pI = 0; pI < 8; ++pI) {
-          const int pp = B.nb[pI];
-          if (pp == -1) continue;
-          const bool pe = T[j][pp].elim;
-          if (!Nn.elim) {
-            if (!pe) {
-              Blk& t = Nn.P2P[pp];
-              if (t.size() == 0) { Blk z = newblk(Nn.P2P[k].r, B.P2P[pp].c); zero(z); assign(t, z); }
-              if (well_sep(j, nn, pp) && nn < pp) record_cand(0, nn, pp, t);
-            } else {
-              Blk& t = Nn.M2P[pp];
-              if (t.size() == 0) { Blk z = newblk(Nn.P2P[k].r, B.M2P[pp].c); zero(z); assign(t, z); }
-            }
-          } else if (!pe) {
-            Blk& t = Nn.P2L[pp];
-            if (t.size() == 0) { Blk z = newblk(Nn.P2L[k].r, B.P2P[pp].c); zero(z); assign(t, z); }
-            if (well_sep(j, nn, pp)) record_cand(1, nn, pp, t);
+    }
+    flush_gemm();
+    flush_norms(0);
+  }
+  // Box k carries no unknowns (F:1843-1957): the reference stores uninitialised blocks
+  // whose intended value (a product with an empty inner dimension) is zero.
+  void eliminate_x_empty(int j, int k) {
+    Box& B = T[j][k];
+    { Blk t = newblk(B.P2M.r, B.L2P.c); zero(t); assign(B.L2M_f, t); }
+    for (int n = 0; n < 8; ++n) {
+      const int nn = B.nb[n];
+      if (nn == -1) continue;
+      if (!T[j][nn].elim) { Blk t = newblk(B.P2M.r, B.P2P[nn].c); zero(t); assign(B.P2M_f[nn], t); }
+      else { Blk t = newblk(B.P2M.r, B.M2P[nn].c); zero(t); assign(B.M2M_f[nn], t); }
+    }
+    for (int n = 0; n < 8; ++n) {
+      const int nn = B.nb[n];
+      if (nn == -1) continue;
+      Box& Nn = T[j][nn];
+      { Blk t = newblk(X_of(Nn, Nn.elim, k).r, B.L2P.c); zero(t); assign(B.Lf[n], t); }
+      for (int pI = 0; pI < 8; ++pI) {
+        const int pp = B.nb[pI];
+        if (pp == -1) continue;
+        const bool pe = T[j][pp].elim;
+        if (!Nn.elim) {
+          if (!pe) {
+            Blk& t = Nn.P2P[pp];
+            if (t.size() == 0) { Blk z = newblk(Nn.P2P[k].r, B.P2P[pp].c); zero(z); assign(t, z); }
+            if (well_sep(j, nn, pp) && nn < pp) record_cand(0, 0, k, nn, pp, t);
+          } else {
+            Blk& t = Nn.M2P[pp];
+            if (t.size() == 0) { Blk z = newblk(Nn.P2P[k].r, B.M2P[pp].c); zero(z); assign(t, z); }
           }
+        } else if (!pe) {
+          Blk& t = Nn.P2L[pp];
+          if (t.size() == 0) { Blk z = newblk(Nn.P2L[k].r, B.P2P[pp].c); zero(z); assign(t, z); }
+          if (well_sep(j, nn, pp)) record_cand(0, 1, k, nn, pp, t);
         }
       }
-      flush_norms(0);
     }
   }
 
   // The factorisation of L2M_f and its solves (F:2090-2113, 2245-2279): they read
   // L2M_f, P2M_f / M2M_f and the local right-hand side of box k and write only k's
   // own blocks, while the x-phase fill-ins write only the neighbours' blocks.
-  bool sz_on = false;
-  void eliminate_z_qr_solves(int j, int k) {
-    Box& B = T[j][k];
-    qr_prepare(B.qz, B.L2M_f, 0.0, true);
+  void eliminate_z_side(int j, std::vector<Step>& ws) {
+    fork();
+    for (Step& S : ws) {
+      Box& B = T[j][S.k];
+      if (B.L2M_f.size() > 0) qr_prepare(B.qz, B.L2M_f, 0.0, true);
+    }
     flush_qr();
-    const int nl = B.L2M_f.c;
-    { Blk t = newblk(nl, B.NumM); solve(B.qz, Blk(), t, CM1, true); assign(B.M2L[k], t); }  // QR2^{-1}(-I)
-    for (int n = 0; n < 8; ++n) {
-      const int nn = B.nb[n];
-      if (nn == -1) continue;
-      if (!T[j][nn].elim) { Blk t = newblk(nl, B.P2M_f[nn].c); solve(B.qz, B.P2M_f[nn], t, C1); assign(B.P2L[nn], t); }
-      else { Blk t = newblk(nl, B.M2M_f[nn].c); solve(B.qz, B.M2M_f[nn], t, C1); assign(B.M2L[nn], t); }
-      // well-separated test of (k, nn) is false for a neighbour: nothing is queued here
+    for (Step& S : ws) {
+      Box& B = T[j][S.k];
+      if (B.L2M_f.size() == 0) continue;
+      const int nl = B.L2M_f.c, k = S.k;
+      { Blk t = newblk(nl, B.NumM); solve(B.qz, Blk(), t, CM1, true); assign(B.M2L[k], t); }  // QR2^{-1}(-I)
+      for (int n = 0; n < 8; ++n) {
+        const int nn = B.nb[n];
+        if (nn == -1) continue;
+        if (!T[j][nn].elim) { Blk t = newblk(nl, B.P2M_f[nn].c); solve(B.qz, B.P2M_f[nn], t, C1); assign(B.P2L[nn], t); }
+        else { Blk t = newblk(nl, B.M2M_f[nn].c); solve(B.qz, B.M2M_f[nn], t, C1); assign(B.M2L[nn], t); }
+        // well-separated test of (k, nn) is false for a neighbour: nothing is queued here
+      }
     }
     flush_solve();
+    unfork();
   }
-  void eliminate_z_side(int j, int k) {
-    sz_on = false;
-    if (T[j][k].L2M_f.size() == 0) return;
-    flush_all();
-    CK(cudaEventRecord(ev_fork, st));
-    CK(cudaStreamWaitEvent(st2, ev_fork, 0));
-    cur = st2;
-    eliminate_z_qr_solves(j, k);
-    CK(cudaEventRecord(ev_join, st2));
-    cur = st;
-    sz_on = true;
-  }
-  void eliminate_z(int j, int k) {  // F:2090-2113, 2245-2372 (and the no-QR branch :2116-2242)
-    Box& B = T[j][k];
-    if (B.L2M_f.size() > 0) {
-      if (sz_on) CK(cudaStreamWaitEvent(st, ev_join, 0));
-      else eliminate_z_qr_solves(j, k);
-      sz_on = false;
+  void eliminate_z(int j, std::vector<Step>& ws) {  // F:2090-2113, 2245-2372
+    CK(cudaStreamWaitEvent(st, ev_join, 0));
+    for (Step& S : ws) {
+      const int k = S.k;
+      Box& B = T[j][k];
+      if (B.L2M_f.size() == 0) { eliminate_z_empty(j, k); continue; }
       const Blk Yneg = B.M2L[k];
       for (int n = 0; n < 8; ++n) {
         const int nn = B.nb[n];
@@ -1669,137 +1750,166 @@ struct aifmm_problem {
           if (!Nn.elim) { tgt = pe ? &Nn.M2P[pp] : &Nn.P2P[pp]; if (!pe && well_sep(j, nn, pp) && nn < pp) kind = 0; }
           else { tgt = pe ? &Nn.M2L[pp] : &Nn.P2L[pp]; if (!pe && well_sep(j, nn, pp)) kind = 1; }
           gemm(*tgt, Lf, 0, Z, 0, CM1, C1);
-          if (kind >= 0) record_cand(kind, nn, pp, *tgt);
+          if (kind >= 0) record_cand(1, kind, k, nn, pp, *tgt);
         }
       }
-      flush_gemm();
-      flush_norms(1);
-    } else {
-      { Blk t = newblk(0, B.NumM); assign(B.M2L[k], t); }
-      for (int n = 0; n < 8; ++n) {
-        const int nn = B.nb[n];
-        if (nn == -1) continue;
-        if (!T[j][nn].elim) { Blk t = newblk(0, B.P2M_f[nn].c); assign(B.P2L[nn], t); }
-        else { Blk t = newblk(0, B.M2M_f[nn].c); assign(B.M2L[nn], t); }
+    }
+    flush_gemm();
+    flush_norms(1);
+  }
+  void eliminate_z_empty(int j, int k) {  // F:2116-2242
+    Box& B = T[j][k];
+    { Blk t = newblk(0, B.NumM); assign(B.M2L[k], t); }
+    for (int n = 0; n < 8; ++n) {
+      const int nn = B.nb[n];
+      if (nn == -1) continue;
+      if (!T[j][nn].elim) { Blk t = newblk(0, B.P2M_f[nn].c); assign(B.P2L[nn], t); }
+      else { Blk t = newblk(0, B.M2M_f[nn].c); assign(B.M2L[nn], t); }
+    }
+    for (int n = 0; n < 8; ++n) {
+      const int nn = B.nb[n];
+      if (nn == -1) continue;
+      Box& Nn = T[j][nn];
+      Blk& tgt = Nn.elim ? Nn.M2L[k] : Nn.M2P[k];
+      if (tgt.size() == 0) { Blk t = newblk(B.Lf[n].r, B.NumM); zero(t); assign(tgt, t); }
+      for (int pI = 0; pI < 8; ++pI) {
+        const int pp = B.nb[pI];
+        if (pp == -1) continue;
+        const bool pe = T[j][pp].elim;
+        if (!Nn.elim && !pe) { if (well_sep(j, nn, pp) && nn < pp) record_cand(1, 0, k, nn, pp, Nn.P2P[pp]); }
+        else if (Nn.elim && !pe) { if (well_sep(j, nn, pp)) record_cand(1, 1, k, nn, pp, Nn.P2L[pp]); }
       }
-      for (int n = 0; n < 8; ++n) {
-        const int nn = B.nb[n];
-        if (nn == -1) continue;
-        Box& Nn = T[j][nn];
-        Blk& tgt = Nn.elim ? Nn.M2L[k] : Nn.M2P[k];
-        if (tgt.size() == 0) { Blk t = newblk(B.Lf[n].r, B.NumM); zero(t); assign(tgt, t); }
-        for (int pI = 0; pI < 8; ++pI) {
-          const int pp = B.nb[pI];
-          if (pp == -1) continue;
-          const bool pe = T[j][pp].elim;
-          if (!Nn.elim && !pe) { if (well_sep(j, nn, pp) && nn < pp) record_cand(0, nn, pp, Nn.P2P[pp]); }
-          else if (Nn.elim && !pe) { if (well_sep(j, nn, pp)) record_cand(1, nn, pp, Nn.P2L[pp]); }
-        }
-      }
-      flush_norms(1);
     }
   }
 
   // ---- recompression (F:1424-1699)
   struct CompressOut { Blk nL, nPt, M2L; };
-  // Both directions in one launch of the fused kernel (one CTA each), then one
-  // synchronisation to read the four ranks.  Returns false, having enqueued
-  // nothing, when a direction's working set does not fit in shared memory.
-  bool compress_P2P_pair_fused(int j, int k, int b, CompressOut& kb, CompressOut& bk) {
-    const int kk[2] = {k, b}, bb[2] = {b, k};
-    CompressOut* out[2] = {&kb, &bk};
-    size_t smem = 0;
-    // both directions on the register QR when its class holds them, else both on the
-    // shared-memory QR
-    int cls[2], ncol = 0;
-    for (int s = 0; s < 2; ++s) {
-      Box& K = T[j][kk[s]];
-      Box& Bb = T[j][bb[s]];
-      const Blk& Pkb = K.P2P[bb[s]];
-      const Blk& m2l = K.M2L[bb[s]];
-      if (Pkb.r != K.L2P.r) throw Fail(AIFMM_ERR_NUMERIC, "compress_P2P: block rows mismatch");
-      if (Bb.P2M.c != Pkb.c || m2l.r != K.L2P.c || m2l.c != Bb.P2M.r)
-        throw Fail(AIFMM_ERR_NUMERIC, "compress_P2P: block shapes");
-      const size_t need = aifmm_compress_smem_bytes(K.L2P.r, K.L2P.c, Pkb.c, Bb.P2M.r, es_);
-      if (need == 0) return false;
-      smem = std::max(smem, need);
-      cls[s] = aifmm_compress_class(K.L2P.r, K.L2P.c, Pkb.c, Bb.P2M.r, es_);
-      const int n1 = K.L2P.c + Pkb.c;
-      ncol = std::max(ncol, std::max(n1, Bb.P2M.r + std::min(K.L2P.r, n1)));
-    }
-    int cl = std::max(cls[0], cls[1]);
-    if (std::min(cls[0], cls[1]) < 0 || !aifmm_compress_class_holds(cl, ncol)) cl = -1;
-    if (cl >= 0) {
-      size_t need = 0;
+  struct PairOp { int k, b; CompressOut kb, bk; };
+  static constexpr int kRankSlots = 1024;
+  // Both directions of every pair of a round (pairs of different steps of a wave) in
+  // one launch of the fused kernel for each kernel class, one CTA a direction, then one
+  // synchronisation to read the ranks.  Pairs of which a direction's working set does
+  // not fit in shared memory take compress_P2P_pair.
+  void compress_P2P_ops(int j, std::vector<PairOp>& ops) {
+    struct Group { std::vector<CompressJob> jobs; size_t smem = 0; int ncol = 0; };
+    std::map<int, Group> groups;
+    struct Fused { PairOp* op; int slot; };
+    std::vector<Fused> fused;
+    std::vector<PairOp*> rest;
+    auto finish = [&] {
+      if (fused.empty()) return;
+      flush_all();
+      for (auto& kv : groups) {
+        Group& g = kv.second;
+        const int n = (int)g.jobs.size();
+        if (kv.first >= 0) {
+          const bool inl = n <= aifmm_compress_inline_max();
+          KL(aifmm_launch_compress_reg(inl ? nullptr : stage.put(g.jobs, st), g.jobs.data(), n, kv.first, g.ncol, g.smem,
+                                       es_, st));
+        } else {
+          KL(aifmm_launch_compress_p2p(stage.put(g.jobs, st), n, g.smem, es_, st));
+        }
+      }
+      sync();
+      for (auto& f : fused) {
+        CompressOut* out[2] = {&f.op->kb, &f.op->bk};
+        for (int s = 0; s < 2; ++s) {
+          const int rc = h_ranks[f.slot + 2 * s], rr = h_ranks[f.slot + 2 * s + 1];
+          if (rc < 0 || rc > out[s]->M2L.r || rr < 0 || rr > out[s]->M2L.c)
+            throw Fail(AIFMM_ERR_NUMERIC, "compress_P2P: rank out of range");
+          out[s]->nL.c = rc;
+          out[s]->nPt.c = rr;
+          out[s]->M2L.r = rc;
+          out[s]->M2L.c = rr;
+        }
+      }
+      groups.clear();
+      fused.clear();
+    };
+    for (PairOp& op : ops) {
+      const int kk[2] = {op.k, op.b}, bb[2] = {op.b, op.k};
+      CompressOut* out[2] = {&op.kb, &op.bk};
+      size_t smem = 0;
+      // both directions on the register QR when its class holds them, else both on the
+      // shared-memory QR
+      int cls[2], ncol = 0;
+      bool fits = true;
+      for (int s = 0; s < 2 && fits; ++s) {
+        Box& K = T[j][kk[s]];
+        Box& Bb = T[j][bb[s]];
+        const Blk& Pkb = K.P2P[bb[s]];
+        const Blk& m2l = K.M2L[bb[s]];
+        if (Pkb.r != K.L2P.r) throw Fail(AIFMM_ERR_NUMERIC, "compress_P2P: block rows mismatch");
+        if (Bb.P2M.c != Pkb.c || m2l.r != K.L2P.c || m2l.c != Bb.P2M.r)
+          throw Fail(AIFMM_ERR_NUMERIC, "compress_P2P: block shapes");
+        const size_t need = aifmm_compress_smem_bytes(K.L2P.r, K.L2P.c, Pkb.c, Bb.P2M.r, es_);
+        if (need == 0) fits = false;
+        smem = std::max(smem, need);
+        cls[s] = aifmm_compress_class(K.L2P.r, K.L2P.c, Pkb.c, Bb.P2M.r, es_);
+        const int n1 = K.L2P.c + Pkb.c;
+        ncol = std::max(ncol, std::max(n1, Bb.P2M.r + std::min(K.L2P.r, n1)));
+      }
+      if (!fits) { rest.push_back(&op); continue; }
+      int cl = std::max(cls[0], cls[1]);
+      if (std::min(cls[0], cls[1]) < 0 || !aifmm_compress_class_holds(cl, ncol)) cl = -1;
+      if (cl >= 0) {
+        size_t need = 0;
+        for (int s = 0; s < 2; ++s) {
+          Box& K = T[j][kk[s]];
+          const Blk& Pkb = K.P2P[bb[s]];
+          need = std::max(need, aifmm_compress_reg_smem_bytes(cl, K.L2P.r, K.L2P.c, Pkb.c, T[j][bb[s]].P2M.r, es_));
+        }
+        if (need <= (size_t(200) << 10)) smem = need;
+        else cl = -1;
+      }
+      if (4 * ((int)fused.size() + 1) > kRankSlots) finish();
+      const int slot = 4 * (int)fused.size();
+      fused.push_back({&op, slot});
+      Group& g = groups[cl];
+      g.smem = std::max(g.smem, smem);
+      g.ncol = std::max(g.ncol, ncol);
       for (int s = 0; s < 2; ++s) {
         Box& K = T[j][kk[s]];
+        Box& Bb = T[j][bb[s]];
         const Blk& Pkb = K.P2P[bb[s]];
-        need = std::max(need, aifmm_compress_reg_smem_bytes(cl, K.L2P.r, K.L2P.c, Pkb.c, T[j][bb[s]].P2M.r, es_));
+        const Blk& m2l = K.M2L[bb[s]];
+        const int m = K.L2P.r, rK = K.L2P.c, c = Pkb.c, rb = Bb.P2M.r, n1 = rK + c;
+        const int rcmax = std::min(m, n1), n2max = rb + rcmax, rrmax = std::min(c, n2max);
+        out[s]->nL = newblk(m, rcmax);
+        out[s]->nPt = newblk(c, rrmax);
+        out[s]->M2L = scr(rcmax, rrmax);
+        CompressJob J{};
+        for (const Blk* x : std::initializer_list<const Blk*>{&K.L2P, &Pkb, &Bb.P2M, &m2l})
+          if (x->size() && x->p.es != es_) throw Fail(AIFMM_ERR_STATE, "compress_P2P: block of the other form");
+        J.L2P = K.L2P.p.v(); J.ldL = K.L2P.ld;
+        J.Pkb = Pkb.p.v(); J.ldP = Pkb.ld;
+        J.P2M = Bb.P2M.p.v(); J.ldM = Bb.P2M.ld;
+        J.M2L = m2l.p.v(); J.ldT = m2l.ld;
+        J.m = m; J.rK = rK; J.c = c; J.rb = rb; J.tol = tol_factor;
+        J.nL = out[s]->nL.p.v(); J.nPt = out[s]->nPt.p.v();
+        J.M2Lo = out[s]->M2L.p.v(); J.ldO = out[s]->M2L.ld;
+        J.ranks = d_ranks + slot + 2 * s;
+        auto cg = [&](long elems) { return scratch.get((size_t)es_ * std::max(1L, elems)); };
+        if (cl < 0) {
+          J.Acol = cg((long)m * n1);
+          J.Arow = cg((long)c * n2max);
+          J.tau = cg(std::max(rcmax, rrmax));
+          J.perm = static_cast<int*>(scratch.get(sizeof(int) * std::max(1, std::max(n1, n2max))));
+          J.info = static_cast<int*>(scratch.get(sizeof(int) * 4));
+        }
+        J.Rkp = cg((long)rcmax * c);
+        J.Rk = cg((long)rcmax * rK);
+        J.Rn = cg((long)rrmax * rb);
+        J.Rnp = cg((long)rrmax * rcmax);
+        J.Tm = cg((long)rcmax * rb);
+        g.jobs.push_back(J);
       }
-      if (need <= (size_t(200) << 10)) smem = need;
-      else cl = -1;
     }
-    std::vector<CompressJob> jobs(2);
-    int* ranks = d_ranks;
-    int rcmax[2], rrmax[2];
-    for (int s = 0; s < 2; ++s) {
-      Box& K = T[j][kk[s]];
-      Box& Bb = T[j][bb[s]];
-      const Blk& Pkb = K.P2P[bb[s]];
-      const Blk& m2l = K.M2L[bb[s]];
-      const int m = K.L2P.r, rK = K.L2P.c, c = Pkb.c, rb = Bb.P2M.r, n1 = rK + c;
-      rcmax[s] = std::min(m, n1);
-      const int n2max = rb + rcmax[s];
-      rrmax[s] = std::min(c, n2max);
-      out[s]->nL = newblk(m, rcmax[s]);
-      out[s]->nPt = newblk(c, rrmax[s]);
-      out[s]->M2L = scr(rcmax[s], rrmax[s]);
-      CompressJob& J = jobs[s];
-      for (const Blk* x : std::initializer_list<const Blk*>{&K.L2P, &Pkb, &Bb.P2M, &m2l})
-        if (x->size() && x->p.es != es_) throw Fail(AIFMM_ERR_STATE, "compress_P2P: block of the other form");
-      J.L2P = K.L2P.p.v(); J.ldL = K.L2P.ld;
-      J.Pkb = Pkb.p.v(); J.ldP = Pkb.ld;
-      J.P2M = Bb.P2M.p.v(); J.ldM = Bb.P2M.ld;
-      J.M2L = m2l.p.v(); J.ldT = m2l.ld;
-      J.m = m; J.rK = rK; J.c = c; J.rb = rb; J.tol = tol_factor;
-      J.nL = out[s]->nL.p.v(); J.nPt = out[s]->nPt.p.v();
-      J.M2Lo = out[s]->M2L.p.v(); J.ldO = out[s]->M2L.ld;
-      J.ranks = ranks + 2 * s;
-      auto cg = [&](long elems) { return scratch.get((size_t)es_ * std::max(1L, elems)); };
-      if (cl < 0) {
-        J.Acol = cg((long)m * n1);
-        J.Arow = cg((long)c * n2max);
-        J.tau = cg(std::max(rcmax[s], rrmax[s]));
-        J.perm = static_cast<int*>(scratch.get(sizeof(int) * std::max(1, std::max(n1, n2max))));
-        J.info = static_cast<int*>(scratch.get(sizeof(int) * 4));
-      } else {
-        J.Acol = J.Arow = J.tau = nullptr;
-        J.perm = J.info = nullptr;
-      }
-      J.Rkp = cg((long)rcmax[s] * c);
-      J.Rk = cg((long)rcmax[s] * rK);
-      J.Rn = cg((long)rrmax[s] * rb);
-      J.Rnp = cg((long)rrmax[s] * rcmax[s]);
-      J.Tm = cg((long)rcmax[s] * rb);
-    }
-    flush_all();
-    if (cl >= 0) KL(aifmm_launch_compress_reg(nullptr, jobs.data(), 2, cl, ncol, smem, es_, st));
-    else KL(aifmm_launch_compress_p2p(stage.put(jobs, st), 2, smem, es_, st));
-    sync();
-    const int* rk = h_ranks;
-    for (int s = 0; s < 2; ++s) {
-      const int rc = rk[2 * s], rr = rk[2 * s + 1];
-      if (rc < 0 || rc > rcmax[s] || rr < 0 || rr > rrmax[s]) throw Fail(AIFMM_ERR_NUMERIC, "compress_P2P: rank out of range");
-      out[s]->nL.c = rc;
-      out[s]->nPt.c = rr;
-      out[s]->M2L.r = rc;
-      out[s]->M2L.c = rr;
-    }
-    return true;
+    finish();
+    for (PairOp* op : rest) compress_P2P_pair(j, op->k, op->b, op->kb, op->bk);
   }
   // Both directions of compress_P2P (F:1532-1559) in lockstep: (k,b) and (b,k)
   void compress_P2P_pair(int j, int k, int b, CompressOut& kb, CompressOut& bk) {
-    if (compress_P2P_pair_fused(j, k, b, kb, bk)) return;
     int kk[2] = {k, b}, bb[2] = {b, k};
     Blk Acol[2], Rk_prime[2], Rk[2], Arow[2];
     QRF qc[2], qw[2];
@@ -1964,122 +2074,166 @@ struct aifmm_problem {
     return t;
   }
 
-  void compress_P2P_Two_Ways(int j, int k, int b) {  // F:1424-1490
-    ++st_compress;
-    CompressOut kb, bk;
-    compress_P2P_pair(j, k, b, kb, bk);
-    Blk nLk = kb.nL, nPtb = kb.nPt, nLb = bk.nL, nPtk = bk.nPt;
-    equalise(nLk, nPtk);
-    equalise(nLb, nPtb);
-    Box& K = T[j][k];
-    Box& Bb = T[j][b];
-    // The two halves (k's locals with b's multipoles; b's locals with k's
+  void compress_P2P_Two_Ways(int j, std::vector<PairOp>& ops) {  // F:1424-1490
+    st_compress += (long)ops.size();
+    compress_P2P_ops(j, ops);
+    // The two halves of a pair (k's locals with b's multipoles; b's locals with k's
     // multipoles) touch disjoint blocks -- M2L[k][x] and M2L[x][b] against M2L[b][x]
     // and M2L[x][k], and the distinct parents of two well-separated boxes -- so
-    // each stage of both halves is one batched launch.
+    // each stage of both halves, of every pair of the round, is one batched launch.
+    struct Half { Blk nL, nPt, m2l, L, Pm, Tk, Tb; int k, b; };
+    std::vector<Half> hs;
+    for (PairOp& op : ops) {
+      Blk nLk = op.kb.nL, nPtb = op.kb.nPt, nLb = op.bk.nL, nPtk = op.bk.nPt;
+      equalise(nLk, nPtk);
+      equalise(nLb, nPtb);
+      Half a{nLk, nPtb, Blk(), Blk(), Blk(), Blk(), Blk(), op.k, op.b}, c{nLb, nPtk, Blk(), Blk(), Blk(), Blk(), Blk(), op.b, op.k};
+      a.m2l = persist_copy(op.kb.M2L, nLk.c, nPtb.c);
+      c.m2l = persist_copy(op.bk.M2L, nLb.c, nPtk.c);
+      hs.push_back(a);
+      hs.push_back(c);
+    }
     // stage 1: the new M2L blocks, the transfer matrices, the new bases
-    Blk m2l_kb = persist_copy(kb.M2L, nLk.c, nPtb.c), m2l_bk = persist_copy(bk.M2L, nLb.c, nPtk.c);
-    Blk Tk = scr(nLk.c, K.L2P.c), Tb = scr(Bb.P2M.r, nPtb.c);
-    Blk Tk2 = scr(nLb.c, Bb.L2P.c), Tb2 = scr(K.P2M.r, nPtk.c);
-    gemm(Tk, nLk, 1, K.L2P, 0, C1, C0);
-    gemm(Tb, Bb.P2M, 0, nPtb, 0, C1, C0);
-    gemm(Tk2, nLb, 1, Bb.L2P, 0, C1, C0);
-    gemm(Tb2, K.P2M, 0, nPtk, 0, C1, C0);
-    Blk Lk = persist_copy(nLk, nLk.r, nLk.c), Pmb = persist_adj(nPtb);
-    Blk Lb = persist_copy(nLb, nLb.r, nLb.c), Pmk = persist_adj(nPtk);
+    for (Half& h : hs) {
+      Box& K = T[j][h.k];
+      Box& Bb = T[j][h.b];
+      h.Tk = scr(h.nL.c, K.L2P.c);
+      h.Tb = scr(Bb.P2M.r, h.nPt.c);
+      gemm(h.Tk, h.nL, 1, K.L2P, 0, C1, C0);
+      gemm(h.Tb, Bb.P2M, 0, h.nPt, 0, C1, C0);
+      h.L = persist_copy(h.nL, h.nL.r, h.nL.c);
+      h.Pm = persist_adj(h.nPt);
+    }
     flush_geam();
     flush_gemm();
-    // stage 2: the other M2L blocks of the four changed bases, and the parents
-    assign(K.M2L[b], m2l_kb);
-    update_other_M2Ls_at_k(j, k, b, Tk);
-    update_other_M2Ls_at_b(j, k, b, Tb);
-    if (j > 2) { update_parent_L2P(j, k, Tk); update_parent_P2M(j, b, Tb); }
-    assign(K.L2P, Lk);
-    assign(Bb.P2M, Pmb);
-    K.NumL = K.L2P.c;
-    Bb.NumM = Bb.P2M.r;
-    assign(Bb.M2L[k], m2l_bk);
-    update_other_M2Ls_at_k(j, b, k, Tk2);
-    update_other_M2Ls_at_b(j, b, k, Tb2);
-    if (j > 2) { update_parent_L2P(j, b, Tk2); update_parent_P2M(j, k, Tb2); }
-    assign(Bb.L2P, Lb);
-    assign(K.P2M, Pmk);
-    Bb.NumL = Bb.L2P.c;
-    K.NumM = K.P2M.r;
+    // stage 2: the other M2L blocks of the changed bases, and the parents
+    for (Half& h : hs) {
+      Box& K = T[j][h.k];
+      Box& Bb = T[j][h.b];
+      assign(K.M2L[h.b], h.m2l);
+      update_other_M2Ls_at_k(j, h.k, h.b, h.Tk);
+      update_other_M2Ls_at_b(j, h.k, h.b, h.Tb);
+      if (j > 2) { update_parent_L2P(j, h.k, h.Tk); update_parent_P2M(j, h.b, h.Tb); }
+      assign(K.L2P, h.L);
+      assign(Bb.P2M, h.Pm);
+      K.NumL = K.L2P.c;
+      Bb.NumM = Bb.P2M.r;
+    }
     flush_geam();
     flush_gemm();
     // the Q blocks were fresh pool allocations; return them
-    drop(kb.nL); drop(kb.nPt); drop(bk.nL); drop(bk.nPt);
+    for (PairOp& op : ops) { drop(op.kb.nL); drop(op.kb.nPt); drop(op.bk.nL); drop(op.bk.nPt); }
   }
 
 
-  void compress_M2P_P2L(int j, int k, int b) {  // F:1492-1530 (k not eliminated, b eliminated)
-    ++st_compress;
-    Box& K = T[j][k];
-    Box& Bb = T[j][b];
+  // F:1492-1530 for the pairs (k not eliminated, b eliminated) of a round, of
+  // different steps of a wave
+  void compress_M2P_P2L(int j, const std::vector<std::pair<int, int>>& prs) {
+    for (size_t i0 = 0; i0 < prs.size(); i0 += kRankSlots / 8)  // the ranks of a batch have slots of their own
+      compress_M2P_P2L_batch(j, std::vector<std::pair<int, int>>(prs.begin() + (long)i0,
+                                                                 prs.begin() + (long)std::min(prs.size(), i0 + kRankSlots / 8)));
+  }
+  void compress_M2P_P2L_batch(int j, const std::vector<std::pair<int, int>>& prs) {
+    st_compress += (long)prs.size();
+    struct Op { int k, b; Blk Acol, Arow, Mkb, Lbk, nL, nPt, Rkp, Rk, Rn, Rnp, M2Lkb, M2Lbk, m2l_kb, m2l_bk, Tk, Tb, L, Pm; QRF qc, qw; };
+    std::vector<Op> ops(prs.size());
     // compress_M2P(j, k, b) (F:1561-1575) and compress_P2L(j, b, k) (F:1577-1591) in lockstep
-    const Blk& Mkb = K.M2P[b];
-    const Blk& Lbk = Bb.P2L[k];
-    if (Mkb.r != K.L2P.r) throw Fail(AIFMM_ERR_NUMERIC, "compress_M2P: block rows mismatch");
-    if (Lbk.c != K.P2M.c) throw Fail(AIFMM_ERR_NUMERIC, "compress_P2L: block cols mismatch");
-    Blk Acol = scr(K.L2P.r, K.L2P.c + Mkb.c);
-    copy(Blk{Acol.p, K.L2P.r, K.L2P.c, Acol.ld}, K.L2P);
-    copy(Blk{Acol.p + (size_t)K.L2P.c * Acol.ld, Mkb.r, Mkb.c, Acol.ld}, Mkb);
-    const int mk = K.P2M.c, rk = K.P2M.r;
-    Blk Arow = scr(mk, rk + Lbk.r);
-    geam(Blk{Arow.p, mk, rk, Arow.ld}, K.P2M, 1, C1, C0);
-    geam(Blk{Arow.p + (size_t)rk * Arow.ld, mk, Lbk.r, Arow.ld}, Lbk, 1, C1, C0);
+    for (size_t i = 0; i < prs.size(); ++i) {
+      Op& o = ops[i];
+      o.k = prs[i].first; o.b = prs[i].second;
+      Box& K = T[j][o.k];
+      Box& Bb = T[j][o.b];
+      o.Mkb = K.M2P[o.b];
+      o.Lbk = Bb.P2L[o.k];
+      if (o.Mkb.r != K.L2P.r) throw Fail(AIFMM_ERR_NUMERIC, "compress_M2P: block rows mismatch");
+      if (o.Lbk.c != K.P2M.c) throw Fail(AIFMM_ERR_NUMERIC, "compress_P2L: block cols mismatch");
+      o.Acol = scr(K.L2P.r, K.L2P.c + o.Mkb.c);
+      copy(Blk{o.Acol.p, K.L2P.r, K.L2P.c, o.Acol.ld}, K.L2P);
+      copy(Blk{o.Acol.p + (size_t)K.L2P.c * o.Acol.ld, o.Mkb.r, o.Mkb.c, o.Acol.ld}, o.Mkb);
+      const int mk = K.P2M.c, rk = K.P2M.r;
+      o.Arow = scr(mk, rk + o.Lbk.r);
+      geam(Blk{o.Arow.p, mk, rk, o.Arow.ld}, K.P2M, 1, C1, C0);
+      geam(Blk{o.Arow.p + (size_t)rk * o.Arow.ld, mk, o.Lbk.r, o.Arow.ld}, o.Lbk, 1, C1, C0);
+    }
     flush_geam();
-    QRF qc, qw;
-    qr_prepare(qc, Acol, tol_factor, false, d_ranks);
-    qr_prepare(qw, Arow, tol_factor, false, d_ranks + 4);
+    for (size_t i = 0; i < ops.size(); ++i) {
+      qr_prepare(ops[i].qc, ops[i].Acol, tol_factor, false, d_ranks + 8 * i);
+      qr_prepare(ops[i].qw, ops[i].Arow, tol_factor, false, d_ranks + 8 * i + 4);
+    }
     flush_qr();
     sync();
-    const int rc = h_ranks[1], rr = h_ranks[5];
-    Blk nLk = newblk(Acol.r, rc), nPtk = newblk(Arow.r, rr);
-    formq(qc, nLk);
-    formq(qw, nPtk);
+    for (size_t i = 0; i < ops.size(); ++i) {
+      Op& o = ops[i];
+      const int rc = h_ranks[8 * i + 1], rr = h_ranks[8 * i + 5];
+      o.nL = newblk(o.Acol.r, rc);
+      o.nPt = newblk(o.Arow.r, rr);
+      formq(o.qc, o.nL);
+      formq(o.qw, o.nPt);
+    }
     flush_formq();
-    Blk Rkp = scr(rc, Mkb.c), Rk = scr(rc, K.L2P.c), Rn = scr(rr, rk), Rnp = scr(rr, Lbk.r);
-    gemm(Rkp, nLk, 1, Mkb, 0, C1, C0);
-    gemm(Rk, nLk, 1, K.L2P, 0, C1, C0);
-    gemm(Rn, nPtk, 1, K.P2M, 1, C1, C0);
-    gemm(Rnp, nPtk, 1, Lbk, 1, C1, C0);
+    for (Op& o : ops) {
+      Box& K = T[j][o.k];
+      o.Rkp = scr(o.nL.c, o.Mkb.c); o.Rk = scr(o.nL.c, K.L2P.c);
+      o.Rn = scr(o.nPt.c, K.P2M.r); o.Rnp = scr(o.nPt.c, o.Lbk.r);
+      gemm(o.Rkp, o.nL, 1, o.Mkb, 0, C1, C0);
+      gemm(o.Rk, o.nL, 1, K.L2P, 0, C1, C0);
+      gemm(o.Rn, o.nPt, 1, K.P2M, 1, C1, C0);
+      gemm(o.Rnp, o.nPt, 1, o.Lbk, 1, C1, C0);
+    }
     flush_gemm();
-    const Blk& m_kb = K.M2L[b];
-    const Blk& m_bk = Bb.M2L[k];
-    if (m_kb.r != K.L2P.c || m_bk.c != K.P2M.r) throw Fail(AIFMM_ERR_NUMERIC, "compress_M2P_P2L: M2L shape");
-    Blk M2Lkb = scr(rc, m_kb.c), M2Lbk = scr(m_bk.r, rr);
-    gemm(M2Lkb, Rk, 0, m_kb, 0, C1, C0);   // Rk M2L[k][b] + Rk'
-    gemm(M2Lbk, m_bk, 0, Rn, 1, C1, C0);   // M2L[b][k] Rn^H + Rn'^H
+    for (Op& o : ops) {
+      Box& K = T[j][o.k];
+      Box& Bb = T[j][o.b];
+      const Blk& m_kb = K.M2L[o.b];
+      const Blk& m_bk = Bb.M2L[o.k];
+      if (m_kb.r != K.L2P.c || m_bk.c != K.P2M.r) throw Fail(AIFMM_ERR_NUMERIC, "compress_M2P_P2L: M2L shape");
+      o.M2Lkb = scr(o.nL.c, m_kb.c); o.M2Lbk = scr(m_bk.r, o.nPt.c);
+      gemm(o.M2Lkb, o.Rk, 0, m_kb, 0, C1, C0);   // Rk M2L[k][b] + Rk'
+      gemm(o.M2Lbk, m_bk, 0, o.Rn, 1, C1, C0);   // M2L[b][k] Rn^H + Rn'^H
+    }
     flush_gemm();
-    geam(M2Lkb, Rkp, 0, C1, C1);
-    geam(M2Lbk, Rnp, 1, C1, C1);
+    for (Op& o : ops) {
+      geam(o.M2Lkb, o.Rkp, 0, C1, C1);
+      geam(o.M2Lbk, o.Rnp, 1, C1, C1);
+    }
     flush_geam();
-    equalise(nLk, nPtk);
     // k's locals and k's multipoles change; the updates touch M2L[k][x], M2L[x][k]
     // and two different blocks of k's parent, so each stage is one batched launch
-    Blk m2l_kb = persist_copy(M2Lkb, nLk.c, M2Lkb.c), m2l_bk = persist_copy(M2Lbk, M2Lbk.r, nPtk.c);
-    Blk Tk = scr(nLk.c, K.L2P.c), Tb = scr(K.P2M.r, nPtk.c);
-    gemm(Tk, nLk, 1, K.L2P, 0, C1, C0);
-    gemm(Tb, K.P2M, 0, nPtk, 0, C1, C0);
-    Blk L = persist_copy(nLk, nLk.r, nLk.c), Pm = persist_adj(nPtk);
+    for (Op& o : ops) {
+      Box& K = T[j][o.k];
+      Blk nLk = o.nL, nPtk = o.nPt;
+      equalise(nLk, nPtk);
+      o.m2l_kb = persist_copy(o.M2Lkb, nLk.c, o.M2Lkb.c);
+      o.m2l_bk = persist_copy(o.M2Lbk, o.M2Lbk.r, nPtk.c);
+      o.Tk = scr(nLk.c, K.L2P.c);
+      o.Tb = scr(K.P2M.r, nPtk.c);
+      gemm(o.Tk, nLk, 1, K.L2P, 0, C1, C0);
+      gemm(o.Tb, K.P2M, 0, nPtk, 0, C1, C0);
+      o.L = persist_copy(nLk, nLk.r, nLk.c);
+      o.Pm = persist_adj(nPtk);
+    }
     flush_geam();
     flush_gemm();
-    assign(K.M2L[b], m2l_kb);
-    update_other_M2Ls_at_k(j, k, b, Tk);
-    if (j > 2) update_parent_L2P(j, k, Tk);
-    assign(Bb.M2L[k], m2l_bk);
-    update_other_M2Ls_at_b(j, b, k, Tb);
-    if (j > 2) update_parent_P2M(j, k, Tb);
-    assign(K.L2P, L);
-    assign(K.P2M, Pm);
-    K.NumL = K.L2P.c;
-    K.NumM = K.P2M.r;
+    for (Op& o : ops) {
+      Box& K = T[j][o.k];
+      Box& Bb = T[j][o.b];
+      assign(K.M2L[o.b], o.m2l_kb);
+      update_other_M2Ls_at_k(j, o.k, o.b, o.Tk);
+      if (j > 2) update_parent_L2P(j, o.k, o.Tk);
+      assign(Bb.M2L[o.k], o.m2l_bk);
+      update_other_M2Ls_at_b(j, o.b, o.k, o.Tb);
+      if (j > 2) update_parent_P2M(j, o.k, o.Tb);
+      assign(K.L2P, o.L);
+      assign(K.P2M, o.Pm);
+      K.NumL = K.L2P.c;
+      K.NumM = K.P2M.r;
+    }
     flush_geam();
     flush_gemm();
-    drop(nLk);
-    drop(nPtk);
+    for (Op& o : ops) {
+      drop(o.nL);
+      drop(o.nPt);
+    }
   }
 
   void initialise_P2P_NonLeafLevel(int j) {  // F:1743-1807
@@ -2117,86 +2271,112 @@ struct aifmm_problem {
     flush_geam();
   }
 
-  // The pairs queued by the previous box step (F:2411-2438): an instance is
+  // The pairs queued by the previous box's step (F:2411-2438): an instance is
   // queued when its fill-in norm exceeds 1e-10 at the time it was recorded, and
   // only instances involving k are compressed, in the order they were queued.
   // The x-phase norms are waited for first; a z-phase instance matters only if
   // its pair was not already queued by an x-phase instance (a repeated pair is
   // a no-op: its block is gone after the first compression), so the z-phase
-  // norms (the end of the previous step's chain) are waited for only then.
-  void take_pending(int j, int k, std::vector<std::pair<int, int>>& p2p, std::vector<std::pair<int, int>>& p2l) {
-    p2p.clear(); p2l.clear();
-    const int n = (int)cands.size();
-    auto inv = [&](int i) { return cands[i].nn == k || cands[i].pp == k; };
-    bool involved = false;
-    for (int i = 0; i < n; ++i) if (inv(i)) { involved = true; break; }
-    if (!involved) { clear_cands(); return; }
-    const int nx = std::min(ncand[0], n);
-    std::vector<char> take(n, 0);
+  // norms (the end of the previous wave's chain) are waited for only then.
+  // Norms of waves before the last are complete once the last wave's x-phase is.
+  bool waited[2] = {false, false};
+  void take_pending(Step& S) {
+    Pend& pd = pend[S.k];
+    if (pd.wave < 0) return;
+    auto ready = [&](int phase) {
+      const int ph = pd.wave + 1 == wave_now ? phase : 0;
+      if (!waited[ph]) { wait_norms(ph); waited[ph] = true; }
+    };
+    auto value = [&](const Cand& c) { return c.slot >= 0 ? h_norms[c.slot] : c.val; };
     std::set<std::tuple<int, int, int>> queued;
-    bool x_inv = false;
-    for (int i = 0; i < nx; ++i) x_inv = x_inv || inv(i);
-    if (x_inv) {
-      wait_norms(0);
-      for (int i = 0; i < nx; ++i)
-        if (inv(i) && h_norms[i] > 1e-10) { take[i] = 1; queued.insert(std::make_tuple(cands[i].kind, cands[i].nn, cands[i].pp)); }
+    auto take = [&](const Cand& c) {
+      if (c.kind == 0) S.p2p.push_back({c.nn, c.pp});
+      else S.p2l.push_back({c.nn, c.pp});
+    };
+    if (!pd.c[0].empty()) {
+      ready(0);
+      for (const Cand& c : pd.c[0])
+        if (value(c) > 1e-10) { take(c); queued.insert(std::make_tuple(c.kind, c.nn, c.pp)); }
     }
     bool need_z = false;
-    for (int i = nx; i < n; ++i)
-      if (inv(i) && !queued.count(std::make_tuple(cands[i].kind, cands[i].nn, cands[i].pp))) { need_z = true; break; }
+    for (const Cand& c : pd.c[1]) need_z = need_z || !queued.count(std::make_tuple(c.kind, c.nn, c.pp));
     if (need_z) {
-      wait_norms(1);
-      for (int i = nx; i < n; ++i)
-        if (inv(i) && !queued.count(std::make_tuple(cands[i].kind, cands[i].nn, cands[i].pp)) && h_norms[i] > 1e-10)
-          take[i] = 1;
+      ready(1);
+      for (const Cand& c : pd.c[1])
+        if (!queued.count(std::make_tuple(c.kind, c.nn, c.pp)) && value(c) > 1e-10) take(c);
     }
-    for (int i = 0; i < n; ++i) {
-      if (!take[i]) continue;
-      if (cands[i].kind == 0) p2p.push_back({cands[i].nn, cands[i].pp});
-      else p2l.push_back({cands[i].nn, cands[i].pp});
+    // a slot that was never waited for is written before any later use of it: the
+    // norm kernels run in stream order
+    for (auto& ph : pd.c) {
+      for (const Cand& c : ph) if (c.slot >= 0) norm_free.push_back(c.slot);
+      ph.clear();
     }
-    clear_cands();
-    (void)j;
+    pd.wave = -1;
   }
 
   void eliminate_phase_efficient() {  // F:2407-2451
-    std::vector<std::pair<int, int>> p2p, p2l;
-    clear_cands();
+    norm_free.clear();
+    for (int i = norm_cap - 1; i >= 0; --i) norm_free.push_back(i);
     for (int j = depth; j >= 2; --j) {
       if (j != depth) initialise_P2P_NonLeafLevel(j);
-      for (int k = 0; k < nBoxes[j]; ++k) {
+      pend.assign((size_t)nBoxes[j] + 1, Pend());  // pending pairs never cross a level
+      wave_now = 0;
+      for (const auto& ks : elimination_waves(j)) {
         auto tp0 = std::chrono::steady_clock::now();
-        eliminate_x_side(j, k);
-        take_pending(j, k, p2p, p2l);
-        for (auto& pr : p2p) {
-          const int nn = pr.first, pp = pr.second;
-          if (k != nn && k != pp) continue;
-          if (T[j][nn].P2P[pp].size() != 0) {
-            compress_P2P_Two_Ways(j, nn, pp);
-            drop(T[j][nn].P2P[pp]);
-            drop(T[j][pp].P2P[nn]);
+        std::vector<Step> ws(ks.size());
+        for (size_t i = 0; i < ks.size(); ++i) ws[i].k = ks[i];
+        eliminate_x_side(j, ws);
+        waited[0] = waited[1] = false;
+        for (Step& S : ws) take_pending(S);
+        // the i-th pair of every step of the wave as one round
+        for (size_t i = 0, more = 1; more; ++i) {
+          more = 0;
+          std::vector<PairOp> ops;
+          for (Step& S : ws) {
+            if (i >= S.p2p.size()) continue;
+            more = 1;
+            const int nn = S.p2p[i].first, pp = S.p2p[i].second;
+            if (T[j][nn].P2P[pp].size() != 0) ops.push_back(PairOp{nn, pp, {}, {}});
+          }
+          if (ops.empty()) continue;
+          compress_P2P_Two_Ways(j, ops);
+          for (PairOp& o : ops) {
+            drop(T[j][o.k].P2P[o.b]);
+            drop(T[j][o.b].P2P[o.k]);
           }
         }
-        for (auto& pr : p2l) {
-          const int nn = pr.first, pp = pr.second;
-          if (k != nn && k != pp) continue;
-          if (T[j][nn].P2L[pp].size() != 0) {
-            compress_M2P_P2L(j, pp, nn);
-            drop(T[j][nn].P2L[pp]);
-            drop(T[j][pp].M2P[nn]);
+        for (size_t i = 0, more = 1; more; ++i) {
+          more = 0;
+          std::vector<std::pair<int, int>> prs;
+          for (Step& S : ws) {
+            if (i >= S.p2l.size()) continue;
+            more = 1;
+            const int nn = S.p2l[i].first, pp = S.p2l[i].second;
+            if (T[j][nn].P2L[pp].size() != 0) prs.push_back({pp, nn});
+          }
+          if (prs.empty()) continue;
+          compress_M2P_P2L(j, prs);
+          for (auto& pr : prs) {
+            drop(T[j][pr.second].P2L[pr.first]);
+            drop(T[j][pr.first].M2P[pr.second]);
           }
         }
         auto tp1 = std::chrono::steady_clock::now();
-        T[j][k].elim = true;
-        eliminate_x(j, k);
-        eliminate_z(j, k);
+        for (Step& S : ws) T[j][S.k].elim = true;
+        eliminate_x(j, ws);
+        eliminate_z(j, ws);
         end_step();
+        ++wave_now;
         auto tp2 = std::chrono::steady_clock::now();
         st_pending_ms += std::chrono::duration<double, std::milli>(tp1 - tp0).count();
         st_elim_ms += std::chrono::duration<double, std::milli>(tp2 - tp1).count();
       }
       sync();
-      clear_cands();  // pending pairs never cross a level
+      // candidates that no step took: their slots
+      for (Pend& pd : pend)
+        for (auto& ph : pd.c)
+          for (const Cand& c : ph) if (c.slot >= 0) norm_free.push_back(c.slot);
+      pend.clear();
     }
     factor_base(2);
   }
