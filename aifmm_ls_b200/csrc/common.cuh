@@ -101,6 +101,7 @@ struct EntryCtx {
   const double2* leafc;   // leaf centres (Morton order)
   const int2* leafxy;     // leaf grid coordinates
   const double2* M;       // far-field coefficients, 121 x rank, column-major
+  const double2* Mt;      // the same, transposed: the rank sources of one order next to each other
   const double2* nearT;   // 9 near tables, rank x rank column-major each
 };
 

@@ -115,9 +115,12 @@ __device__ double block_sum(double x, double* sh) {
   return r;
 }
 
-// entry of the primary vector p at secondary position s
+// entry of the primary vector p at secondary position s; ENX as the two sites of the
+// kernel have always rounded it (entry.cuh): 2 for the first term, 1 in the loop
+template <int ENX>
 __device__ __forceinline__ double2 ent(const AcaJob& J, bool rows_first, int p, int s, const EntryCtx& c) {
-  return rows_first ? lsa_entry(J.rows[p], J.cols[s], c) : lsa_entry(J.rows[s], J.cols[p], c);
+  const int i = rows_first ? J.rows[p] : J.rows[s], j = rows_first ? J.cols[s] : J.cols[p];
+  return lsa_entry<true, ENX>(i, j, c);
 }
 
 __global__ void __launch_bounds__(kThreads) aca_kernel(const AcaJob* __restrict__ jobs, double tol, EntryCtx ctx) {
@@ -144,7 +147,7 @@ __global__ void __launch_bounds__(kThreads) aca_kernel(const AcaJob* __restrict_
   // ---- first primary vector with a non-negligible entry
   int p0 = -1, spiv = -1;
   for (int l = 0; l < np; ++l) {
-    for (int s = tid; s < ns; s += kThreads) J.P[s] = ent(J, rows_first, l, s, ctx);
+    for (int s = tid; s < ns; s += kThreads) J.P[s] = ent<2>(J, rows_first, l, s, ctx);
     __syncthreads();
     ArgMax r = block_pick(ns, [&](int s) { double2 v = J.P[s]; return hypot(v.x, v.y); }, sa, si);
     if (r.v > tol_robust) { p0 = l; spiv = r.i; break; }
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(kThreads) aca_kernel(const AcaJob* __restrict_
     }
   }
   for (int t = tid; t < np; t += kThreads) {
-    double2 sv = ent(J, rows_first, t, spiv, ctx);
+    double2 sv = ent<2>(J, rows_first, t, spiv, ctx);
     J.S[t] = sv;
     J.U[t] = sv;
     if (!keepP) {
@@ -185,11 +188,11 @@ __global__ void __launch_bounds__(kThreads) aca_kernel(const AcaJob* __restrict_
     for (int l = tid; l < rank; l += kThreads) coef[l] = J.U[(size_t)l * np + pnext];
     __syncthreads();
     for (int s = tid; s < ns; s += kThreads) {
-      double2 pv = ent(J, rows_first, pnext, s, ctx);
+      double2 pv = ent<1>(J, rows_first, pnext, s, ctx);
       if (keepP) {
         if (J.want_rows) J.out[rank + (size_t)s * rmax] = pv; else J.out[s + (size_t)rank * ns] = pv;
       }
-      for (int l = 0; l < rank; ++l) pv = csub(pv, cmul(coef[l], J.V[(size_t)l * ns + s]));
+      for (int l = 0; l < rank; ++l) pv = csub(pv, cmul_f<1, 2>(coef[l], J.V[(size_t)l * ns + s]));
       J.P[s] = pv;
     }
     __syncthreads();
@@ -206,11 +209,11 @@ __global__ void __launch_bounds__(kThreads) aca_kernel(const AcaJob* __restrict_
     __syncthreads();
     double un2 = 0.0;
     for (int t = tid; t < np; t += kThreads) {
-      double2 sv = ent(J, rows_first, t, snew, ctx);
+      double2 sv = ent<1>(J, rows_first, t, snew, ctx);
       if (!keepP) {
         if (J.want_rows) J.out[rank + (size_t)t * rmax] = sv; else J.out[t + (size_t)rank * np] = sv;
       }
-      for (int l = 0; l < rank; ++l) sv = csub(sv, cmul(coef[l], J.U[(size_t)l * np + t]));
+      for (int l = 0; l < rank; ++l) sv = csub(sv, cmul_f<1, 2>(coef[l], J.U[(size_t)l * np + t]));
       J.S[t] = sv;
       J.U[(size_t)rank * np + t] = sv;
       un2 += cabs2(sv);

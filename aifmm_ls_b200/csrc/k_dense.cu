@@ -763,8 +763,9 @@ __global__ void __launch_bounds__(kT) skel_lu_kernel(const SkelLUJob* __restrict
   __shared__ int s_p;
   for (int e = tid; e < r * r; e += kT) {
     int i = e % r, j = e / r;
-    if (J.adjD) D[i + (size_t)j * r] = cconj(lsa_entry(J.rows[j], J.cols[i], ctx));
-    else D[i + (size_t)j * r] = lsa_entry(J.rows[i], J.cols[j], ctx);
+    // (the two sites have always rounded the entry's rotation differently, see entry.cuh)
+    if (J.adjD) D[i + (size_t)j * r] = cconj(lsa_entry<true, 2>(J.rows[j], J.cols[i], ctx));
+    else D[i + (size_t)j * r] = lsa_entry<true, 1>(J.rows[i], J.cols[j], ctx);
   }
   for (int e = tid; e < r * m; e += kT) {
     int i = e % r, j = e / r;
@@ -793,7 +794,7 @@ __global__ void __launch_bounds__(kT) skel_lu_kernel(const SkelLUJob* __restrict
     __syncthreads();
     for (int e = tid; e < (r - k - 1) * (r - k - 1); e += kT) {
       int i = k + 1 + e % (r - k - 1), j = k + 1 + e / (r - k - 1);
-      D[i + (size_t)j * r] = csub(D[i + (size_t)j * r], cmul(D[i + (size_t)k * r], D[k + (size_t)j * r]));
+      D[i + (size_t)j * r] = csub(D[i + (size_t)j * r], cmul_f<1, 2>(D[i + (size_t)k * r], D[k + (size_t)j * r]));
     }
     __syncthreads();
   }
@@ -802,12 +803,12 @@ __global__ void __launch_bounds__(kT) skel_lu_kernel(const SkelLUJob* __restrict
     double2* x = X + (size_t)j * r;
     for (int i = 0; i < r; ++i) {
       double2 s = x[i];
-      for (int l = 0; l < i; ++l) s = csub(s, cmul(D[i + (size_t)l * r], x[l]));
+      for (int l = 0; l < i; ++l) s = csub(s, cmul_f<1, 2>(D[i + (size_t)l * r], x[l]));
       x[i] = s;
     }
     for (int i = r - 1; i >= 0; --i) {
       double2 s = x[i];
-      for (int l = i + 1; l < r; ++l) s = csub(s, cmul(D[i + (size_t)l * r], x[l]));
+      for (int l = i + 1; l < r; ++l) s = csub(s, cmul_f<1, 2>(D[i + (size_t)l * r], x[l]));
       x[i] = cdiv(s, D[i + (size_t)i * r]);
     }
   }

@@ -136,6 +136,17 @@ int aifmm_launch_incident_field(const double2* pts, double kappa, int N, int nrh
   return (int)cudaGetLastError();
 }
 
+namespace {
+// b (c x r) = a^T (a: r x c), column-major
+__global__ void transpose_kernel(const double2* __restrict__ a, double2* __restrict__ b, int r, int c) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < r * c; e += gridDim.x * blockDim.x) b[e] = a[e / c + (size_t)(e % c) * r];
+}
+}  // namespace
+int aifmm_launch_transpose(const double2* a, double2* b, int r, int c, cudaStream_t s) {
+  transpose_kernel<<<(r * c + 255) / 256, 256, 0, s>>>(a, b, r, c);
+  return (int)cudaGetLastError();
+}
+
 int aifmm_launch_gather_segments(const int* src, const int4* segs, long nseg, int* dst, cudaStream_t s) {
   if (nseg <= 0) return 0;
   long blocks = (nseg * 32 + 255) / 256;

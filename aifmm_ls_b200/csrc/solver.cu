@@ -39,6 +39,7 @@ int aifmm_launch_rhs_plane_wave(const double2* pts, const double* q, double kapp
                                 const double* theta, double2* b, cudaStream_t s);
 int aifmm_launch_incident_field(const double2* pts, double kappa, int N, int nrhs, const double* theta, double2* u,
                                 cudaStream_t s);
+int aifmm_launch_transpose(const double2* a, double2* b, int r, int c, cudaStream_t s);
 int aifmm_launch_gather_segments(const int* src, const int4* segs, long nseg, int* dst, cudaStream_t s);
 size_t aifmm_error_norms_scratch_bytes();
 int aifmm_launch_error_norms(const double2* x, long ldx, const double2* t, long ldt, long n, int nrhs, double* part,
@@ -419,7 +420,7 @@ struct aifmm_problem {
   double tol = 0;         // ACA (assembly) tolerance, 10^-tol_pow
   double tol_factor = 0;  // recompression tolerance of the factorisation (tol unless set)
   // device geometry and tables
-  double2 *d_pts = nullptr, *d_leafc = nullptr, *d_M = nullptr, *d_near = nullptr;
+  double2 *d_pts = nullptr, *d_leafc = nullptr, *d_M = nullptr, *d_Mt = nullptr, *d_near = nullptr;
   double* d_q = nullptr;
   int2* d_leafxy = nullptr;
   int* d_iota = nullptr;
@@ -456,7 +457,7 @@ struct aifmm_problem {
   EntryCtx ctx() const {
     EntryCtx c;
     c.rank = rank; c.depth = depth; c.kappa = d.kappa;
-    c.pts = d_pts; c.q = d_q; c.leafc = d_leafc; c.leafxy = d_leafxy; c.M = d_M; c.nearT = d_near;
+    c.pts = d_pts; c.q = d_q; c.leafc = d_leafc; c.leafxy = d_leafxy; c.M = d_M; c.Mt = d_Mt; c.nearT = d_near;
     return c;
   }
 
@@ -980,6 +981,7 @@ struct aifmm_problem {
     CK(cudaMalloc(&d_leafc, sizeof(double2) * nleaf));
     CK(cudaMalloc(&d_leafxy, sizeof(int2) * nleaf));
     CK(cudaMalloc(&d_M, sizeof(double2) * 121 * rank));
+    CK(cudaMalloc(&d_Mt, sizeof(double2) * 121 * rank));
     CK(cudaMalloc(&d_near, sizeof(double2) * 9 * rank * rank));
     CK(cudaMalloc(&d_iota, sizeof(int) * N));
     std::vector<int> iota(N);
@@ -1004,7 +1006,7 @@ struct aifmm_problem {
     if (st2) cudaStreamSynchronize(st2);
     release_plans();
     pool.release_all();
-    cudaFree(d_pts); cudaFree(d_q); cudaFree(d_leafc); cudaFree(d_leafxy); cudaFree(d_M); cudaFree(d_near);
+    cudaFree(d_pts); cudaFree(d_q); cudaFree(d_leafc); cudaFree(d_leafxy); cudaFree(d_M); cudaFree(d_Mt); cudaFree(d_near);
     cudaFree(d_iota);
     if (h_norms) cudaFreeHost(h_norms);
     if (h_ranks) cudaFreeHost(h_ranks);
@@ -1015,6 +1017,11 @@ struct aifmm_problem {
     if (ev_join) cudaEventDestroy(ev_join);
   }
 
+  // the far-field coefficients with the sources of an order next to each other (entry.cuh)
+  void transpose_M() {
+    KL(aifmm_launch_transpose(d_M, d_Mt, 121, rank, st));
+    sync();
+  }
   void tables_compute(int do_round) {
     auto t0 = std::chrono::steady_clock::now();
     double glx[10], glw[10];
@@ -1051,6 +1058,7 @@ struct aifmm_problem {
       CK(cudaMemcpyAsync(d_near, Nt.data(), sizeof(double) * Nt.size(), cudaMemcpyHostToDevice, st));
       sync();
     }
+    transpose_M();
     pool.commit_frees();
     tables_ready = true;
     ms[1] = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -3512,7 +3520,7 @@ aifmm_status aifmm_tables_set(aifmm_problem* p, const double* M, const double* n
   return guard(p, [&] {
     CK(cudaMemcpyAsync(p->d_M, M, sizeof(double2) * 121 * p->rank, cudaMemcpyHostToDevice, p->st));
     CK(cudaMemcpyAsync(p->d_near, near_tables, sizeof(double2) * 9 * p->rank * p->rank, cudaMemcpyHostToDevice, p->st));
-    p->sync();
+    p->transpose_M();
     p->tables_ready = true;
   });
 }
@@ -3567,6 +3575,7 @@ aifmm_status aifmm_entries(aifmm_problem* p, long n, const int* I, const int* J,
     if (!dev)
       for (long t = 0; t < n; ++t)
         if (I[t] < 0 || I[t] >= p->N || J[t] < 0 || J[t] >= p->N) throw Fail(AIFMM_ERR_ARG, "point index out of range");
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
     aifmm_problem::Tmp tI(p, dev ? 1 : sizeof(int) * n), tJ(p, dev ? 1 : sizeof(int) * n);
     aifmm_problem::Tmp tO(p, dev ? 1 : sizeof(double2) * n);
     if (!dev) {
@@ -3585,18 +3594,31 @@ aifmm_status aifmm_get_matrix(aifmm_problem* p, int nr, const int* rows, int nc,
                               int flags) {
   if (!p || nr < 0 || nc < 0 || (nr * (long)nc > 0 && (!rows || !cols || !out))) return AIFMM_ERR_ARG;
   if (!p->tables_ready) { p->err = "tables not ready"; return AIFMM_ERR_STATE; }
-  if (flags & AIFMM_PTR_DEVICE) {
-    return guard(p, [&] {
-      BlockDesc bd{rows, cols, nr, nc, reinterpret_cast<double2*>(out), nr, 0};
-      std::vector<BlockDesc> v{bd};
-      p->launch_blocks(v);
-      p->sync();
-    });
-  }
-  std::vector<int> I((size_t)nr * nc), J((size_t)nr * nc);
-  for (int c = 0; c < nc; ++c)
-    for (int r = 0; r < nr; ++r) { I[r + (size_t)c * nr] = rows[r]; J[r + (size_t)c * nr] = cols[c]; }
-  return aifmm_entries(p, (long)nr * nc, I.data(), J.data(), out, AIFMM_PTR_HOST);
+  return guard(p, [&] {
+    const bool dev = flags & AIFMM_PTR_DEVICE;
+    if ((long)nr * nc == 0) return;
+    if (!dev) {
+      for (int r = 0; r < nr; ++r)
+        if (rows[r] < 0 || rows[r] >= p->N) throw Fail(AIFMM_ERR_ARG, "point index out of range");
+      for (int c = 0; c < nc; ++c)
+        if (cols[c] < 0 || cols[c] >= p->N) throw Fail(AIFMM_ERR_ARG, "point index out of range");
+    }
+    // host memory: the index lists travel and the block comes back
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
+    const size_t bytes = sizeof(double2) * (size_t)nr * nc;
+    aifmm_problem::Tmp tr(p, dev ? 1 : sizeof(int) * (size_t)nr), tc(p, dev ? 1 : sizeof(int) * (size_t)nc);
+    aifmm_problem::Tmp to(p, dev ? 1 : bytes);
+    BlockDesc bd{rows, cols, nr, nc, reinterpret_cast<double2*>(out), nr, 0};
+    if (!dev) {
+      CK(cudaMemcpyAsync(tr.ptr, rows, sizeof(int) * (size_t)nr, cudaMemcpyHostToDevice, p->st));
+      CK(cudaMemcpyAsync(tc.ptr, cols, sizeof(int) * (size_t)nc, cudaMemcpyHostToDevice, p->st));
+      bd.rows = tr.as<int>(); bd.cols = tc.as<int>(); bd.out = to.as<double2>();
+    }
+    std::vector<BlockDesc> v{bd};
+    p->launch_blocks(v);
+    if (!dev) CK(cudaMemcpyAsync(out, to.ptr, bytes, cudaMemcpyDeviceToHost, p->st));
+    p->sync();
+  });
 }
 
 aifmm_status aifmm_build_tree(aifmm_problem* p) {
