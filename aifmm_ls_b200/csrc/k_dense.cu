@@ -722,9 +722,14 @@ __global__ void __launch_bounds__(kT) norm_kernel(const NormDesc* __restrict__ d
   pdl_wait();
   __shared__ double sh[kW + 1];
   double s = 0.0;
-  for (long long e = threadIdx.x; e < (long long)D.m * D.n; e += kT) {
-    int i = (int)(e % D.m), j = (int)(e / D.m);
-    s += cabs2(ld_any(D.A, i + (size_t)j * D.lda, D.es));
+  const int tot = D.m * D.n;
+  if (D.lda == D.m) {  // contiguous: no division per element
+    for (int e = threadIdx.x; e < tot; e += kT) s += cabs2(ld_any(D.A, e, D.es));
+  } else {
+    for (int e = threadIdx.x; e < tot; e += kT) {
+      const int j = e / D.m, i = e - j * D.m;
+      s += cabs2(ld_any(D.A, i + (size_t)j * D.lda, D.es));
+    }
   }
   s = block_sum(s, sh);
   if (threadIdx.x == 0) {

@@ -1565,6 +1565,7 @@ struct aifmm_problem {
   struct Step {
     int k;
     bool on = false;   // box k carries unknowns
+    bool bases_kept = false;  // no recompression in this step
     Blk XL, W[8];
     std::vector<std::pair<int, int>> p2p, p2l;
   };
@@ -1585,7 +1586,7 @@ struct aifmm_problem {
     CK(cudaEventRecord(ev_join, st2));
     cur = st;
   }
-  void eliminate_x_side(int j, std::vector<Step>& ws) {
+  void eliminate_x_factor(int j, std::vector<Step>& ws) {
     fork();
     for (Step& S : ws) {
       Box& B = T[j][S.k];
@@ -1593,6 +1594,13 @@ struct aifmm_problem {
       if (S.on) qr_prepare(B.qx, B.P2P[S.k], 0.0, true);  // factored in place; P2P[k][k] is not read again
     }
     flush_qr();
+    cur = st;
+  }
+  // The solves follow once the pending pairs are known: a box without any keeps its
+  // bases in this step, so the solve with L2P_k joins the batch instead of waiting for
+  // the recompressions.
+  void eliminate_x_side(int j, std::vector<Step>& ws) {
+    cur = st2;
     for (Step& S : ws) {
       if (!S.on) continue;
       Box& B = T[j][S.k];
@@ -1604,6 +1612,11 @@ struct aifmm_problem {
         S.W[pI] = scr(m, src.c);
         solve(B.qx, src, S.W[pI], C1);
       }
+      S.bases_kept = S.p2p.empty() && S.p2l.empty();
+      if (S.bases_kept) {
+        S.XL = scr(m, B.L2P.c);
+        solve(B.qx, B.L2P, S.XL, C1);
+      }
     }
     flush_solve();
     unfork();
@@ -1612,6 +1625,7 @@ struct aifmm_problem {
     CK(cudaStreamWaitEvent(st, ev_join, 0));
     for (Step& S : ws) {
       if (!S.on) { eliminate_x_empty(j, S.k); continue; }
+      if (S.bases_kept) continue;
       Box& B = T[j][S.k];
       S.XL = scr(B.P2P[S.k].c, B.L2P.c);
       solve(B.qx, B.L2P, S.XL, C1);
@@ -2333,9 +2347,10 @@ struct aifmm_problem {
         auto tp0 = std::chrono::steady_clock::now();
         std::vector<Step> ws(ks.size());
         for (size_t i = 0; i < ks.size(); ++i) ws[i].k = ks[i];
-        eliminate_x_side(j, ws);
+        eliminate_x_factor(j, ws);
         waited[0] = waited[1] = false;
         for (Step& S : ws) take_pending(S);
+        eliminate_x_side(j, ws);
         // the i-th pair of every step of the wave as one round
         for (size_t i = 0, more = 1; more; ++i) {
           more = 0;
