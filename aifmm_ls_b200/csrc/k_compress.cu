@@ -204,37 +204,40 @@ __device__ __forceinline__ void cta_gemm_s(C* Cm, int ldc, int m, int n, int k, 
 
 // One step range of formq: the reflectors k in [4 I0, 4 I1), downwards, on the
 // group's column cc (nothing while k > cc).
+// All lanes of a warp run along, those of columns without reflector k with a zero
+// update, so that the shuffles name the whole warp.
 template <typename C, int RPL, int I0>
 __device__ __forceinline__ void formq_reg_phase(const C* F, int ldf, const C* tau, int m, int kmax, int cc, int p,
                                                 int lane, C (&q)[RPL]) {
   constexpr int I1 = I0 + qr_phase_rows(RPL) < RPL ? I0 + qr_phase_rows(RPL) : RPL;
   if constexpr (I1 < RPL) formq_reg_phase<C, RPL, I1>(F, ldf, tau, m, kmax, cc, p, lane, q);
-  const unsigned gm = 0xfu << (lane & ~3);
+  const unsigned full = 0xffffffffu;
   for (int k = min(kmax, 4 * I1 - 1); k >= 4 * I0; --k) {
-    if (k > cc) continue;
     const C* v = F + (size_t)k * ldf;
+    const bool on = k <= cc;
     C qk = cplx<C>::mk(0.0, 0.0);
 #pragma unroll
     for (int i = I0; i < I1; ++i)
       if (p + 4 * i == k) qk = q[i];
     const int src = (lane & ~3) | (k & 3);
-    qk.x = __shfl_sync(gm, qk.x, src);
-    qk.y = __shfl_sync(gm, qk.y, src);
+    qk.x = __shfl_sync(full, qk.x, src);
+    qk.y = __shfl_sync(full, qk.y, src);
     C d = cplx<C>::mk(0.0, 0.0);
 #pragma unroll
     for (int i = I0; i < RPL; ++i)
       if ((unsigned)(p + 4 * i - k - 1) < (unsigned)(m - k - 1)) d = cfmac(v[p + 4 * i], q[i], d);
-    d.x += __shfl_xor_sync(gm, d.x, 1); d.y += __shfl_xor_sync(gm, d.y, 1);
-    d.x += __shfl_xor_sync(gm, d.x, 2); d.y += __shfl_xor_sync(gm, d.y, 2);
-    const C tw = cmul_p(cconj(tau[k]), cadd(qk, d));
+    d.x += __shfl_xor_sync(full, d.x, 1); d.y += __shfl_xor_sync(full, d.y, 1);
+    d.x += __shfl_xor_sync(full, d.x, 2); d.y += __shfl_xor_sync(full, d.y, 2);
+    C tw = cmul_p(cconj(tau[k]), cadd(qk, d));
+    const C qn = csub(qk, tw);
+    if (!on) tw = cplx<C>::mk(0.0, 0.0);
     if (RPL > 16) asm volatile("" ::: "memory");
 #pragma unroll
     for (int i = I0; i < RPL; ++i)
       if ((unsigned)(p + 4 * i - k - 1) < (unsigned)(m - k - 1)) q[i] = csub(q[i], cmul_p(v[p + 4 * i], tw));
-    const C qn = csub(qk, tw);
 #pragma unroll
     for (int i = I0; i < I1; ++i)
-      if (p + 4 * i == k) q[i] = qn;
+      if (on && p + 4 * i == k) q[i] = qn;
   }
 }
 
@@ -245,7 +248,7 @@ template <typename C, int RPL>
 __device__ __forceinline__ void cta_formq_reg(C* F, int ldf, const C* tau, int m, int size, int ncols, C* Q) {
   const int lane = threadIdx.x & 31, p = threadIdx.x & 3, cc = threadIdx.x >> 2;
   C q[RPL];
-  if (cc < ncols) {
+  if (cc - (lane >> 2) < ncols) {  // the same in a whole warp
 #pragma unroll
     for (int i = 0; i < RPL; ++i) q[i] = cplx<C>::mk(p + 4 * i == cc ? 1.0 : 0.0, 0.0);
     formq_reg_phase<C, RPL, 0>(F, ldf, tau, m, min(size, ncols) - 1, cc, p, lane, q);

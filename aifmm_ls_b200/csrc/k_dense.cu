@@ -518,17 +518,17 @@ __global__ void __launch_bounds__(32 * WM * WN * (NS == 1 ? 1 : 2)) gemm_kernel(
 // R, the column permutation.
 // What bounds it: the chain of 2 nzp dependent steps; a reflector's is its dot
 // product over eight lanes (three shuffles: the two upper levels of the sum over 32
-// rows stay in a lane), tau and the update, about 430 cycles of it instruction issue
-// and latency in equal parts.  36 x 36, 12 boxes, 8 columns: 18.6 us (a warp per
-// column: 20.8 us); 300 boxes: 21 us (36 us).
+// rows stay in a lane), tau and the update, about 350 cycles of it instruction issue
+// and latency in equal parts.  36 x 36, 12 boxes, 8 columns: 15.2 us (a warp per
+// column: 20.8 us); 300 boxes: 19 us (36 us).
 // Sums run in the order of 32 lanes over the rows (row mod 32), levels 16 to 1.
 constexpr int kSolveCols = 16, kSolveT = 8 * kSolveCols;
 // rows of a phase (x 8): the rows of earlier phases cost nothing in a forward step
 __host__ __device__ constexpr int solve_phase(int rpl) { return (rpl + 5) / 6; }
 
 template <typename C, int RPL, int I0>
-__device__ __forceinline__ void solve_forward(const C* F, int ldf, const C* tau, int m, int nzp, int q, unsigned gm,
-                                              C (&b)[RPL]) {
+__device__ __forceinline__ void solve_forward(const C* F, int ldf, const C* tau, int m, int nzp, int q, C (&b)[RPL]) {
+  const unsigned full = 0xffffffffu;  // every lane of a warp runs along
   constexpr int I1 = I0 + solve_phase(RPL) < RPL ? I0 + solve_phase(RPL) : RPL;
   const int kend = min(8 * I1, nzp);
   constexpr bool ahead = RPL <= 12;  // more rows: the registers do not hold two reflectors
@@ -558,13 +558,13 @@ __device__ __forceinline__ void solve_forward(const C* F, int ldf, const C* tau,
 #pragma unroll
     for (int t = I0; t < I1; ++t)
       if (q + 8 * t == k) bk = b[t];
-    bk.x = __shfl_sync(gm, bk.x, k & 7, 8);
-    bk.y = __shfl_sync(gm, bk.y, k & 7, 8);
+    bk.x = __shfl_sync(full, bk.x, k & 7, 8);
+    bk.y = __shfl_sync(full, bk.y, k & 7, 8);
     C z = cadd(cadd(s[0], s[2]), cadd(s[1], s[3]));
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) {
-      z.x += __shfl_xor_sync(gm, z.x, o);
-      z.y += __shfl_xor_sync(gm, z.y, o);
+      z.x += __shfl_xor_sync(full, z.x, o);
+      z.y += __shfl_xor_sync(full, z.y, o);
     }
     // (the complex64 form has always fused the other product here)
     const C tw = sizeof(C) == 16 ? cmul_p(tk, cadd(bk, z)) : cmul_t(tk, cadd(bk, z));
@@ -576,15 +576,15 @@ __device__ __forceinline__ void solve_forward(const C* F, int ldf, const C* tau,
     }
   }
   if constexpr (I1 < RPL) {
-    if (nzp > 8 * I1) solve_forward<C, RPL, I1>(F, ldf, tau, m, nzp, q, gm, b);
+    if (nzp > 8 * I1) solve_forward<C, RPL, I1>(F, ldf, tau, m, nzp, q, b);
   }
 }
 template <typename C, int RPL, int I0>
-__device__ __forceinline__ void solve_backward(const C* F, int ldf, const double2* rinv, int nzp, int q, unsigned gm,
-                                               C (&b)[RPL]) {
+__device__ __forceinline__ void solve_backward(const C* F, int ldf, const double2* rinv, int nzp, int q, C (&b)[RPL]) {
+  const unsigned full = 0xffffffffu;
   constexpr int I1 = I0 + solve_phase(RPL) < RPL ? I0 + solve_phase(RPL) : RPL;
   if constexpr (I1 < RPL) {
-    if (nzp > 8 * I1) solve_backward<C, RPL, I1>(F, ldf, rinv, nzp, q, gm, b);
+    if (nzp > 8 * I1) solve_backward<C, RPL, I1>(F, ldf, rinv, nzp, q, b);
   }
   for (int i = min(nzp, 8 * I1) - 1; i >= 8 * I0; --i) {
     C r[RPL];
@@ -596,8 +596,8 @@ __device__ __forceinline__ void solve_backward(const C* F, int ldf, const double
 #pragma unroll
     for (int t = I0; t < I1; ++t)
       if (q + 8 * t == i) bi = b[t];
-    bi.x = __shfl_sync(gm, bi.x, i & 7, 8);
-    bi.y = __shfl_sync(gm, bi.y, i & 7, 8);
+    bi.x = __shfl_sync(full, bi.x, i & 7, 8);
+    bi.y = __shfl_sync(full, bi.y, i & 7, 8);
     const C xi = cplx<C>::from(cmul_p(c2d(bi), ri));
 #pragma unroll
     for (int t = 0; t < I1; ++t) {
@@ -656,22 +656,22 @@ __global__ void __launch_bounds__(kSolveT) qr_solve_reg_kernel(const SolveJob* _
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
-  if (!mine) return;
+  if (c - (lane >> 3) >= J.nrhs) return;  // the same in a whole warp
   C* x = static_cast<C*>(J.X) + (size_t)c * J.ldx;
-  const unsigned gm = 0xffu << (lane & ~7);
   if (nzp > 0) {
-    solve_forward<C, RPL, 0>(F, ldf, tau, m, nzp, q, gm, b);
-    solve_backward<C, RPL, 0>(F, ldf, rinv, nzp, q, gm, b);
+    solve_forward<C, RPL, 0>(F, ldf, tau, m, nzp, q, b);
+    solve_backward<C, RPL, 0>(F, ldf, rinv, nzp, q, b);
   }
   if (nzp < n) {
-    for (int i = q; i < n; i += 8) x[i] = cplx<C>::mk(0.0, 0.0);
-    __syncwarp(gm);
+    if (mine)
+      for (int i = q; i < n; i += 8) x[i] = cplx<C>::mk(0.0, 0.0);
+    __syncwarp();
   }
   const C alpha = cplx<C>::from(J.alpha);
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
     const int i = q + 8 * t;
-    if (i < nzp) x[J.perm[i]] = cmul(alpha, b[t]);
+    if (mine && i < nzp) x[J.perm[i]] = cmul(alpha, b[t]);
   }
 }
 

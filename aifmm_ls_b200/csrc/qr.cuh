@@ -29,7 +29,9 @@ constexpr int kQrGroups = kT / 4;
 //   4. barrier.
 // What bounds it: the chain of a step -- the norm reduction, square root and
 // division of the reflector, the columns' dot products, the square root of the
-// downdate -- not FP64 throughput.  Finished columns stay in registers until the
+// downdate -- not FP64 throughput: about 2,500 cycles a step.  36 x 57 complex128:
+// 94 us with the shared-memory kernel, 49 us here; 64 x 64: 180 and 101 us; 90 x 90: 406
+// and 255 us.  Finished columns stay in registers until the
 // end; rows above 4 I0 are finished in phase I0 and cost nothing there.
 // Sums run in the order of qr_smem_body, so that a block's factors do not depend on
 // the kernel that takes it: lane p adds its rows with i = row / 4 even and odd in two
@@ -61,14 +63,14 @@ struct RegQr {
 
 // the sum of squares of this column's rows > k0 in the order of 32 lanes over rows k0 + 1 + l
 template <typename C, int RPL, int I0>
-__device__ __forceinline__ double qr_reg_tail(const C (&col)[RPL], int k0, int p, int nfree, unsigned gm) {
+__device__ __forceinline__ double qr_reg_tail(const C (&col)[RPL], int k0, int p, int nfree, unsigned full) {
   double s[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int i = I0; i < RPL; ++i)
     if (i >= nfree || p + 4 * i > k0) s[i & 7] += cabs2_p(col[i]);
   double z = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));
-  z += __shfl_xor_sync(gm, z, 2);
-  z += __shfl_xor_sync(gm, z, 1);
+  z += __shfl_xor_sync(full, z, 2);
+  z += __shfl_xor_sync(full, z, 1);
   return z;
 }
 
@@ -76,7 +78,7 @@ template <typename C, int RPL, int NQ, int I0>
 __device__ __forceinline__ void qr_reg_phase(RegQr<C>& S, C (&col)[RPL]) {
   constexpr int I1 = I0 + qr_phase_rows(RPL) < RPL ? I0 + qr_phase_rows(RPL) : RPL;
   constexpr int I2 = I1 + 1 < RPL ? I1 + 1 : RPL;  // row k + 1 may be the next phase's first
-  const unsigned full = 0xffffffffu, gm = 0xfu << (S.lane & ~3);
+  const unsigned full = 0xffffffffu;
   const int m = S.m, n = S.n, lane = S.lane, p = S.p;
   const int kend = min(4 * I1, S.size);
   C* const V = S.V;
@@ -131,6 +133,7 @@ __device__ __forceinline__ void qr_reg_phase(RegQr<C>& S, C (&col)[RPL]) {
     // 2. the owner's reflector, rows k..m-1; the others' norms
     const double2 c0 = c2d(S.a);
     const double root = sqrt(owner ? cabs2_p(c0) + S.z : S.tt);
+    double rkk = 0.0;
     if (owner) {
       double beta;
       C t;
@@ -170,26 +173,33 @@ __device__ __forceinline__ void qr_reg_phase(RegQr<C>& S, C (&col)[RPL]) {
       if (p == 0) {
         *S.s_tau = t;
         *S.s_pos = S.pos;
-        S.srd[k] = fabs(beta);
-        // exactly nonzero pivots; the norm itself only near the threshold
-        const double lim = S.thr_helper * (double)(m - k);
-        if (!(S.tt > 2.0 * lim) && *S.s_nzp == S.size) {
-          const double nub = sqrt(S.tt);
-          if (nub * nub < lim) *S.s_nzp = k;
-        }
       }
       S.tau = t;
       S.pos = k;
       S.done = true;
+      rkk = fabs(beta);
     }
     __syncthreads();
-    // 3. G = I - t v v^H on the columns at positions > k; norm downdates
+    if (owner && p == 0) {
+      S.srd[k] = rkk;
+      // exactly nonzero pivots; the norm itself only near the threshold
+      const double lim = S.thr_helper * (double)(m - k);
+      if (!(S.tt > 2.0 * lim) && *S.s_nzp == S.size) {
+        const double nub = sqrt(S.tt);
+        if (nub * nub < lim) *S.s_nzp = k;
+      }
+    }
+    // 3. G = I - t v v^H on the columns at positions > k; norm downdates.  The lanes of
+    //    finished columns run along with a zero update, so that a warp never splits and
+    //    its shuffles name all lanes; a warp of finished columns skips the step.
     unsigned hnext = 0;
-    if (!S.done) {
+    if (!__all_sync(full, S.done)) {
+      const bool on = !S.done;
       const double nu = root;
-      if (S.fresh) { S.nd = nu; S.fresh = false; }
+      if (on && S.fresh) S.nd = nu;
+      S.fresh = false;
       const C t = *S.s_tau;
-      if (S.pos == k) S.pos = *S.s_pos;
+      if (on && S.pos == k) S.pos = *S.s_pos;
       C d0 = cplx<C>::mk(0.0, 0.0), d1 = cplx<C>::mk(0.0, 0.0);
 #pragma unroll
       for (int i = I0; i < RPL; ++i)
@@ -198,43 +208,42 @@ __device__ __forceinline__ void qr_reg_phase(RegQr<C>& S, C (&col)[RPL]) {
           else d0 = cfmac(V[p + 4 * i], col[i], d0);
         }
       C d = cadd(d0, d1);
-      d.x += __shfl_xor_sync(gm, d.x, 1); d.y += __shfl_xor_sync(gm, d.y, 1);
-      d.x += __shfl_xor_sync(gm, d.x, 2); d.y += __shfl_xor_sync(gm, d.y, 2);
-      const C tw = cmul_t(t, cadd(S.a, d));
+      d.x += __shfl_xor_sync(full, d.x, 1); d.y += __shfl_xor_sync(full, d.y, 1);
+      d.x += __shfl_xor_sync(full, d.x, 2); d.y += __shfl_xor_sync(full, d.y, 2);
+      C tw = cmul_t(t, cadd(S.a, d));
       const C rkj = csub(S.a, tw);
+      if (!on) tw = cplx<C>::mk(0.0, 0.0);
       if (RPL > 16) asm volatile("" ::: "memory");  // read v again rather than keep it in registers
 #pragma unroll
       for (int i = I0; i < RPL; ++i)
         if (i >= I1 || p + 4 * i > k) col[i] = csub(col[i], cmul_p(V[p + 4 * i], tw));
 #pragma unroll
       for (int i = I0; i < I1; ++i)
-        if (p + 4 * i == k) col[i] = rkj;
+        if (on && p + 4 * i == k) col[i] = rkj;
       // the next step's element and sum of squares
       C an = cplx<C>::mk(0.0, 0.0);
 #pragma unroll
       for (int i = I0; i < I2; ++i)
         if (p + 4 * i == k + 1) an = col[i];
       const int src = (lane & ~3) | ((k + 1) & 3);
-      S.a.x = __shfl_sync(gm, an.x, src);
-      S.a.y = __shfl_sync(gm, an.y, src);
-      S.z = qr_reg_tail<C, RPL, I0>(col, k + 1, p, I2, gm);
-      if (nu != 0.0) {
-        const double ar = sqrt(cabs2_p(rkj));
-        double tt = (nu - ar) * (nu + ar);
-        if (tt < 0.0) tt = 0.0;
-        if (tt <= S.downdate_thr * (S.nd * S.nd)) {
-          double q = 0.0;
+      S.a.x = __shfl_sync(full, an.x, src);
+      S.a.y = __shfl_sync(full, an.y, src);
+      S.z = qr_reg_tail<C, RPL, I0>(col, k + 1, p, I2, full);
+      const double ar = sqrt(cabs2_p(rkj));
+      double tt = (nu - ar) * (nu + ar);
+      if (tt < 0.0) tt = 0.0;
+      const bool again = on && nu != 0.0 && tt <= S.downdate_thr * (S.nd * S.nd);
+      if (__any_sync(full, again)) {
+        double q = 0.0;
 #pragma unroll
-          for (int i = I0; i < RPL; ++i)
-            if (i >= I1 || p + 4 * i > k) q += cabs2_p(col[i]);
-          q += __shfl_xor_sync(gm, q, 1);
-          q += __shfl_xor_sync(gm, q, 2);
-          tt = q;
-          S.fresh = true;
-        }
-        S.tt = tt;
+        for (int i = I0; i < RPL; ++i)
+          if (i >= I1 || p + 4 * i > k) q += cabs2_p(col[i]);
+        q += __shfl_xor_sync(full, q, 1);
+        q += __shfl_xor_sync(full, q, 2);
+        if (again) { tt = q; S.fresh = true; }
       }
-      hnext = (unsigned)__double2hiint(S.tt);
+      if (on && nu != 0.0) S.tt = tt;
+      if (on) hnext = (unsigned)__double2hiint(S.tt);
     }
     if (p == 0 && S.g < n) S.hi2[((k + 1) & 1) * n + S.g] = hnext;
     __syncthreads();
