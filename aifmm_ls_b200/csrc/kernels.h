@@ -134,6 +134,7 @@ struct CompressJob {
 int aifmm_launch_tables(int n_cheb, int degree, double kappa, double r, const double* gl_x, const double* gl_w,
                         const int2* basis, const double* cheb, double2* Cwork, double2* Vwork, int* status,
                         double* qpinv, double2* M, double2* nearT, cudaStream_t stream);
+int aifmm_launch_round6(double2* M, double2* nearT, int rank, int* left, cudaStream_t stream);
 int aifmm_launch_block_entries(const BlockDesc* d_desc, const long long* d_off, int nd, long long total,
                                const EntryCtx& ctx, cudaStream_t stream);
 int aifmm_launch_list_entries(const int* I, const int* J, long n, double2* out, const EntryCtx& ctx,

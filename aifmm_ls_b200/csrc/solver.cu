@@ -1039,15 +1039,17 @@ struct aifmm_problem {
     const int2* db = stage.put(basis, st);
     const double* dc = stage.put(cheb, st);
     Tmp Cw(this, sizeof(double2) * 121 * nb), Vw(this, sizeof(double2) * 9 * rank * nb);
-    Tmp status(this, sizeof(int)), qp(this, sizeof(double) * nb * rank);
-    CK(cudaMemsetAsync(status.ptr, 0, sizeof(int), st));
+    Tmp status(this, 2 * sizeof(int)), qp(this, sizeof(double) * nb * rank);
+    CK(cudaMemsetAsync(status.ptr, 0, 2 * sizeof(int), st));
     KL(aifmm_launch_tables(d.n_cheb, d.degree, d.kappa, r, dx, dw, db, dc, Cw.as<double2>(), Vw.as<double2>(),
                            status.as<int>(), qp.as<double>(), d_M, d_near, st));
-    int h_status = 0;
-    CK(cudaMemcpyAsync(&h_status, status.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // the reference's 6-digit text round trip (LS_Assembly.hpp:1178-1228, 1382-1459)
+    if (do_round) KL(aifmm_launch_round6(d_M, d_near, rank, status.as<int>() + 1, st));
+    int h_status[2] = {0, 0};
+    CK(cudaMemcpyAsync(h_status, status.ptr, sizeof h_status, cudaMemcpyDeviceToHost, st));
     sync();
-    if (h_status) throw Fail(AIFMM_ERR_NUMERIC, "adaptive quadrature exhausted its panel budget");
-    if (do_round) {  // the reference's 6-digit text round trip (LS_Assembly.hpp:1178-1228, 1382-1459)
+    if (h_status[0]) throw Fail(AIFMM_ERR_NUMERIC, "adaptive quadrature exhausted its panel budget");
+    if (h_status[1]) {  // a value of 9e5 or above, which the device leaves: all through text here
       std::vector<double> M(2 * 121 * rank), Nt(2 * 9 * rank * rank);
       CK(cudaMemcpyAsync(M.data(), d_M, sizeof(double) * M.size(), cudaMemcpyDeviceToHost, st));
       CK(cudaMemcpyAsync(Nt.data(), d_near, sizeof(double) * Nt.size(), cudaMemcpyDeviceToHost, st));
