@@ -103,6 +103,7 @@ struct EntryCtx {
   const double2* M;       // far-field coefficients, 121 x rank, column-major
   const double2* Mt;      // the same, transposed: the rank sources of one order next to each other
   const double2* nearT;   // 9 near tables, rank x rank column-major each
+  const double* far_bound;  // no far entry exceeds kappa^2 |q| times this (far_bound_kernel)
 };
 
 #define AIFMM_CUDA_OK(call) ((call) == cudaSuccess)

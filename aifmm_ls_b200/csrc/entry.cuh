@@ -231,8 +231,13 @@ __device__ __forceinline__ int near_dir(int dx, int dy) {
 // factor, no identity), the operator the reference applies to the solution to
 // get the scattered field (hybrid.cpp:263-281).
 // ENX: see far_series (the ACA's entries have always fused the other product).
+// Entries below 1e-16 are zero (LS_Assembly.hpp:536-538); a far entry whose bound
+// kappa^2 |q_i| max_j sum_n |M_nj| |H_n| is below half of `floor` is returned as zero
+// without its series.  With the floor of 1e-16 that changes no result: the bound holds
+// for every distance (|H_n| decreases), and half leaves room for the rounding of both.
+// Rows outside the contrast's support cost one load instead of 61 orders.
 template <bool PHI = true, int ENX = 1>
-__device__ __forceinline__ double2 lsa_entry(int i, int j, const EntryCtx& c) {
+__device__ __forceinline__ double2 lsa_entry(int i, int j, const EntryCtx& c, double floor = 1e-16) {
   const int rank = c.rank;
   const int li = i / rank, ii = i - li * rank;
   const int lj = j / rank, jj = j - lj * rank;
@@ -253,6 +258,7 @@ __device__ __forceinline__ double2 lsa_entry(int i, int j, const EntryCtx& c) {
     if (hypot(e.x, e.y) < 1e-16) e = make_double2(0.0, 0.0);
     return e;
   }
+  if (PHI && c.kappa * c.kappa * fabs(qi) * __ldg(c.far_bound) < 0.5 * floor) return make_double2(0.0, 0.0);
   const double2 ri = __ldg(&c.pts[i]);
   const double2 cj = __ldg(&c.leafc[lj]);
   const double ddy = ri.y - cj.y, ddx = ri.x - cj.x;

@@ -5,6 +5,7 @@
 // 2 TR, 3 TL; leaf nodes r * cheb + centre, local index y*n + x) and the
 // contrast / right-hand side functions of LS/LS_functions.hpp:1-120.
 #include <algorithm>
+#include <cfloat>
 
 #include "kernels.h"
 
@@ -142,6 +143,40 @@ __global__ void transpose_kernel(const double2* __restrict__ a, double2* __restr
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < r * c; e += gridDim.x * blockDim.x) b[e] = a[e / c + (size_t)(e % c) * r];
 }
 }  // namespace
+namespace {
+// max_j (1/4) sum_n |M_nj| |H_n(x)| at the smallest far distance x = 3 kappa r (a point of
+// one leaf, half side r, to the centre of a leaf that does not touch it): with J_n^2 + Y_n^2
+// decreasing, a bound of every far entry / (kappa^2 q).  Infinite if a term is not finite.
+__global__ void far_bound_kernel(const double2* __restrict__ M, int rank, double x, double* out) {
+  constexpr int NS = 60;  // orders of the far field
+  __shared__ double H[NS + 1], top[32];
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  if (tid <= NS) H[tid] = hypot(jn(tid, x), yn(tid, x));
+  __syncthreads();
+  double best = 0.0;
+  for (int j = w; j < rank; j += blockDim.x >> 5) {
+    double s = 0.0;
+    for (int n = lane - NS; n <= NS; n += 32) {
+      const double2 m = M[(size_t)j * (2 * NS + 1) + n + NS];
+      s += hypot(m.x, m.y) * H[n < 0 ? -n : n];
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (!(s < DBL_MAX)) s = INFINITY;
+    best = fmax(best, s);
+  }
+  if (lane == 0) top[w] = best;
+  __syncthreads();
+  if (tid == 0) {
+    for (int k = 1; k < (int)blockDim.x >> 5; ++k) best = fmax(best, top[k]);
+    *out = 0.25 * best;
+  }
+}
+}  // namespace
+int aifmm_launch_far_bound(const double2* M, int rank, double kappa, double r, double* out, cudaStream_t s) {
+  far_bound_kernel<<<1, 1024, 0, s>>>(M, rank, 3.0 * kappa * r, out);
+  return (int)cudaGetLastError();
+}
+
 int aifmm_launch_transpose(const double2* a, double2* b, int r, int c, cudaStream_t s) {
   transpose_kernel<<<(r * c + 255) / 256, 256, 0, s>>>(a, b, r, c);
   return (int)cudaGetLastError();

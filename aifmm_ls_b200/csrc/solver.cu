@@ -39,6 +39,7 @@ int aifmm_launch_rhs_plane_wave(const double2* pts, const double* q, double kapp
                                 const double* theta, double2* b, cudaStream_t s);
 int aifmm_launch_incident_field(const double2* pts, double kappa, int N, int nrhs, const double* theta, double2* u,
                                 cudaStream_t s);
+int aifmm_launch_far_bound(const double2* M, int rank, double kappa, double r, double* out, cudaStream_t s);
 int aifmm_launch_transpose(const double2* a, double2* b, int r, int c, cudaStream_t s);
 int aifmm_launch_gather_segments(const int* src, const int4* segs, long nseg, int* dst, cudaStream_t s);
 size_t aifmm_error_norms_scratch_bytes();
@@ -420,6 +421,7 @@ struct aifmm_problem {
   double tol = 0;         // ACA (assembly) tolerance, 10^-tol_pow
   double tol_factor = 0;  // recompression tolerance of the factorisation (tol unless set)
   // device geometry and tables
+  double* d_bound = nullptr;  // of the far entries (EntryCtx)
   double2 *d_pts = nullptr, *d_leafc = nullptr, *d_M = nullptr, *d_Mt = nullptr, *d_near = nullptr;
   double* d_q = nullptr;
   int2* d_leafxy = nullptr;
@@ -458,6 +460,7 @@ struct aifmm_problem {
     EntryCtx c;
     c.rank = rank; c.depth = depth; c.kappa = d.kappa;
     c.pts = d_pts; c.q = d_q; c.leafc = d_leafc; c.leafxy = d_leafxy; c.M = d_M; c.Mt = d_Mt; c.nearT = d_near;
+    c.far_bound = d_bound;
     return c;
   }
 
@@ -982,6 +985,7 @@ struct aifmm_problem {
     CK(cudaMalloc(&d_leafxy, sizeof(int2) * nleaf));
     CK(cudaMalloc(&d_M, sizeof(double2) * 121 * rank));
     CK(cudaMalloc(&d_Mt, sizeof(double2) * 121 * rank));
+    CK(cudaMalloc(&d_bound, sizeof(double)));
     CK(cudaMalloc(&d_near, sizeof(double2) * 9 * rank * rank));
     CK(cudaMalloc(&d_iota, sizeof(int) * N));
     std::vector<int> iota(N);
@@ -1007,6 +1011,7 @@ struct aifmm_problem {
     release_plans();
     pool.release_all();
     cudaFree(d_pts); cudaFree(d_q); cudaFree(d_leafc); cudaFree(d_leafxy); cudaFree(d_M); cudaFree(d_Mt); cudaFree(d_near);
+    cudaFree(d_bound);
     cudaFree(d_iota);
     if (h_norms) cudaFreeHost(h_norms);
     if (h_ranks) cudaFreeHost(h_ranks);
@@ -1017,9 +1022,11 @@ struct aifmm_problem {
     if (ev_join) cudaEventDestroy(ev_join);
   }
 
-  // the far-field coefficients with the sources of an order next to each other (entry.cuh)
+  // what the entries take from the far-field coefficients: the sources of an order next to
+  // each other, and a bound (entry.cuh)
   void transpose_M() {
     KL(aifmm_launch_transpose(d_M, d_Mt, 121, rank, st));
+    KL(aifmm_launch_far_bound(d_M, rank, d.kappa, d.L / (double)(1 << depth), d_bound, st));
     sync();
   }
   void tables_compute(int do_round) {
