@@ -48,146 +48,215 @@ __device__ R block_sum(R x, R* sh) {
 }
 
 // ---------------------------------------------------------------- QR factor
-// The factorisation runs on A (lda), nu/nd (norm arrays) and perm, either in
-// global memory or staged in shared memory (qr_factor_smem_kernel).
+// Blocks that neither the registers nor the shared memory of a CTA hold (qr.cuh): the
+// matrix in global memory, one CTA of 32 warps, the norms and the reflector in shared
+// memory where they fit.  A pivot step:
+//   1. every warp picks the pivot by itself from the norms (no barrier);
+//   2. the pivot column changes places, into shared memory too;
+//   3. the sum of squares below the diagonal: 256 partial sums, folded in eight groups
+//      of 32, then in order; the reflector;
+//   4. every warp applies it to two columns at a time;
+//   5. the norms are downdated, a thread a column.
+// What bounds it: the columns' way from L2 through one SM (a block of 120 x 120 is 230 KB)
+// and the chain of a step.  With 8 warps, the norms in global memory, a thread that scans
+// them for the pivot and a warp's 32 lanes all downdating one norm: 1.41 ms for 130 x 120
+// complex128, 4.74 ms for 200 x 200, 3.68 ms for 200 x 200 complex64; now 0.84, 2.34 and
+// 1.55 ms.
+constexpr int kQrT = 1024, kQrW = kQrT / 32, kQrSumW = 8;
+
 template <typename C>
-__device__ void qr_factor_body(const QRJob& J, C* A, int lda, double* nu, double* nd, int* perm) {
-  __shared__ double sh[kW + 1];
-  __shared__ double sv[kW]; __shared__ int si[kW];
+__global__ void __launch_bounds__(kQrT) qr_factor_kernel(const QRJob* __restrict__ jobs, int mcap, int ncap) {
+  constexpr unsigned full = 0xffffffffu;
+  const QRJob J = jobs[blockIdx.x];
+  extern __shared__ double2 qr_sm[];
+  __shared__ double sh[kQrSumW];
   __shared__ C s_tau;
-  __shared__ int s_big;
+  __shared__ int s_rank;
+  C* const A = static_cast<C*>(J.a);
+  const int lda = J.lda;
   C* tau = static_cast<C*>(J.tau);
+  int* perm = J.perm;
   const int m = J.m, n = J.n, size = min(m, n);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  for (int j = tid; j < n; j += kT) perm[j] = j;
+  const bool staged = m <= mcap && n <= ncap;
+  C* const sv = reinterpret_cast<C*>(qr_sm);
+  double* const nu = staged ? reinterpret_cast<double*>(sv + ((mcap + 1) & ~1)) : J.norms;
+  double* const nd = nu + n;
+  C* const row = reinterpret_cast<C*>(nu + 2 * ncap);  // row k, for the norms
+  for (int j = tid; j < n; j += kQrT) perm[j] = j;
+  if (tid == 0) s_rank = 0;
   // initial column norms (one warp per column)
-  for (int j = w; j < n; j += kW) {
+  for (int j = w; j < n; j += kQrW) {
     double s = 0.0;
-    for (int i = lane; i < m; i += 32) s += cabs2d(A[i + (size_t)j * lda]);
+    for (int i = lane; i < m; i += 32) s += cabs2_p(A[i + (size_t)j * lda]);
     s = warp_sum(s);
     if (lane == 0) { nu[j] = sqrt(s); nd[j] = nu[j]; }
   }
   __syncthreads();
   double maxnorm = 0.0;
-  for (int j = 0; j < n; ++j) maxnorm = fmax(maxnorm, nu[j]);
+  for (int j = lane; j < n; j += 32) maxnorm = fmax(maxnorm, nu[j]);
+  for (int o = 16; o > 0; o >>= 1) maxnorm = fmax(maxnorm, __shfl_xor_sync(full, maxnorm, o));
   const double eps = rl<typename cplx<C>::R>::eps;  // the precision of the data
   const double thr_helper = m > 0 ? (maxnorm * eps) * (maxnorm * eps) / m : 0.0;
   const double downdate_thr = sqrt(eps);
   int nzp = size;
   double maxpivot = 0.0;
   for (int k = 0; k < size; ++k) {
-    // pivot: first largest updated norm among columns k..n-1
-    double bv = -1.0; int bi = -1;
-    for (int j = k + tid; j < n; j += kT) {
-      double v = nu[j];
-      if (bi < 0 || v > bv) { bv = v; bi = j; }
+    // 1. the largest updated norm among columns k..n-1; norms within kPivotTie of it
+    // count as tied: first index wins.  Norms are not negative: their bits order as
+    // their values do.
+    unsigned hi = 0, lo = 0;
+    for (int j = k + lane; j < n; j += 32) {
+      const double v = nu[j];
+      const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+      if (h > hi || (h == hi && l > lo)) { hi = h; lo = l; }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      double ov = __shfl_down_sync(0xffffffffu, bv, o);
-      int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (oi >= 0 && (bi < 0 || ov > bv || (ov == bv && oi < bi))) { bv = ov; bi = oi; }
+    const unsigned mh = __reduce_max_sync(full, hi);
+    const unsigned ml = __reduce_max_sync(full, hi == mh ? lo : 0u);
+    const double cut = __hiloint2double((int)mh, (int)ml) * (1.0 - kPivotTie);
+    unsigned first = (unsigned)n;
+    for (int j = k + lane; j < n; j += 32)
+      if (nu[j] >= cut) { first = (unsigned)j; break; }
+    first = __reduce_min_sync(full, first);
+    const int big = first < (unsigned)n ? (int)first : k;
+    const double nub = nu[big];
+    if (nzp == size && nub * nub < thr_helper * (double)(m - k)) nzp = k;
+    // 2. columns k and big change places
+    C* const ck = A + (size_t)k * lda;
+    C* const v = staged ? sv : ck;
+    for (int i = tid; i < m; i += kQrT) {
+      C* const cb = A + (size_t)big * lda;
+      const C y = cb[i];
+      if (big != k) { cb[i] = ck[i]; ck[i] = y; }
+      if (staged) v[i] = y;
     }
-    if (lane == 0) { sv[w] = bv; si[w] = bi; }
     __syncthreads();
-    if (tid == 0) {
-      double v = sv[0]; int i = si[0];
-      for (int q = 1; q < kW; ++q)
-        if (si[q] >= 0 && (i < 0 || sv[q] > v || (sv[q] == v && si[q] < i))) { v = sv[q]; i = si[q]; }
-      // norms within kPivotTie of the largest count as tied: first index wins
-      const double cut = v * (1.0 - kPivotTie);
-      for (int j = k; j < n; ++j)
-        if (nu[j] >= cut) { i = j; break; }
-      s_big = i;
+    if (tid == 0 && big != k) {
+      double t = nu[k]; nu[k] = nu[big]; nu[big] = t;
+      t = nd[k]; nd[k] = nd[big]; nd[big] = t;
+      int p = perm[k]; perm[k] = perm[big]; perm[big] = p;
     }
+    // 3. reflector for A(k:m, k)
+    if (w < kQrSumW) {
+      double tail = 0.0;
+      for (int i = k + 1 + tid; i < m; i += 32 * kQrSumW) tail += cabs2_p(v[i]);
+      tail = warp_sum(tail);
+      if (lane == 0) sh[w] = tail;
+    }
+    const double2 c0 = c2d(v[k]);
     __syncthreads();
-    const int big = s_big;
-    if (nzp == size && nu[big] * nu[big] < thr_helper * (double)(m - k)) nzp = k;
-    if (big != k) {
-      for (int i = tid; i < m; i += kT) {
-        C t = A[i + (size_t)k * lda];
-        A[i + (size_t)k * lda] = A[i + (size_t)big * lda];
-        A[i + (size_t)big * lda] = t;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double t = nu[k]; nu[k] = nu[big]; nu[big] = t;
-        t = nd[k]; nd[k] = nd[big]; nd[big] = t;
-        int p = perm[k]; perm[k] = perm[big]; perm[big] = p;
-      }
-    }
-    // reflector for A(k:m, k)
     double tail = 0.0;
-    for (int i = k + 1 + tid; i < m; i += kT) tail += cabs2d(A[i + (size_t)k * lda]);
-    tail = block_sum(tail, sh);
-    const double2 c0 = c2d(A[k + (size_t)k * lda]);
+#pragma unroll
+    for (int q = 0; q < kQrSumW; ++q) tail += sh[q];
     double beta;
     if (tail <= DBL_MIN && c0.y * c0.y <= DBL_MIN) {
       beta = c0.x;
-      if (tid == 0) { s_tau = cplx<C>::mk(0.0, 0.0); }
-      for (int i = k + 1 + tid; i < m; i += kT) A[i + (size_t)k * lda] = cplx<C>::mk(0.0, 0.0);
+      if (tid == 0) s_tau = cplx<C>::mk(0.0, 0.0);
+      for (int i = k + 1 + tid; i < m; i += kQrT) {
+        ck[i] = cplx<C>::mk(0.0, 0.0);
+        if (staged) v[i] = cplx<C>::mk(0.0, 0.0);
+      }
     } else {
-      beta = sqrt(cabs2(c0) + tail);
+      beta = sqrt(cabs2_p(c0) + tail);
       if (c0.x >= 0.0) beta = -beta;
       const double2 den = make_double2(c0.x - beta, c0.y);
-      if (tid == 0) {
-        s_tau = cplx<C>::from(cconj(cdiv(make_double2(beta - c0.x, -c0.y), make_double2(beta, 0.0))));
+      if (w == kQrW - 1) {
+        const C t = cplx<C>::from(cconj(cdiv(make_double2(beta - c0.x, -c0.y), make_double2(beta, 0.0))));
+        if (lane == 0) s_tau = t;
       }
-      for (int i = k + 1 + tid; i < m; i += kT)
-        A[i + (size_t)k * lda] = cplx<C>::from(cdiv(c2d(A[i + (size_t)k * lda]), den));
+      for (int i = k + 1 + tid; i < m; i += kQrT) {
+        const C y = cplx<C>::from(cdiv(c2d(v[i]), den));
+        ck[i] = y;
+        if (staged) v[i] = y;
+      }
     }
     __syncthreads();
     const C t = s_tau;
-    if (tid == 0) { A[k + (size_t)k * lda] = cplx<C>::mk(beta, 0.0); tau[k] = t; }
+    if (tid == 0) { ck[k] = cplx<C>::mk(beta, 0.0); tau[k] = t; }
     maxpivot = fmax(maxpivot, fabs(beta));
-    // apply G = I - t v v^H to columns k+1.. (one warp per column), then downdate norms
-    for (int j = k + 1 + w; j < n; j += kW) {
-      C* col = A + (size_t)j * lda;
-      const C* v = A + (size_t)k * lda;
-      C s = cplx<C>::mk(0.0, 0.0);
-      for (int i = k + 1 + lane; i < m; i += 32) s = cfmac(v[i], col[i], s);
-      s = warp_sum2(s);
-      const C wv = cadd(col[k], s);
-      const C tw = cmul(t, wv);
-      for (int i = k + 1 + lane; i < m; i += 32) col[i] = csub(col[i], cmul(cmul(t, v[i]), wv));
+    // 4. G = I - t v v^H on columns k+1.., then their norms
+    for (int j = k + 1 + w; j < n; j += 2 * kQrW) {
+      const bool two = j + kQrW < n;
+      C* const col[2] = {A + (size_t)j * lda, A + (size_t)(two ? j + kQrW : j) * lda};
+      C s[2] = {cplx<C>::mk(0.0, 0.0), cplx<C>::mk(0.0, 0.0)}, wv[2];
+      for (int i = k + 1 + lane; i < m; i += 32) {
+        const C y = v[i];
+        s[0] = cfmac(y, col[0][i], s[0]);
+        s[1] = cfmac(y, col[1][i], s[1]);
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          s[q].x += __shfl_xor_sync(full, s[q].x, o);
+          s[q].y += __shfl_xor_sync(full, s[q].y, o);
+        }
+      }
+      C rkj[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const C akj = col[q][k];
+        wv[q] = cadd(akj, s[q]);
+        rkj[q] = csub(akj, cmul_t(t, wv[q]));
+      }
       __syncwarp();
-      if (lane == 0) col[k] = csub(col[k], tw);
-      __syncwarp();
-      // LAWN 176 downdate
-      double upd = nu[j];
-      if (upd != 0.0) {
-        const double2 rkj = c2d(col[k]);
-        double tmp = hypot(rkj.x, rkj.y) / upd;
-        tmp = (1.0 + tmp) * (1.0 - tmp);
-        if (tmp < 0.0) tmp = 0.0;
-        double rr = upd / nd[j];
-        double tmp2 = tmp * rr * rr;
-        if (tmp2 <= downdate_thr) {
-          double ss = 0.0;
-          for (int i = k + 1 + lane; i < m; i += 32) ss += cabs2d(col[i]);
-          ss = warp_sum(ss);
-          if (lane == 0) { nd[j] = sqrt(ss); nu[j] = nd[j]; }
-        } else if (lane == 0) {
-          nu[j] = upd * sqrt(tmp);
+      for (int i = k + 1 + lane; i < m; i += 32) {
+        const C tv = cmul_t(t, v[i]);
+        col[0][i] = csub(col[0][i], cmul_p(tv, wv[0]));
+        if (two) col[1][i] = csub(col[1][i], cmul_p(tv, wv[1]));
+      }
+      if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (q == 1 && !two) break;
+          col[q][k] = rkj[q];
+          if (staged) row[j + q * kQrW] = rkj[q];
         }
       }
     }
     __syncthreads();
+    // 5. LAWN 176 downdate of the norms, a thread a column; -1 marks those to be summed anew
+    int again = 0;
+    for (int j = k + 1 + tid; j < n; j += kQrT) {
+      const double upd = nu[j];
+      if (upd != 0.0) {
+        const double2 r = c2d(staged ? row[j] : A[k + (size_t)j * lda]);
+        double tmp = hypot(r.x, r.y) / upd;
+        tmp = (1.0 + tmp) * (1.0 - tmp);
+        if (tmp < 0.0) tmp = 0.0;
+        const double rr = upd / nd[j];
+        const double tmp2 = tmp * rr * rr;
+        if (tmp2 <= downdate_thr) {
+          nd[j] = -1.0;
+          again = 1;
+        } else {
+          nu[j] = upd * sqrt(tmp);
+        }
+      }
+    }
+    if (__syncthreads_or(again)) {
+      for (int j = k + 1 + w; j < n; j += kQrW) {
+        if (nd[j] >= 0.0) continue;
+        double ss = 0.0;
+        for (int i = k + 1 + lane; i < m; i += 32) ss += cabs2_p(A[i + (size_t)j * lda]);
+        ss = sqrt(warp_sum(ss));
+        __syncwarp();
+        if (lane == 0) nu[j] = nd[j] = ss;
+      }
+      __syncthreads();
+    }
   }
+  const double thr = J.thr > 0.0 ? J.thr : (double)size * eps;
+  const double pre = fabs(maxpivot) * thr;
+  int rk = 0;
+  for (int i = tid; i < nzp; i += kQrT) rk += (cabsd(A[i + (size_t)i * lda]) > pre);
+  rk = __reduce_add_sync(full, rk);
+  if (lane == 0 && rk) atomicAdd(&s_rank, rk);
+  __syncthreads();
   if (tid == 0) {
-    const double thr = J.thr > 0.0 ? J.thr : (double)size * eps;
-    const double pre = fabs(maxpivot) * thr;
-    int rk = 0;
-    for (int i = 0; i < nzp; ++i) rk += (cabsd(A[i + (size_t)i * lda]) > pre);
     J.info[0] = nzp;
-    J.info[1] = rk;
+    J.info[1] = s_rank;
     if (J.maxpiv) J.maxpiv[0] = maxpivot;
   }
-}
-
-template <typename C>
-__global__ void __launch_bounds__(kT) qr_factor_kernel(const QRJob* __restrict__ jobs) {
-  const QRJob J = jobs[blockIdx.x];
-  qr_factor_body<C>(J, static_cast<C*>(J.a), J.lda, J.norms, J.norms + J.n, J.perm);
 }
 
 // ---------------------------------------------------------------- QR solve
@@ -827,11 +896,20 @@ __global__ void __launch_bounds__(kT) skel_lu_kernel(const SkelLUJob* __restrict
 
 }  // namespace
 
-int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int es, cudaStream_t s) {
+int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int mmax, int nmax, int es, cudaStream_t s) {
   if (njobs <= 0) return 0;
   if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  if (es == 16) qr_factor_kernel<double2><<<njobs, kT, 0, s>>>(d_jobs);
-  else qr_factor_kernel<float2><<<njobs, kT, 0, s>>>(d_jobs);
+  // reflector and norms in shared memory; in global memory where a block is too large
+  size_t smem = (size_t)es * (((mmax + 1) & ~1) + (size_t)nmax) + 2 * sizeof(double) * (size_t)nmax;
+  if (smem > size_t(200) << 10) smem = mmax = nmax = 0;
+  static bool attr[2] = {false, false};
+  if (es == 16) {
+    smem_attr_once(qr_factor_kernel<double2>, attr[0]);
+    qr_factor_kernel<double2><<<njobs, kQrT, smem, s>>>(d_jobs, mmax, nmax);
+  } else {
+    smem_attr_once(qr_factor_kernel<float2>, attr[1]);
+    qr_factor_kernel<float2><<<njobs, kQrT, smem, s>>>(d_jobs, mmax, nmax);
+  }
   return (int)cudaGetLastError();
 }
 

@@ -738,12 +738,19 @@ struct aifmm_problem {
     struct Group { std::vector<QRJob> jobs; int n = 0; size_t smem = 0; double fl = 0; };
     std::map<int, Group> groups;
     std::vector<QRJob> large;
+    int m_large = 0, n_large = 0;
     double fl_large = 0;
     const int es = qr_es;
     for (auto& j : qj) {
       const int cls = aifmm_qr_class(j.m, j.n);
       const size_t b = aifmm_qr_smem_bytes(j.m, j.n, es);
-      if (cls < 0 && b > size_t(200) << 10) { large.push_back(j); fl_large += qr_flops(j.m, j.n); continue; }
+      if (cls < 0 && b > size_t(200) << 10) {
+        large.push_back(j);
+        m_large = std::max(m_large, j.m);
+        n_large = std::max(n_large, j.n);
+        fl_large += qr_flops(j.m, j.n);
+        continue;
+      }
       Group& g = groups[cls];
       g.jobs.push_back(j);
       g.n = std::max(g.n, j.n);
@@ -764,7 +771,7 @@ struct aifmm_problem {
       const QRJob* dq = stage.put(large, cur);
       cudaEvent_t a;
       const bool pr = prof_begin(0, a);
-      KL(aifmm_launch_qr_factor(dq, (int)large.size(), es, cur));
+      KL(aifmm_launch_qr_factor(dq, (int)large.size(), m_large, n_large, es, cur));
       if (pr) prof_end(0, a, fl_large);
     }
     qj.clear();
