@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kQrT) qr_factor_kernel(const QRJob* __restrict
 }
 
 // ---------------------------------------------------------------- QR solve
-// one warp per right-hand side column
+// one warp per right-hand side column, the column in global memory: systems of any size
 template <typename C>
 __global__ void __launch_bounds__(kT) qr_solve_kernel(const SolveJob* __restrict__ jobs, const int* __restrict__ col_off,
                                                       int njobs, int total_cols) {
@@ -310,6 +310,103 @@ __global__ void __launch_bounds__(kT) qr_solve_kernel(const SolveJob* __restrict
   __syncwarp();
   const C alpha = cplx<C>::from(J.alpha);
   for (int i = lane; i < nzp; i += 32) x[J.perm[i]] = cmul(alpha, wv[i]);
+}
+
+// The same for up to 32 RPL rows: a column in a warp's registers (row i in lane i mod 32,
+// register i / 32), the factor's next column fetched while the one before it is applied.
+// Eight columns a CTA read the factor together.
+// What bounds it: the chain of a reflector (dot product, its reduction, update) and of a
+// row of the back substitution (division, broadcast, update), 0.6 us each.  One column of
+// 130 rows, rank 120: 230 us with the column in global memory, 142 us here; 32 columns of
+// 200 rows: 498 and 259 us; 300 rows: 878 and 442 us.  Beyond 384 rows (207 registers) the
+// kernel above is the faster one.
+template <typename C, int RPL>
+__global__ void __launch_bounds__(kT) qr_solve_wide_kernel(const SolveJob* __restrict__ jobs,
+                                                           const int* __restrict__ col_off, int njobs, int total_cols) {
+  constexpr unsigned full = 0xffffffffu;
+  const int gw = blockIdx.x * kW + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (gw >= total_cols) return;
+  int lo = 0, hi = njobs - 1;
+  while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (col_off[mid] <= gw) lo = mid; else hi = mid - 1; }
+  const SolveJob J = jobs[lo];
+  const C* Jqr = static_cast<const C*>(J.qr);
+  const C* Jtau = static_cast<const C*>(J.tau);
+  const C* JB = static_cast<const C*>(J.B);
+  const int c = gw - col_off[lo];
+  const int m = J.m, n = J.n;
+  const int nzp = J.info[0];
+  C* x = static_cast<C*>(J.X) + (size_t)c * J.ldx;
+  if (nzp == 0) {
+    for (int i = lane; i < n; i += 32) x[i] = cplx<C>::mk(0.0, 0.0);
+    return;
+  }
+  const C zero = cplx<C>::mk(0.0, 0.0);
+  C wv[RPL], nx[RPL];
+#pragma unroll
+  for (int q = 0; q < RPL; ++q) {
+    const int i = lane + 32 * q;
+    wv[q] = i >= m ? zero : JB ? JB[i + (size_t)c * J.ldb] : cplx<C>::mk(i == c ? 1.0 : 0.0, 0.0);
+  }
+  auto fetch = [&](int k) {
+    const C* v = Jqr + (size_t)k * J.ldq;
+#pragma unroll
+    for (int q = 0; q < RPL; ++q) nx[q] = lane + 32 * q < m ? v[lane + 32 * q] : zero;
+  };
+  auto from_lane = [&](C a, int l) { return C{__shfl_sync(full, a.x, l), __shfl_sync(full, a.y, l)}; };
+  // Q^H b with the first nzp reflectors
+  fetch(0);
+  C tn = Jtau[0];
+#pragma unroll
+  for (int Q = 0; Q < RPL; ++Q) {
+    for (int kk = 0; kk < 32; ++kk) {
+      const int k = 32 * Q + kk;
+      if (k >= nzp) break;
+      C v[RPL];
+#pragma unroll
+      for (int q = Q; q < RPL; ++q) v[q] = nx[q];
+      const C t = tn;
+      if (k + 1 < nzp) { fetch(k + 1); tn = Jtau[k + 1]; }
+      C s = zero;
+#pragma unroll
+      for (int q = Q; q < RPL; ++q) {
+        const int i = lane + 32 * q;
+        if (i > k && i < m) s = cfmac(v[q], wv[q], s);
+      }
+      s = warp_sum2(s);
+      const C w = cadd(from_lane(wv[Q], kk), s);
+#pragma unroll
+      for (int q = Q; q < RPL; ++q) {
+        const int i = lane + 32 * q;
+        if (i > k && i < m) wv[q] = csub(wv[q], cmul_p(cmul_t(t, v[q]), w));
+      }
+      if (lane == kk) wv[Q] = csub(wv[Q], cmul_t(t, w));
+    }
+  }
+  // back substitution with R(0:nzp, 0:nzp), column oriented
+  fetch(nzp - 1);
+#pragma unroll
+  for (int Q = RPL - 1; Q >= 0; --Q) {
+    for (int kk = 31; kk >= 0; --kk) {
+      const int i = 32 * Q + kk;
+      if (i >= nzp) continue;
+      C r[RPL];
+#pragma unroll
+      for (int q = 0; q <= Q; ++q) r[q] = nx[q];
+      if (i > 0) fetch(i - 1);
+      const C xi = cplx<C>::from(cdiv(c2d(from_lane(wv[Q], kk)), c2d(from_lane(r[Q], kk))));
+#pragma unroll
+      for (int q = 0; q <= Q; ++q)
+        if (lane + 32 * q < i) wv[q] = csub(wv[q], cmul_p(r[q], xi));
+      if (lane == kk) wv[Q] = xi;
+    }
+  }
+  for (int i = lane; i < n; i += 32) x[i] = zero;
+  __syncwarp();
+  const C alpha = cplx<C>::from(J.alpha);
+#pragma unroll
+  for (int q = 0; q < RPL; ++q)
+    if (lane + 32 * q < nzp) x[J.perm[lane + 32 * q]] = cmul_p(alpha, wv[q]);
 }
 
 // ---------------------------------------------------------------- form Q
@@ -944,15 +1041,24 @@ int aifmm_launch_qr_solve_reg(const SolveBatch& g, int es, cudaStream_t s) {
   return es == 16 ? launch_solve_reg<double2>(g, smem, s) : launch_solve_reg<float2>(g, smem, s);
 }
 
-int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,
+int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int mmax, int es,
                           cudaStream_t s) {
   if (njobs <= 0 || total_cols <= 0) return 0;
   if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  const int grid = (total_cols + kW - 1) / kW;
-  if (es == 16) qr_solve_kernel<double2><<<grid, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
-  else qr_solve_kernel<float2><<<grid, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
+  const int blocks = (total_cols + kW - 1) / kW;
+#define AIFMM_SOLVE_WIDE(R)                                                                                     \
+  if (mmax <= 32 * R) {                                                                                         \
+    if (es == 16) qr_solve_wide_kernel<double2, R><<<blocks, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols); \
+    else qr_solve_wide_kernel<float2, R><<<blocks, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);           \
+    return (int)cudaGetLastError();                                                                             \
+  }
+  AIFMM_SOLVE_WIDE(4) AIFMM_SOLVE_WIDE(8) AIFMM_SOLVE_WIDE(12)
+#undef AIFMM_SOLVE_WIDE
+  if (es == 16) qr_solve_kernel<double2><<<blocks, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
+  else qr_solve_kernel<float2><<<blocks, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
   return (int)cudaGetLastError();
 }
+
 int aifmm_launch_formq(const FormQJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,
                        cudaStream_t s) {
   if (njobs <= 0 || total_cols <= 0) return 0;

@@ -148,7 +148,7 @@ int aifmm_launch_green_matvec_add(const double2* x, double2* y, int N, int nrhs,
                                   cudaStream_t stream);
 int aifmm_launch_aca(const AcaJob* d_jobs, int njobs, double tol, const EntryCtx& ctx, cudaStream_t stream);
 int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int mmax, int nmax, int es, cudaStream_t s);
-int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int es,
+int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int mmax, int es,
                           cudaStream_t s);
 size_t aifmm_qr_smem_bytes(int m, int n, int es);
 // eight lanes per right-hand side, the column in registers; m <= 224 and the factor's

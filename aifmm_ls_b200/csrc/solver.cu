@@ -797,7 +797,7 @@ struct aifmm_problem {
   void flush_solve() {
     if (sj.empty()) return;
     // m <= 224 whose factor fits in shared memory: the columns in registers; larger
-    // systems (the base level): the global-memory kernel
+    // systems (the base level, the widest mosaics): the factor stays in global memory
     std::vector<SolveJob> small, large;
     int mmax = 1, nmax = 1;
     const int es = solve_es;
@@ -850,10 +850,11 @@ struct aifmm_problem {
     }
     if (!large.empty()) {
       std::vector<int> off(large.size());
-      int tot = 0;
+      int tot = 0, mlarge = 0;
       for (size_t i = 0; i < large.size(); ++i) {
         off[i] = tot;
         tot += large[i].nrhs;
+        mlarge = std::max(mlarge, large[i].m);
         large[i].work = scratch.get((size_t)es * large[i].m * large[i].nrhs);
       }
       auto ptrs = put_many_({{large.data(), large.size() * sizeof(SolveJob)}, {off.data(), off.size() * sizeof(int)}});
@@ -865,7 +866,7 @@ struct aifmm_problem {
         const SolveJob* d0 = static_cast<const SolveJob*>(ptrs[0]);
         const int* d1 = static_cast<const int*>(ptrs[1]);
         const int nj = (int)large.size();
-        KL(run_op([=](cudaStream_t s_) { return aifmm_launch_qr_solve(d0, d1, nj, tot, es, s_); }));
+        KL(run_op([=](cudaStream_t s_) { return aifmm_launch_qr_solve(d0, d1, nj, tot, mlarge, es, s_); }));
       }
       if (pr) prof_end(1, a, fl);
     }
