@@ -23,8 +23,6 @@ struct AcaJob {
   double2* U;        // rmax x n_prim
   double2* V;        // rmax x n_sec
   double2* P;        // n_sec
-  double2* S;        // n_prim
-  double2* coef;     // rmax + 1
   double2* dots_u;   // rmax + 1
   double2* dots_v;   // rmax + 1
   unsigned char* remP;

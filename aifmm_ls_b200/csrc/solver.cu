@@ -1231,7 +1231,7 @@ struct aifmm_problem {
       auto job_bytes = [&](int t, size_t& wsb, size_t& acb) {
         const int n1 = ji[t].n1, n2 = ji[t].n2, rmax = std::min(n1, n2);
         const int np = n1 < n2 ? n1 : n2, ns = n1 < n2 ? n2 : n1;
-        const size_t b = sizeof(double2) * ((size_t)rmax * np + (size_t)rmax * ns + ns + np + 3 * (size_t)rmax + 3) + np + ns + 16;
+        const size_t b = sizeof(double2) * ((size_t)rmax * np + (size_t)rmax * ns + ns + 2 * (size_t)rmax + 2) + np + ns + 16;
         wsb = (b + 255) & ~size_t(255);
         acb = (sizeof(double2) * (size_t)rmax * ((t % 2) == 0 ? n2 : n1) + 255) & ~size_t(255);
       };
@@ -1280,8 +1280,6 @@ struct aifmm_problem {
           J.U = reinterpret_cast<double2*>(base); base += sizeof(double2) * (size_t)rmax * np;
           J.V = reinterpret_cast<double2*>(base); base += sizeof(double2) * (size_t)rmax * ns;
           J.P = reinterpret_cast<double2*>(base); base += sizeof(double2) * ns;
-          J.S = reinterpret_cast<double2*>(base); base += sizeof(double2) * np;
-          J.coef = reinterpret_cast<double2*>(base); base += sizeof(double2) * (rmax + 1);
           J.dots_u = reinterpret_cast<double2*>(base); base += sizeof(double2) * (rmax + 1);
           J.dots_v = reinterpret_cast<double2*>(base); base += sizeof(double2) * (rmax + 1);
           J.remP = reinterpret_cast<unsigned char*>(base); base += np;
