@@ -49,7 +49,7 @@ __global__ void list_entries_kernel(const int* __restrict__ I, const int* __rest
 // What bounds it: latency and issue of the FP64 recurrences (about 1,900 double
 // instructions per target, leaf and one right-hand side; the moments are warp-
 // uniform reads of shared memory).  36,864 unknowns, one right-hand side, through
-// dense_matvec with host buffers: 958 ms with a series per entry, 10.3 ms with a
+// dense_matvec with host buffers: 958 ms with a series per entry, 5.6 ms with a
 // series per leaf; 2,304 unknowns: 4.4 ms and 0.14 ms; 256 unknowns: 99 us and 66 us.
 constexpr int kMvRows = 128;
 constexpr int kMvMaxRhs = 8;
