@@ -431,6 +431,13 @@ __device__ void qr_smem_body(const QRJob& J, C* qsm) {
       }
     }
     key = __reduce_min_sync(full, key);
+    if (key == 0xffffffffu) {  // norms that are not numbers: no swap, as in qr_reg_phase
+      for (int q = 0; q < nscan; ++q) {
+        const int s = lane + 32 * q;
+        if (s < n && spos[s] >= k) key = min(key, (unsigned)spos[s] * 1024u + (unsigned)s);
+      }
+      key = __reduce_min_sync(full, key);
+    }
     const int big = (int)(key >> 10), bslot = (int)(key & 1023u);
     const double nub = snu[bslot];
     if (nzp == size && nub * nub < thr_helper * (double)(m - k)) nzp = k;
