@@ -1030,6 +1030,24 @@ struct aifmm_problem {
     if (ev_join) cudaEventDestroy(ev_join);
   }
 
+  // After a call that failed, by whatever stage it left: nothing of it is still running,
+  // queued or recorded, and what it held goes back.  Later calls count on that: their
+  // first launch flushes the pending batches of `cur`, and they take the freed blocks.
+  void recover() {
+    if (st) cudaStreamSynchronize(st);
+    if (st2) cudaStreamSynchronize(st2);
+    cudaGetLastError();  // a failed allocation's status, which the next launch would report as its own
+    cur = st;
+    gd.clear(); gt.clear(); ged.clear(); sj.clear(); qj.clear(); fq.clear(); ndv.clear();
+    recording = false;
+    rec_ops.clear();
+    rec_host.clear();
+    for (auto& b : rec_dev) pool.defer_free(b.first, b.second);
+    rec_dev.clear();
+    scratch.reset();
+    pool.commit_frees();
+  }
+
   // what the entries take from the far-field coefficients: the sources of an order next to
   // each other, and a bound (entry.cuh)
   void transpose_M() {
@@ -1152,6 +1170,7 @@ struct aifmm_problem {
     es_ = 16;
     if (!tables_ready) throw Fail(AIFMM_ERR_STATE, "tables not computed or set");
     if (!tree_ready) throw Fail(AIFMM_ERR_STATE, "tree not built");
+    assembled = false;  // until it is complete
     auto t0 = std::chrono::steady_clock::now();
     const long l0 = launches_;
     const EntryCtx cx = ctx();
@@ -2948,7 +2967,7 @@ struct aifmm_problem {
     try {
       solve_core(nr, pl.bin, N, pl.xout, N);
     } catch (...) {
-      recording = false;
+      for (auto& o : pl.owned) pool.defer_free(o.first, o.second);
       throw;
     }
     recording = false;
@@ -3490,10 +3509,10 @@ aifmm_status guard(aifmm_problem* p, F&& f) {
     if (p) p->err.clear();
     return AIFMM_OK;
   } catch (const Fail& e) {
-    if (p) p->err = e.what();
+    if (p) { p->err = e.what(); p->recover(); }
     return e.st;
   } catch (const std::exception& e) {
-    if (p) p->err = e.what();
+    if (p) { p->err = e.what(); p->recover(); }
     return AIFMM_ERR_NUMERIC;
   }
 }
@@ -3605,7 +3624,7 @@ aifmm_status aifmm_entries(aifmm_problem* p, long n, const int* I, const int* J,
     if (!dev)
       for (long t = 0; t < n; ++t)
         if (I[t] < 0 || I[t] >= p->N || J[t] < 0 || J[t] >= p->N) throw Fail(AIFMM_ERR_ARG, "point index out of range");
-    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised, also one that fails (recover)
     aifmm_problem::Tmp tI(p, dev ? 1 : sizeof(int) * n), tJ(p, dev ? 1 : sizeof(int) * n);
     aifmm_problem::Tmp tO(p, dev ? 1 : sizeof(double2) * n);
     if (!dev) {
@@ -3634,7 +3653,7 @@ aifmm_status aifmm_get_matrix(aifmm_problem* p, int nr, const int* rows, int nc,
         if (cols[c] < 0 || cols[c] >= p->N) throw Fail(AIFMM_ERR_ARG, "point index out of range");
     }
     // host memory: the index lists travel and the block comes back
-    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised, also one that fails (recover)
     const size_t bytes = sizeof(double2) * (size_t)nr * nc;
     aifmm_problem::Tmp tr(p, dev ? 1 : sizeof(int) * (size_t)nr), tc(p, dev ? 1 : sizeof(int) * (size_t)nc);
     aifmm_problem::Tmp to(p, dev ? 1 : bytes);
@@ -3867,7 +3886,7 @@ aifmm_status aifmm_dense_matvec(aifmm_problem* p, int nrhs, const double* x, dou
   if (!p || !x || !y || nrhs < 1 || nrhs > 8) return AIFMM_ERR_ARG;
   if (!p->tables_ready) { p->err = "tables not ready"; return AIFMM_ERR_STATE; }
   return guard(p, [&] {
-    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised, also one that fails (recover)
     const size_t bytes = sizeof(double2) * (size_t)p->N * nrhs;
     const bool dev = flags & AIFMM_PTR_DEVICE;
     const double2* dx = reinterpret_cast<const double2*>(x);
@@ -3890,7 +3909,7 @@ aifmm_status aifmm_total_field(aifmm_problem* p, int nrhs, const double* theta, 
   if (!p || !theta || !phi || !u || nrhs < 1 || nrhs > 8) return AIFMM_ERR_ARG;
   if (!p->tables_ready) { p->err = "tables not ready"; return AIFMM_ERR_STATE; }
   return guard(p, [&] {
-    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised
+    p->pool.commit_frees();  // the previous call's buffers: every call ends synchronised, also one that fails (recover)
     const size_t bytes = sizeof(double2) * (size_t)p->N * nrhs;
     const bool dev = flags & AIFMM_PTR_DEVICE;
     const double2* dphi = reinterpret_cast<const double2*>(phi);
