@@ -369,8 +369,8 @@ __global__ void __launch_bounds__(qr_threads(RPL)) compress_reg_kernel(const Com
 template <typename C, int RPL>
 int launch_compress_reg(const CompressJob* d_jobs, const CompressJob* h_jobs, int njobs, int n, size_t smem,
                         cudaStream_t s) {
-  static bool attr = false;
-  smem_attr_once(compress_reg_kernel<C, RPL>, attr);
+  static SmemLimit attr;
+  if (const int e = smem_limit(compress_reg_kernel<C, RPL>, attr)) return e;
   CompressInline inl;
   if (!d_jobs) memcpy(inl.b, h_jobs, sizeof(CompressJob) * njobs);
   return launch_chain(compress_reg_kernel<C, RPL>, dim3(njobs), threads_for(n), smem, s, d_jobs, inl);
@@ -388,12 +388,12 @@ size_t aifmm_compress_smem_bytes(int m, int rK, int c, int rb, int es) {
 int aifmm_launch_compress_p2p(const CompressJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s) {
   if (njobs <= 0) return 0;
   if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  static bool attr[2] = {false, false};
+  static SmemLimit attr[2];
   if (es == 16) {
-    smem_attr_once(compress_p2p_kernel<double2>, attr[0]);
+    if (const int e = smem_limit(compress_p2p_kernel<double2>, attr[0])) return e;
     compress_p2p_kernel<double2><<<njobs, kT, smem, s>>>(d_jobs);
   } else {
-    smem_attr_once(compress_p2p_kernel<float2>, attr[1]);
+    if (const int e = smem_limit(compress_p2p_kernel<float2>, attr[1])) return e;
     compress_p2p_kernel<float2><<<njobs, kT, smem, s>>>(d_jobs);
   }
   return (int)cudaGetLastError();

@@ -999,12 +999,12 @@ int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int mmax, int nmax, i
   // reflector and norms in shared memory; in global memory where a block is too large
   size_t smem = (size_t)es * (((mmax + 1) & ~1) + (size_t)nmax) + 2 * sizeof(double) * (size_t)nmax;
   if (smem > size_t(200) << 10) smem = mmax = nmax = 0;
-  static bool attr[2] = {false, false};
+  static SmemLimit attr[2];
   if (es == 16) {
-    smem_attr_once(qr_factor_kernel<double2>, attr[0]);
+    if (const int e = smem_limit(qr_factor_kernel<double2>, attr[0])) return e;
     qr_factor_kernel<double2><<<njobs, kQrT, smem, s>>>(d_jobs, mmax, nmax);
   } else {
-    smem_attr_once(qr_factor_kernel<float2>, attr[1]);
+    if (const int e = smem_limit(qr_factor_kernel<float2>, attr[1])) return e;
     qr_factor_kernel<float2><<<njobs, kQrT, smem, s>>>(d_jobs, mmax, nmax);
   }
   return (int)cudaGetLastError();
@@ -1013,7 +1013,7 @@ int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int mmax, int nmax, i
 namespace {
 template <typename C>
 int launch_solve_reg(const SolveBatch& g, size_t smem, cudaStream_t s) {
-  static bool attr[6] = {false, false, false, false, false, false};
+  static SmemLimit attr[6];
   SolveInline inl;
   dim3 grid(g.nctas);
   if (!g.d) {
@@ -1022,7 +1022,7 @@ int launch_solve_reg(const SolveBatch& g, size_t smem, cudaStream_t s) {
   }
 #define AIFMM_SOLVE_CASE(I, R)                                                                                       \
   if (g.mmax <= 8 * R) {                                                                                             \
-    smem_attr_once(qr_solve_reg_kernel<C, R>, attr[I]);                                                              \
+    if (const int e = smem_limit(qr_solve_reg_kernel<C, R>, attr[I])) return e;                                      \
     return launch_chain(qr_solve_reg_kernel<C, R>, grid, kSolveT, smem, s, g.d, g.ctas, (int)g.early, inl);          \
   }
   AIFMM_SOLVE_CASE(0, 3) AIFMM_SOLVE_CASE(1, 5) AIFMM_SOLVE_CASE(2, 8) AIFMM_SOLVE_CASE(3, 12)
@@ -1071,8 +1071,8 @@ int aifmm_launch_formq(const FormQJob* d_jobs, const int* d_col_off, int njobs, 
 namespace {
 template <typename C, int WM, int WN, int NS>
 int launch_gemm_ns(const GemmBatch& g, int tk, cudaStream_t s) {
-  static bool attr = false;
-  smem_attr_once(gemm_kernel<C, WM, WN, NS>, attr);
+  static SmemLimit attr;
+  if (const int e = smem_limit(gemm_kernel<C, WM, WN, NS>, attr)) return e;
   const size_t smem = sizeof(C) * NS * (size_t)(gemm_area(8 * WM, tk) + gemm_area(8 * WN, tk));
   GemmInline<NS> inl;
   dim3 grid(g.ntiles);

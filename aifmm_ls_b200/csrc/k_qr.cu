@@ -29,8 +29,8 @@ __global__ void __launch_bounds__(kT) qr_factor_smem_kernel(const QRJob* __restr
 
 template <typename C, int RPL>
 int launch_qr_reg(const QRJob* d_jobs, const QRJob* h_jobs, int njobs, int n, size_t smem, cudaStream_t s) {
-  static bool attr = false;
-  smem_attr_once(qr_factor_reg_kernel<C, RPL>, attr);
+  static SmemLimit attr;
+  if (const int e = smem_limit(qr_factor_reg_kernel<C, RPL>, attr)) return e;
   QrInline inl;
   if (!d_jobs) memcpy(inl.b, h_jobs, sizeof(QRJob) * njobs);
   return launch_chain(qr_factor_reg_kernel<C, RPL>, dim3(njobs), threads_for(n), smem, s, d_jobs, inl);
@@ -64,12 +64,12 @@ size_t aifmm_qr_smem_bytes(int m, int n, int es) {
 int aifmm_launch_qr_factor_smem(const QRJob* d_jobs, int njobs, size_t smem, int es, cudaStream_t s) {
   if (njobs <= 0) return 0;
   if (!valid_es(es)) return (int)cudaErrorInvalidValue;
-  static bool attr[2] = {false, false};
+  static SmemLimit attr[2];
   if (es == 16) {
-    smem_attr_once(qr_factor_smem_kernel<double2>, attr[0]);
+    if (const int e = smem_limit(qr_factor_smem_kernel<double2>, attr[0])) return e;
     qr_factor_smem_kernel<double2><<<njobs, kT, smem, s>>>(d_jobs);
   } else {
-    smem_attr_once(qr_factor_smem_kernel<float2>, attr[1]);
+    if (const int e = smem_limit(qr_factor_smem_kernel<float2>, attr[1])) return e;
     qr_factor_smem_kernel<float2><<<njobs, kT, smem, s>>>(d_jobs);
   }
   return (int)cudaGetLastError();
