@@ -88,15 +88,5 @@ struct Inline {
 
 // the element size of a batch: 16 (complex128) or 8 (complex64)
 inline bool valid_es(int es) { return es == 16 || es == 8; }
-// opt a kernel into the large dynamic shared memory on the current device
-template <typename K>
-int smem_limit(K kernel, SmemLimit& limit) {
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return (int)e;
-  return limit.once(device, [&] {
-    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-  });
-}
 
 }  // namespace

@@ -11,6 +11,7 @@
 //    accepted when |I_parent - sum I_child| < 1e-7, otherwise every child is refined;
 //    the result is the sum of accepted panels' own estimates in depth-first order.
 #include "kernels.h"
+#include "smem_limit.h"
 
 namespace {
 
@@ -508,13 +509,14 @@ int aifmm_launch_tables(int n_cheb, int degree, double kappa, double r, const do
   const double eps = 1e-7;  // LS/FarFieldInteraction.hpp:37, LS/NearFieldInteraction1.hpp:112
   const size_t qs = quad_smem_bytes(P.nb, degree);
   if (P.nb > 64 || qs > 220 * 1024) return (int)cudaErrorInvalidValue;
-  cudaFuncSetAttribute(quad_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qs);
-  cudaFuncSetAttribute(quad_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qs);
+  static SmemLimit attr[3];
+  if (const int e = smem_limit(quad_kernel<true>, attr[0])) return e;
+  if (const int e = smem_limit(quad_kernel<false>, attr[1])) return e;
+  if (const int e = smem_limit(tables_finish_kernel, attr[2])) return e;
   quad_kernel<true><<<121, 32 * kWarps, qs, stream>>>(P, degree, eps);
   quad_kernel<false><<<9 * P.rank, 32 * kWarps, qs, stream>>>(P, degree, eps);
   size_t smem = sizeof(double) * ((size_t)P.rank * P.nb + P.nb * P.nb + P.nb * P.rank);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  cudaFuncSetAttribute(tables_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   tables_finish_kernel<<<1, 256, smem, stream>>>(P, qpinv);
   const int entries = 121 * P.rank + 9 * P.rank * P.rank;
   tables_product_kernel<<<(entries + 127) / 128, 128, 0, stream>>>(P, qpinv, M, nearT);

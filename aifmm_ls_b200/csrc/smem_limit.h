@@ -23,3 +23,18 @@ class SmemLimit {
   static constexpr int kDevices = 64;
   std::atomic<bool> done_[kDevices] = {};
 };
+
+#ifdef __CUDACC__
+namespace {
+// opt a kernel into the large dynamic shared memory on the current device
+template <typename K>
+int smem_limit(K kernel, SmemLimit& limit) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return (int)e;
+  return limit.once(device, [&] {
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  });
+}
+}  // namespace
+#endif
