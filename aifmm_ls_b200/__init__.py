@@ -247,7 +247,8 @@ class LSKernel:
         return C
 
     def dense_matvec(self, x):
-        """y = A x with exact entries (the find_error fixture product); x: (nrhs, N)."""
+        """y = A x without compression (the find_error fixture product); x: (nrhs, N).
+        Far entries below 1e-16, zero in getMatrix, take part."""
         x = np.atleast_2d(np.asarray(x, dtype=np.complex128))
         xi = np.ascontiguousarray(x)
         y = np.zeros_like(xi)

@@ -226,18 +226,25 @@ __device__ __forceinline__ int near_dir(int dx, int dy) {
   return tab[(dy + 1) * 3 + (dx + 1)];
 }
 
+// Entries below it are zero (LS_Assembly.hpp:536-538).
+constexpr double kEntryFloor = 1e-16;
+// Whether every far entry of a row with the contrast qi is below half of `floor`
+__device__ __forceinline__ bool far_is_zero(double qi, const EntryCtx& c, double floor) {
+  return c.kappa * c.kappa * fabs(qi) * __ldg(c.far_bound) < 0.5 * floor;
+}
+
 // PHI = true: the system matrix A (findPhi, LS_Assembly.hpp:506-511, 528-533);
 // PHI = false: the bare integral operator G of the same entry (no kappa^2 q(x_i)
 // factor, no identity), the operator the reference applies to the solution to
 // get the scattered field (hybrid.cpp:263-281).
 // ENX: see far_series (the ACA's entries have always fused the other product).
-// Entries below 1e-16 are zero (LS_Assembly.hpp:536-538); a far entry whose bound
+// Entries below kEntryFloor are zero; a far entry whose bound
 // kappa^2 |q_i| max_j sum_n |M_nj| |H_n| is below half of `floor` is returned as zero
 // without its series.  With the floor of 1e-16 that changes no result: the bound holds
 // for every distance (|H_n| decreases), and half leaves room for the rounding of both.
 // Rows outside the contrast's support cost one load instead of 61 orders.
 template <bool PHI = true, int ENX = 1>
-__device__ __forceinline__ double2 lsa_entry(int i, int j, const EntryCtx& c, double floor = 1e-16) {
+__device__ __forceinline__ double2 lsa_entry(int i, int j, const EntryCtx& c, double floor = kEntryFloor) {
   const int rank = c.rank;
   const int li = i / rank, ii = i - li * rank;
   const int lj = j / rank, jj = j - lj * rank;
@@ -255,10 +262,10 @@ __device__ __forceinline__ double2 lsa_entry(int i, int j, const EntryCtx& c, do
       e.x = e.x * qi; e.y = e.y * qi;
       if (i == j) e.x = 1.0 + e.x;
     }
-    if (hypot(e.x, e.y) < 1e-16) e = make_double2(0.0, 0.0);
+    if (hypot(e.x, e.y) < kEntryFloor) e = make_double2(0.0, 0.0);
     return e;
   }
-  if (PHI && c.kappa * c.kappa * fabs(qi) * __ldg(c.far_bound) < 0.5 * floor) return make_double2(0.0, 0.0);
+  if (PHI && far_is_zero(qi, c, floor)) return make_double2(0.0, 0.0);
   const double2 ri = __ldg(&c.pts[i]);
   const double2 cj = __ldg(&c.leafc[lj]);
   const double ddy = ri.y - cj.y, ddx = ri.x - cj.x;
@@ -272,6 +279,6 @@ __device__ __forceinline__ double2 lsa_entry(int i, int j, const EntryCtx& c, do
     s.x *= kq; s.y *= kq;
     if (i == j) s.x += 1.0;
   }
-  if (hypot(s.x, s.y) < 1e-16) s = make_double2(0.0, 0.0);
+  if (hypot(s.x, s.y) < kEntryFloor) s = make_double2(0.0, 0.0);
   return s;
 }

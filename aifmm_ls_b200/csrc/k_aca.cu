@@ -39,7 +39,6 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCluster = 8;
-constexpr double kEntryFloor = 1e-16;  // entries below it are zero (lsa_entry)
 constexpr int kMag = 4;      // magnitudes a thread keeps in shared memory (the rest: computed twice)
 constexpr int kCoef = 32;   // coefficients of a residual held in shared memory (the rest: global memory)
 typedef unsigned long long u64;

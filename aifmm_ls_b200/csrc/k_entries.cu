@@ -43,13 +43,15 @@ __global__ void list_entries_kernel(const int* __restrict__ I, const int* __rest
 // whose Hankel values and angles depend on the target point and the source LEAF
 // only.  So the sources of a leaf are summed first: m(n, s) = sum_j M(n, j) x(j, s)
 // (moments_kernel), and one series per (target, leaf) replaces one per entry --
-// rank times fewer Bessel recurrences.
+// rank times fewer Bessel recurrences.  Rows whose far entries are all zero by the
+// entries' own bound have no series; in the others the far entries below 1e-16, zero
+// in the matrix, are part of the sum.
 //   sum_n H_n(R) e^{in th} m_n = sum_{n >= 0} (J_n + i Y_n) (p_n cos n th + q_n sin n th)
 //   p_n = m_n + (-1)^n m_{-n},  q_n = i (m_n - (-1)^n m_{-n}),  p_0 = m_0,  q_0 = 0
 // What bounds it: latency and issue of the FP64 recurrences (about 1,900 double
 // instructions per target, leaf and one right-hand side; the moments are warp-
 // uniform reads of shared memory).  36,864 unknowns, one right-hand side, through
-// dense_matvec with host buffers: 958 ms with a series per entry, 5.6 ms with a
+// dense_matvec with host buffers: 958 ms with a series per entry, 3.2 ms with a
 // series per leaf; 2,304 unknowns: 4.4 ms and 0.14 ms; 256 unknowns: 99 us and 66 us.
 constexpr int kMvRows = 128;
 constexpr int kMvMaxRhs = 8;
@@ -205,14 +207,13 @@ __global__ void __launch_bounds__(kMvRows) leaf_matvec_kernel(const double2* __r
   const int i = min((int)(blockIdx.x * kMvRows + threadIdx.x), N - 1);
   const int l0 = blockIdx.y * leaves_per_slice;
   const int l1 = min(nleaf, l0 + leaves_per_slice);
-  const int rank = ctx.rank, li = i / rank, ii = i - li * rank;
+  const int rank = ctx.rank, li = i / rank;
   const int2 me = __ldg(&ctx.leafxy[li]);
   const double2 ri = __ldg(&ctx.pts[i]);
   const double qi = __ldg(&ctx.q[i]);
   const double kq = ctx.kappa * ctx.kappa * qi;
-  // Entries below 1e-16 are zero (entry.cuh).  The operator's own entries are at
-  // most a few units, so a row with kappa^2 |q| < 1e-30 holds the identity alone.
-  const bool only_identity = PHI && !(fabs(kq) >= 1e-30);
+  // the rows whose far entries are zero in the matrix too (entry.cuh)
+  const bool no_far = PHI && far_is_zero(qi, ctx, kEntryFloor);
   double2 far[NR], near[NR];
 #pragma unroll
   for (int s = 0; s < NR; ++s) far[s] = near[s] = make_double2(0.0, 0.0);
@@ -227,14 +228,13 @@ __global__ void __launch_bounds__(kMvRows) leaf_matvec_kernel(const double2* __r
     const int2 b = __ldg(&ctx.leafxy[lj]);
     const int dx = b.x - me.x, dy = b.y - me.y;
     const bool close = dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1;
-    const bool series = !close && !only_identity;
+    const bool series = !close && !no_far;
     const unsigned mask = __ballot_sync(0xffffffffu, series);
     if (series) {
       const double2 c = __ldg(&ctx.leafc[lj]);
       moment_series<NR>(ri.x - c.x, ri.y - c.y, ctx.kappa, sm, mask, far);
-    } else if (close && (!only_identity || lj == li)) {
-      const int j0 = only_identity ? ii : 0, j1 = only_identity ? ii + 1 : rank;
-      for (int j = j0; j < j1; ++j) {
+    } else if (close) {
+      for (int j = 0; j < rank; ++j) {
         const double2 a = lsa_entry<PHI>(i, lj * rank + j, ctx);
         if (a.x == 0.0 && a.y == 0.0) continue;
 #pragma unroll

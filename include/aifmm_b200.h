@@ -209,7 +209,9 @@ aifmm_status aifmm_zgemm(aifmm_problem* p, int opA, int opB, int m, int n, int k
                          int flags);
 
 /* The dense product of the find_error fixture generator (FMM2DTree_gen_rhs_x.hpp:2864-2871):
- * y = A x with exact entries, x and y N x nrhs complex (nrhs <= 8). */
+ * y = A x without compression, x and y N x nrhs complex (nrhs <= 8).  The far sources of
+ * a leaf are summed before the series, so entries below 1e-16, which aifmm_get_matrix
+ * returns as zero, take part: y differs by at most 1e-16 of sum |x| from that. */
 aifmm_status aifmm_dense_matvec(aifmm_problem* p, int nrhs, const double* x, double* y, int flags);
 
 /* The total field from a solution (hybrid.cpp:263-281, with the kernel's findPhi
