@@ -53,21 +53,48 @@ __global__ void list_entries_kernel(const int* __restrict__ I, const int* __rest
 // uniform reads of shared memory).  36,864 unknowns, one right-hand side, through
 // dense_matvec with host buffers: 958 ms with a series per entry, 3.2 ms with a
 // series per leaf; 2,304 unknowns: 4.4 ms and 0.14 ms; 256 unknowns: 99 us and 66 us.
+//
+// The recurrences run unnormalised, between 1e-250 and 1e212, and a moment multiplies them:
+// so a leaf's sources are divided by the power of two of their largest part, which comes
+// back exactly where the normalised sums are added up (a vector of 1e100 or 1e-100 would
+// overflow or vanish on the way).
 constexpr int kMvRows = 128;
 constexpr int kMvMaxRhs = 8;
 constexpr size_t kMvMomentBytes = size_t(64) << 20;  // moments of one chunk of leaves
 struct Moment { double2 p, q; };
+// of a leaf and a right-hand side: the orders 0 .. 60, then the power of two (in p.x)
+constexpr int kMoments = AIFMM_SERIES + 2;
 
 __global__ void __launch_bounds__(128) moments_kernel(const double2* __restrict__ x, Moment* __restrict__ mom, int N,
                                                       int nrhs, int leaf0, int rank, const double2* __restrict__ M) {
   const int leaf = leaf0 + blockIdx.x;
-  for (int t = threadIdx.x; t < (AIFMM_SERIES + 1) * nrhs; t += blockDim.x) {
+  __shared__ int s_exp[kMvMaxRhs];
+  // the exponents of the leaf's largest parts, a warp a right-hand side
+  for (int s = threadIdx.x >> 5; s < nrhs; s += blockDim.x >> 5) {
+    unsigned top = 0;
+    for (int j = threadIdx.x & 31; j < rank; j += 32) {
+      const double2 xv = __ldg(&x[(size_t)leaf * rank + (size_t)s * N + j]);
+      top = max(top, max((unsigned)__double2hiint(xv.x) & 0x7fffffffu, (unsigned)__double2hiint(xv.y) & 0x7fffffffu));
+    }
+    top = __reduce_max_sync(0xffffffffu, top) >> 20;
+    // infinities and NaN as they are; 2^-1000 .. 2^1000: its inverse is a double too
+    if ((threadIdx.x & 31) == 0) s_exp[s] = top == 0x7ff ? 0 : max(-1000, min(1000, (int)top - 1023));
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < kMoments * nrhs; t += blockDim.x) {
     const int n = t / nrhs, s = t - n * nrhs;
+    Moment* const out = mom + ((size_t)blockIdx.x * kMoments + n) * nrhs + s;
+    if (n > AIFMM_SERIES) {
+      const double2 two = make_double2(__hiloint2double((1023 + s_exp[s]) << 20, 0), 0.0);
+      *out = Moment{two, make_double2(0.0, 0.0)};
+      continue;
+    }
     const double2* xs = x + (size_t)leaf * rank + (size_t)s * N;
+    const double down = __hiloint2double((1023 - s_exp[s]) << 20, 0);
     double2 a = make_double2(0.0, 0.0), b = a;
     for (int j = 0; j < rank; ++j) {
       const double2* Mc = M + (size_t)j * (2 * AIFMM_SERIES + 1) + AIFMM_SERIES;
-      const double2 xv = __ldg(&xs[j]);
+      const double2 xv = cscale(__ldg(&xs[j]), down);
       a = cfma(__ldg(&Mc[n]), xv, a);
       b = cfma(__ldg(&Mc[-n]), xv, b);
     }
@@ -81,7 +108,7 @@ __global__ void __launch_bounds__(128) moments_kernel(const double2* __restrict_
       o.p = cadd(a, b);
       o.q = make_double2(-d.y, d.x);
     }
-    mom[((size_t)blockIdx.x * (AIFMM_SERIES + 1) + n) * nrhs + s] = o;
+    *out = o;
   }
 }
 
@@ -160,10 +187,15 @@ __device__ __forceinline__ void moment_series(double dx, double dy, double kappa
   const double inorm = 1.0 / (2.0 * norm - jcur);
   const double J0 = jcur * inorm, J1 = jp1 * inorm;
   S0 *= inorm; S1 *= inorm;
+  // the power of two of inorm first, so that the one of the leaf meets a normalised sum
+  const int hi = __double2hiint(inorm);
+  const double ipow = __hiloint2double(hi & 0x7ff00000, 0);
+  const double iman = __hiloint2double((hi & 0x800fffff) | 0x3ff00000, __double2loint(inorm));
 #pragma unroll
   for (int s = 0; s < NR; ++s) {
-    acc[s].x = fma(a[s].x, inorm, acc[s].x);
-    acc[s].y = fma(a[s].y, inorm, acc[s].y);
+    const double w = iman * mom[(AIFMM_SERIES + 1) * NR + s].p.x;
+    acc[s].x = fma(a[s].x * ipow, w, acc[s].x);
+    acc[s].y = fma(a[s].y * ipow, w, acc[s].y);
     a[s] = make_double2(0.0, 0.0);
   }
   // ---- upward: Y_n, n = 0 .. 60
@@ -190,8 +222,9 @@ __device__ __forceinline__ void moment_series(double dx, double dy, double kappa
   }
 #pragma unroll
   for (int s = 0; s < NR; ++s) {  // + i SY
-    acc[s].x -= a[s].y;
-    acc[s].y += a[s].x;
+    const double w = mom[(AIFMM_SERIES + 1) * NR + s].p.x;
+    acc[s].x = fma(-w, a[s].y, acc[s].x);
+    acc[s].y = fma(w, a[s].x, acc[s].y);
   }
 }
 
@@ -202,7 +235,7 @@ template <bool PHI, int NR>
 __global__ void __launch_bounds__(kMvRows) leaf_matvec_kernel(const double2* __restrict__ x, double2* y, int N,
                                                                int leaf0, int nleaf, int leaves_per_slice,
                                                                const Moment* __restrict__ mom, EntryCtx ctx) {
-  __shared__ Moment sm[(AIFMM_SERIES + 1) * NR];
+  __shared__ Moment sm[kMoments * NR];
   const bool live = blockIdx.x * kMvRows + threadIdx.x < N;
   const int i = min((int)(blockIdx.x * kMvRows + threadIdx.x), N - 1);
   const int l0 = blockIdx.y * leaves_per_slice;
@@ -220,8 +253,8 @@ __global__ void __launch_bounds__(kMvRows) leaf_matvec_kernel(const double2* __r
   for (int l = l0; l < l1; ++l) {
     // the leaf's moments, read by every thread order by order: one load latency
     // for all of them instead of one per order
-    const double2* src = reinterpret_cast<const double2*>(mom + (size_t)l * (AIFMM_SERIES + 1) * NR);
-    for (int t = threadIdx.x; t < 2 * (AIFMM_SERIES + 1) * NR; t += kMvRows)
+    const double2* src = reinterpret_cast<const double2*>(mom + (size_t)l * kMoments * NR);
+    for (int t = threadIdx.x; t < 2 * kMoments * NR; t += kMvRows)
       reinterpret_cast<double2*>(sm)[t] = __ldg(&src[t]);
     __syncthreads();
     const int lj = leaf0 + l;
@@ -276,7 +309,7 @@ int aifmm_launch_list_entries(const int* I, const int* J, long n, double2* out, 
 
 // bytes of moment scratch a dense product needs: one chunk of leaves
 size_t aifmm_matvec_scratch_bytes(int N, int rank, int nrhs) {
-  const size_t per_leaf = sizeof(Moment) * (AIFMM_SERIES + 1) * (size_t)nrhs;
+  const size_t per_leaf = sizeof(Moment) * kMoments * (size_t)nrhs;
   const size_t nleaf = (size_t)N / rank;
   return per_leaf * std::min(nleaf, std::max<size_t>(1, kMvMomentBytes / per_leaf));
 }
@@ -293,7 +326,7 @@ int launch_matvec(const double2* x, double2* y, int N, int nrhs, void* scratch, 
   if (nrhs < 1 || nrhs > kMvMaxRhs) return (int)cudaErrorInvalidValue;
   Moment* mom = static_cast<Moment*>(scratch);
   const int nleaf = N / ctx.rank;
-  const int chunk = (int)(aifmm_matvec_scratch_bytes(N, ctx.rank, nrhs) / (sizeof(Moment) * (AIFMM_SERIES + 1) * nrhs));
+  const int chunk = (int)(aifmm_matvec_scratch_bytes(N, ctx.rank, nrhs) / (sizeof(Moment) * kMoments * nrhs));
   const int row_blocks = (N + kMvRows - 1) / kMvRows;
   for (int leaf0 = 0; leaf0 < nleaf; leaf0 += chunk) {
     const int nl = std::min(chunk, nleaf - leaf0);

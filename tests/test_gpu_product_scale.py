@@ -25,7 +25,10 @@ def test_powers_of_two(n_cheb, depth, kappa, e):
 
     got = times(K.dense_matvec(times(x, e)), -e)
     scale = np.abs(x).sum(axis=1).max()
-    tiny = np.ldexp(4.0 * K.N, -1074 - e) if e < -1000 else 0.0  # the products' own rounding to subnormals
+    # sums of subnormals: half a unit an addition, of the near entries and of the leaves' far sums,
+    # which kappa^2 q <= 1.5 kappa^2 multiplies
+    units = 18 * K.rank + (2 * 4 ** depth + 4) * max(1.0, 1.5 * kappa ** 2)
+    tiny = np.ldexp(units, -1074 - e) if e < -1000 else 0.0
     assert np.all(np.abs(got - y) <= 1e-13 * scale + tiny)
 
 
