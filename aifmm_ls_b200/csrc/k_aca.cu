@@ -19,6 +19,7 @@
 //     new term, prev_normS is not updated when the rank becomes 2).
 // The unmodified rows (Ar) or columns (Ac) are the outputs the solver keeps.
 #include <cfloat>
+#include "aca_cluster.h"
 #include "kernels.h"
 #include "entry.cuh"
 
@@ -38,7 +39,7 @@ namespace {
 // disk), 37 (depth 5) and 108 ms (depth 6, a narrow Gaussian); now 1.07, 9.4, 28 and 17 ms.
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
-constexpr int kMaxCluster = 8;
+constexpr int kMaxCluster = kAcaMaxCluster;
 constexpr int kMag = 4;      // magnitudes a thread keeps in shared memory (the rest: computed twice)
 constexpr int kCoef = 32;   // coefficients of a residual held in shared memory (the rest: global memory)
 typedef unsigned long long u64;
@@ -333,15 +334,10 @@ __global__ void __launch_bounds__(kThreads, 4) aca_kernel(const AcaJob* __restri
 
 }  // namespace
 
-int aifmm_launch_aca(const AcaJob* d_jobs, int njobs, double tol, const EntryCtx& ctx, cudaStream_t stream) {
+int aifmm_launch_aca(const AcaJob* d_jobs, int njobs, long level_jobs, double tol, const EntryCtx& ctx,
+                     cudaStream_t stream) {
   if (njobs <= 0) return 0;
-  // Two CTAs a job at least, up to eight while four of them a slot of the device (four CTAs
-  // on each of 148 SMs) are not reached.  Measured, whole assemblies with all levels at one,
-  // two, four and eight: depth 3 (128 and 32 jobs) 2.5, 1.16, 1.16, 1.07 ms; depth 4, 8 x 8
-  // nodes (512 ..) 19.6, 11.6, 10.5, 10.6 ms; depth 5 (2048 ..) 47.5, 31.7, 32.8, 38.3 ms.
-  constexpr long kCtas = 4 * (4 * 148);
-  int csize = kMaxCluster;
-  while (csize > 2 && (long)njobs * csize > kCtas) csize /= 2;
+  const int csize = aca_cluster_size(level_jobs);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(njobs * csize));
   cfg.blockDim = dim3(kThreads);

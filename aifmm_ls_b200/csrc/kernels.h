@@ -144,7 +144,9 @@ int aifmm_launch_dense_matvec(const double2* x, double2* y, int N, int nrhs, voi
 // y += G x with G the entries without kappa^2 q and identity (findPhi = false)
 int aifmm_launch_green_matvec_add(const double2* x, double2* y, int N, int nrhs, void* scratch, const EntryCtx& ctx,
                                   cudaStream_t stream);
-int aifmm_launch_aca(const AcaJob* d_jobs, int njobs, double tol, const EntryCtx& ctx, cudaStream_t stream);
+// level_jobs: the jobs of the whole level that these are some of (aca_cluster.h)
+int aifmm_launch_aca(const AcaJob* d_jobs, int njobs, long level_jobs, double tol, const EntryCtx& ctx,
+                     cudaStream_t stream);
 int aifmm_launch_qr_factor(const QRJob* d_jobs, int njobs, int mmax, int nmax, int es, cudaStream_t s);
 int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njobs, int total_cols, int mmax, int es,
                           cudaStream_t s);

@@ -1316,7 +1316,7 @@ struct aifmm_problem {
         ta = clk::now();
         const AcaJob* dj = stage.put(jobs, st);
         CK(cudaEventRecord(ea, st));
-        KL(aifmm_launch_aca(dj, nj, tol, cx, st));
+        KL(aifmm_launch_aca(dj, nj, 2L * nbx, tol, cx, st));
         CK(cudaEventRecord(eb, st));
         // ---- ranks and skeletons back to the host
         std::vector<int> hres(2 * (size_t)nj + nres + 1);
