@@ -14,6 +14,7 @@
 // The n and -n terms are paired, J_{-n} = (-1)^n J_n, Y_{-n} = (-1)^n Y_n.
 #pragma once
 #include "common.cuh"
+#include "quotient.cuh"
 
 #define AIFMM_SERIES 60
 
@@ -21,24 +22,11 @@
 // time in the ACA, the rest is the latency of the recurrences at 16 warps an SM).
 // 592 ACA jobs of 972 x 36 points, ranks 19 to 21: 11.4 ms each way with plain
 // divisions and a column of coefficients per lane, 6.2 ms now.  Divisions by R
-// and by whole numbers are correctly rounded quotients from a reciprocal (quotient
-// below), the counters are doubles (conversions run at a fraction of the FP64 rate),
+// and by whole numbers are correctly rounded quotients from a reciprocal
+// (quotient.cuh), the counters are doubles (conversions run at a fraction of the FP64 rate),
 // and the coefficients are laid out with the sources of a leaf next to each other (Mt:
 // the lanes of a warp read neighbouring sources).  Results are those of plain IEEE
 // divisions, bit for bit.
-
-// a / b correctly rounded, y = 1 / b correctly rounded: P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34
-// (1990), Theorem: from a q within one unit in the last place, q + (a - b q) y rounds
-// to a / b.  The first correction brings a y there, the second rounds.  a, b, the
-// quotient and the remainders stay away from the ends of the exponent range
-// (kQuotLo, kQuotHi below).
-__device__ __forceinline__ double quotient(double a, double b, double y) {
-  double q = __dmul_rn(a, y);
-  q = __fma_rn(__fma_rn(-b, q, a), y, q);
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-constexpr double kQuotLo = 1e-20, kQuotHi = 1e20;  // R; the recurrences' values lie in 1e-270 .. 1e230
 
 // 1 / k
 constexpr int kRecips = 1024;
