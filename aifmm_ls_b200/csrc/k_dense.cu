@@ -1046,6 +1046,7 @@ int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njob
   if (njobs <= 0 || total_cols <= 0) return 0;
   if (!valid_es(es)) return (int)cudaErrorInvalidValue;
   const int blocks = (total_cols + kW - 1) / kW;
+  // up to kSolveWideMax rows the column stays in registers (the jobs' `work` may be nullptr)
 #define AIFMM_SOLVE_WIDE(R)                                                                                     \
   if (mmax <= 32 * R) {                                                                                         \
     if (es == 16) qr_solve_wide_kernel<double2, R><<<blocks, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols); \
@@ -1054,6 +1055,7 @@ int aifmm_launch_qr_solve(const SolveJob* d_jobs, const int* d_col_off, int njob
   }
   AIFMM_SOLVE_WIDE(4) AIFMM_SOLVE_WIDE(8) AIFMM_SOLVE_WIDE(12)
 #undef AIFMM_SOLVE_WIDE
+  static_assert(kSolveWideMax == 32 * 12, "the largest case above");
   if (es == 16) qr_solve_kernel<double2><<<blocks, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
   else qr_solve_kernel<float2><<<blocks, kT, 0, s>>>(d_jobs, d_col_off, njobs, total_cols);
   return (int)cudaGetLastError();

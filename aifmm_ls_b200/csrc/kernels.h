@@ -55,8 +55,9 @@ struct SolveJob {        // X = alpha * QR^{-1} B
   void* X; int ldx;
   int nrhs;
   double2 alpha;
-  void* work;            // m x nrhs
+  void* work;            // m x nrhs, for more than kSolveWideMax rows
 };
+constexpr int kSolveWideMax = 384;
 
 struct FormQJob {
   const void* qr; int ldq; int m, n;

@@ -855,8 +855,9 @@ struct aifmm_problem {
         off[i] = tot;
         tot += large[i].nrhs;
         mlarge = std::max(mlarge, large[i].m);
-        large[i].work = scratch.get((size_t)es * large[i].m * large[i].nrhs);
       }
+      if (mlarge > kSolveWideMax)  // the column in global memory
+        for (auto& j : large) j.work = scratch.get((size_t)es * j.m * j.nrhs);
       auto ptrs = put_many_({{large.data(), large.size() * sizeof(SolveJob)}, {off.data(), off.size() * sizeof(int)}});
       double fl = 0;
       for (auto& j : large) { const double mz = std::min(j.m, j.n); fl += (16.0 * j.m * mz - 4.0 * mz * mz) * j.nrhs; }
