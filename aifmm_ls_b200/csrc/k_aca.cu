@@ -32,11 +32,12 @@ namespace {
 // memory.  Maxima, first indices and norms are folded in each CTA and exchanged through
 // the cluster's shared memory; every CTA then holds the same values, takes the same
 // decisions and meets the others at the same barriers.
-// What bounds it: the 61 orders of an entry, a serial chain of FP64 (39% of the FP64 rate
-// at the leaves of depth 4), one primary vector after the other.  With one CTA of 256
-// threads a job, and every row outside the contrast's support evaluated in search of a
-// first vector, the assemblies' ACA took 2.5 ms (depth 3), 26.7 (depth 4, 8 x 8 nodes, a
-// disk), 37 (depth 5) and 108 ms (depth 6, a narrow Gaussian); now 1.07, 9.4, 28 and 17 ms.
+// What bounds it: the 61 orders of an entry, a serial chain of FP64 (34% of the FP64 rate
+// at the leaves of depth 4, 17% at the level above), one primary vector after the other.
+// With one CTA of 256 threads a job, and every row outside the contrast's support
+// evaluated in search of a first vector, the assemblies' ACA took 2.5 ms (depth 3), 26.7
+// (depth 4, 8 x 8 nodes, a disk), 37 (depth 5) and 108 ms (depth 6, a narrow Gaussian);
+// now 1.07, 9.4, 28 and 17 ms.
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCluster = kAcaMaxCluster;

@@ -684,8 +684,8 @@ __global__ void __launch_bounds__(32 * WM * WN * (NS == 1 ? 1 : 2)) gemm_kernel(
 // R, the column permutation.
 // What bounds it: the chain of 2 nzp dependent steps; a reflector's is its dot
 // product over eight lanes (three shuffles: the two upper levels of the sum over 32
-// rows stay in a lane), tau and the update, about 350 cycles of it instruction issue
-// and latency in equal parts.  36 x 36, 12 boxes, 8 columns: 15.2 us (a warp per
+// rows stay in a lane), tau and the update, about 350 cycles; a scheduler has one warp,
+// which issues in 28% of them and waits for a dependent result in most others.  36 x 36, 12 boxes, 8 columns: 15.2 us (a warp per
 // column: 20.8 us); 300 boxes: 19 us (36 us).
 // Sums run in the order of 32 lanes over the rows (row mod 32), levels 16 to 1.
 constexpr int kSolveCols = 16, kSolveT = 8 * kSolveCols;

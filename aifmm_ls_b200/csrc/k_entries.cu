@@ -50,9 +50,9 @@ __global__ void list_entries_kernel(const int* __restrict__ I, const int* __rest
 //   p_n = m_n + (-1)^n m_{-n},  q_n = i (m_n - (-1)^n m_{-n}),  p_0 = m_0,  q_0 = 0
 // What bounds it: latency and issue of the FP64 recurrences (about 1,900 double
 // instructions per target, leaf and one right-hand side; the moments are warp-
-// uniform reads of shared memory).  36,864 unknowns, one right-hand side, through
+// uniform reads of shared memory; FP64 pipe 47% busy).  36,864 unknowns, one right-hand side, through
 // dense_matvec with host buffers: 958 ms with a series per entry, 3.2 ms with a
-// series per leaf; 2,304 unknowns: 4.4 ms and 0.14 ms; 256 unknowns: 99 us and 66 us.
+// series per leaf; 2,304 unknowns: 4.4 ms and 0.13 ms; 256 unknowns: 99 us and 63 us.
 //
 // The recurrences run unnormalised, between 1e-250 and 1e212, and a moment multiplies them:
 // so a leaf's sources are divided by the power of two of their largest part, which comes

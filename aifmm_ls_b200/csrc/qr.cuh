@@ -356,7 +356,7 @@ __device__ __forceinline__ void qr_reg_body(int m, int n, Load load, C* out, int
 // Norms and positions are double-buffered by step parity, so a warp running
 // ahead never changes what a slower warp is still scanning.  Columns left at
 // positions >= min(m, n) are written out at the end.
-// Arithmetic: pivot ties as in qr_factor_body; the reflector scalars tau and
+// Arithmetic: pivot ties as in qr_factor_kernel (kPivotTie); the reflector scalars tau and
 // 1/(a_kk - beta) come from one division; the norm downdate of LAPACK Working
 // Note 176 is evaluated without divisions -- with T = (nu - |r|)(nu + |r|) (the
 // LAWN quantity (1 - (|r|/nu)^2) times nu^2), the column is recomputed when

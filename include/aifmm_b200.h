@@ -12,7 +12,9 @@
  * selected with AIFMM_PTR_DEVICE in `flags`; everything else is host memory.
  * Calls on one handle must not overlap (one CUDA stream per handle); separate
  * handles are independent.  Every call returns a status; aifmm_last_error()
- * gives the message of the last failure on a handle.
+ * gives the message of the last failure on a handle.  A failed call leaves nothing
+ * running on its handle, which can be used on (after a failed factorisation: from
+ * aifmm_build_tree, or from a kept assembly).
  */
 #ifndef AIFMM_B200_H
 #define AIFMM_B200_H
