@@ -80,6 +80,23 @@ def test_after_a_failed_factorisation(reference, part):
     _check(K, T, reference)
 
 
+@pytest.mark.parametrize("part", [0.2, 0.5, 0.85])
+def test_a_kept_assembly_survives_a_failed_factorisation(reference, part):
+    import aifmm_ls_b200 as A
+    K, T = _handle()
+    T.assemble()
+    before = _pool(T)
+    T.factorize(keep_assembly=True)
+    grown = _pool(T) - before
+    K, T = _handle()
+    T.assemble()
+    with _Full(int(part * grown)):  # in the copy of the assembly, or in the elimination
+        with pytest.raises(A.AifmmError, match="cudaMalloc"):
+            T.factorize(keep_assembly=True)
+    T.factorize(keep_assembly=True)
+    assert np.array_equal(T.solve_factored(reference["b"]), reference["x"])
+
+
 def test_after_a_failed_assembly(reference):
     import aifmm_ls_b200 as A
     K, T = _handle()
